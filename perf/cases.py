@@ -86,7 +86,7 @@ def _provider(case: dict, seed: int, layers: int, capacity: int):
     """A handle with its layers bound: what a serving process builds once."""
     device = torch.device("cuda", torch.cuda.current_device())
     provider = aima.MoeProvider(layers=layers, max_prefill_tokens=capacity)
-    distinct = [aima.synth.layer_weights_cuda_fast(seed, layer, device) for layer in range(min(layers, MAX_DISTINCT))]
+    distinct = _layer_weights(layers, seed)
     for layer in range(layers):
         provider.bind_layer(layer, distinct[layer % len(distinct)])
     routing = case.get("routing", "uniform")
@@ -97,6 +97,11 @@ def _provider(case: dict, seed: int, layers: int, capacity: int):
     elif routing == "ties":
         provider.set_router_hooks(None, quantize_eighths=True)
     return provider
+
+
+def _layer_weights(layers: int, seed: int) -> list:
+    device = torch.device("cuda", torch.cuda.current_device())
+    return [aima.synth.layer_weights_cuda_fast(seed, layer, device) for layer in range(min(layers, MAX_DISTINCT))]
 
 
 def prepare(case: dict, seed: int) -> dict:
@@ -189,3 +194,71 @@ def tolerance(case: dict):
     if kind == "gemm":
         return {"rel": 4.0e-3, "max": 0.016}      # one BF16 rounding: rel 1.7e-3 / max 3.9e-3 against FP64
     return {"rel": 1.1e-3, "max": 0.05}
+
+
+# ---- the same values in 64 bits ----------------------------------------------------------------------------------
+
+def _norm64(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    return x * torch.rsqrt((x * x).mean(dim=-1, keepdim=True) + 1.0e-6) * (1.0 + weight.double())
+
+
+def _moe64(h: torch.Tensor, weights: dict, logit_hook) -> torch.Tensor:
+    """routed + shared experts of one layer for the rows of h, everything but the routing decision unrounded."""
+    logits = logit_hook(h @ weights["router"].double().T)
+    order = torch.sort(logits, dim=1, descending=True, stable=True)           # ties: lowest expert first
+    ids, share = order.indices[:, :TOP_K], torch.softmax(order.values[:, :TOP_K], dim=1)
+    out = torch.zeros_like(h)
+    for expert in torch.unique(ids).tolist():
+        row, slot = torch.nonzero(ids == expert, as_tuple=True)
+        gate, up = (h[row] @ weights["expert_gate_up"][expert].double().T).split(INTER, dim=1)
+        down = (torch.nn.functional.silu(gate) * up) @ weights["expert_down"][expert].double().T
+        out.index_add_(0, row, down * share[row, slot].unsqueeze(1))
+    act = torch.nn.functional.silu(h @ weights["shared_gate_proj"].double().T) * (h @ weights["shared_up_proj"].double().T)
+    return out + torch.sigmoid(h @ weights["shared_gate"].double().T) * (act @ weights["shared_down_proj"].double().T)
+
+
+def exact(case: dict, seed: int):
+    kind, generator = case["kind"], _generator(seed)
+    if kind == "gemm":
+        a = _normal(generator, case["m"], case["k"])
+        return a.double() @ _normal(generator, case["n"], case["k"], std=0.02).double().T
+    if kind == "lm_head":
+        # the logits of the int8 copy; the few rows that are evaluated exactly move the norm by less than it is off
+        weight, hidden = _normal(generator, case["rows"], HIDDEN, std=0.02), _normal(generator, HIDDEN).double()
+        parts = []
+        for rows in weight.split(16384):
+            scale = rows.float().abs().amax(dim=1).clamp_min(1.0e-12) * np.float32(1.0 / 127.0)
+            q = (rows.float() / scale.unsqueeze(1)).round().clamp(-127, 127)
+            parts.append((q.double() @ hidden) * scale.double())
+        return torch.cat(parts), None, None
+    layers = case.get("layers", 1)
+    if layers > 20:
+        return None          # a token through that many layers of random weights: roundings decide its later experts
+    weights = _layer_weights(layers, seed)
+    if kind in ("decode_calls", "decode_stack"):
+        x = _normal(generator, HIDDEN).double().unsqueeze(0)
+        for layer in range(layers):
+            w = weights[layer % len(weights)]
+            x = x + _moe64(_norm64(x, w["post_attention_layernorm"]), w, lambda logits: logits)
+        return x[0]
+    routing, device = case.get("routing", "uniform"), weights[0]["router"].device
+    bias = {"zipf": lambda: aima.synth.zipf_router_bias(seed).to(device),
+            "hot": lambda: aima.synth.hot_expert_bias(range(3, EXPERTS, 32)).to(device)}.get(routing, lambda: 0.0)()
+
+    def hook(logits: torch.Tensor) -> torch.Tensor:      # the path routes by BF16 logits
+        logits = logits + bias
+        if routing == "ties":
+            logits = (logits * 8.0).round() * 0.125
+        return logits.bfloat16().double()
+
+    a = _normal(generator, case["tokens"], HIDDEN).double()
+    if kind == "prefill_stack":
+        for layer in range(layers):
+            a = a + _moe64(_norm64(a, weights[layer]["post_attention_layernorm"]), weights[layer], hook)
+        return a
+    b = _normal(generator, case["tokens"], HIDDEN).double()
+    if kind == "prefill":
+        return b + _moe64(a, weights[0], hook)
+    residual = a + b
+    out = residual + _moe64(_norm64(residual, weights[0]["post_attention_layernorm"]), weights[0], hook)
+    return out, _norm64(out, _normal(generator, HIDDEN, std=0.02))
