@@ -104,6 +104,16 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// One lane of a converged warp.  The producer and MMA loops below are run by their WHOLE warp and only the issuing
+// instructions are guarded by this: the operands of TMA and tcgen05 instructions live in the warp's uniform registers,
+// and inside a branch on `lane == 0` the compiler has to move every one of them there again under divergence.  With
+// that branch around the loops a stage cost its TMA thread 680 cycles (two loads) and its MMA thread 320 (four MMAs)
+// of issue time -- more than the 512 cycles the tensor cores need for it.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+  return chosen != 0;
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                :: "r"(bar) : "memory");
@@ -311,7 +321,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kStages * kStageBytes + 8 * (2 * kStages + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + kStages * kStageBytes + 8 * (2 * kStages + 4) + 8);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // known to be the same in all lanes
   const int lane = threadIdx.x & 31;
   const GroupedGemm& g = pb.g;
 
@@ -375,43 +385,44 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;
-      bool alive = true;
-      for (int unit = blockIdx.x; unit < total_units && alive; unit += gridDim.x) {
-        int tile, chunk, expert, row0, rows;
-        unit_tile(unit, tile, chunk, expert, row0, rows);
-        int b0_row, b1_row;
-        if (kDual) {
-          b0_row = expert * pb.b_rows_per_expert + chunk * (kBN / 2);
-          b1_row = expert * pb.b_rows_per_expert + pb.up_row_offset + chunk * (kBN / 2);
-        } else {
-          b0_row = expert * pb.b_rows_per_expert + chunk * kBN;
-          b1_row = b0_row + kBN / 2;
-        }
-        for (int kb = 0; kb < k_blocks; ++kb) {
+    int stage = 0;
+    uint32_t phase = 0;
+    int issued = 0;
+    bool alive = true;
+    for (int unit = blockIdx.x; unit < total_units && alive; unit += gridDim.x) {
+      int tile, chunk, expert, row0, rows;
+      unit_tile(unit, tile, chunk, expert, row0, rows);
+      int b0_row, b1_row;
+      if (kDual) {
+        b0_row = expert * pb.b_rows_per_expert + chunk * (kBN / 2);
+        b1_row = expert * pb.b_rows_per_expert + pb.up_row_offset + chunk * (kBN / 2);
+      } else {
+        b0_row = expert * pb.b_rows_per_expert + chunk * kBN;
+        b1_row = b0_row + kBN / 2;
+      }
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (elect_one()) {
           const uint32_t a_dst = smem_base + stage * kStageBytes;
           const uint32_t b_dst = a_dst + kStageABytes;
-          if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
           mbar_arrive_expect_tx(full_bar(stage), kGather ? kStageBBytes : kStageBytes);
           if (!kGather) tma_load_2d(a_dst, &maps.a, kb * kBK, row0, full_bar(stage));
           tma_load_2d(b_dst, &maps.b0, kb * kBK, b0_row, full_bar(stage));
           tma_load_2d(b_dst + kStageBBytes / 2, kDual ? &maps.b1 : &maps.b0, kb * kBK, b1_row, full_bar(stage));
-          ++issued;
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
+        __syncwarp();
+        ++issued;
+        if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
-      // drain on abort: wait (bounded) for the stages whose copies are still in flight
-      if (*abort_flag != 0) {
-        volatile int ignore = 0;
-        int s = stage;
-        uint32_t ph = phase;
-        for (int i = 0; i < min(issued, kStages); ++i) {
-          if (--s < 0) { s = kStages - 1; ph ^= 1u; }
-          mbar_wait_bounded(full_bar(s), ph, &ignore);
-        }
+    }
+    // drain on abort: wait (bounded) for the stages whose copies are still in flight
+    if (lane == 0 && *abort_flag != 0) {
+      volatile int ignore = 0;
+      int s = stage;
+      uint32_t ph = phase;
+      for (int i = 0; i < min(issued, kStages); ++i) {
+        if (--s < 0) { s = kStages - 1; ph ^= 1u; }
+        mbar_wait_bounded(full_bar(s), ph, &ignore);
       }
     }
   } else if (kGather && (warp == 2 || warp == 3)) {
@@ -435,8 +446,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int r = (lt >> 3) + 8 * j;
-        const int token = g.sorted_rows[row0 + min(r, rows - 1)] >> 3;   // rows past the tile's end repeat its last row
-        source[j] = token * g.lda + piece * 8;
+        source[j] = r < rows ? (g.sorted_rows[row0 + r] >> 3) * g.lda + piece * 8 : -1;   // nothing past the tile's end
       }
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
@@ -444,7 +454,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int r = (lt >> 3) + 8 * j;
-          cp_async_16(base + r * 128 + ((piece ^ (r & 7)) << 4), g.gather_src + source[j] + kb * kBK);
+          if (source[j] >= 0) cp_async_16(base + r * 128 + ((piece ^ (r & 7)) << 4), g.gather_src + source[j] + kb * kBK);
         }
         cp_async_arrive_noinc(full_bar(stage));
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
@@ -453,26 +463,25 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
     cp_async_wait_all();     // nothing of this thread's may be in flight when the block exits
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int local = 0;
-      bool alive = true;
-      for (int unit = blockIdx.x; unit < total_units && alive; unit += gridDim.x, ++local) {
-        const int buf = local & 1;
-        const uint32_t use = static_cast<uint32_t>(local >> 1);
-        // the epilogue must have drained this accumulator buffer (first use: free)
-        if (!mbar_wait_bounded(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+    int stage = 0;
+    uint32_t phase = 0;
+    int local = 0;
+    bool alive = true;
+    for (int unit = blockIdx.x; unit < total_units && alive; unit += gridDim.x, ++local) {
+      const int buf = local & 1;
+      const uint32_t use = static_cast<uint32_t>(local >> 1);
+      // the epilogue must have drained this accumulator buffer (first use: free)
+      if (!mbar_wait_bounded(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kBN);
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_bounded(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
+        if (kGather) fence_async_proxy();     // rows written by cp.async are read through the async proxy
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kBN);
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
-          if (kGather) fence_async_proxy();     // rows written by cp.async are read through the async proxy
-          tc_fence_after();
+        if (elect_one()) {
           const uint32_t a_addr = smem_base + stage * kStageBytes;
-          const uint32_t b_addr = a_addr + kStageABytes;
           const uint64_t adesc = smem_desc_k_major_sw128(a_addr);
-          const uint64_t bdesc = smem_desc_k_major_sw128(b_addr);
+          const uint64_t bdesc = smem_desc_k_major_sw128(a_addr + kStageABytes);
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             // advancing 16 elements (32 bytes) along K inside the swizzled row
@@ -480,9 +489,10 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
                       kInstrDesc, (kb | k) != 0 ? 1u : 0u);
           }
           umma_commit(empty_bar(stage));      // frees the stage when the MMAs above retire
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if (kb + 1 == k_blocks) umma_commit(tfull_bar(buf));
         }
-        if (alive) umma_commit(tfull_bar(buf));
+        __syncwarp();
+        if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp >= 4) {
@@ -511,29 +521,45 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
 }
 
 // ---------------------------------------------------------------------------
-// Two-SM form.  A pair of blocks (a cluster of two) works on one tile of up to 256 rows of one expert x
-// 256 accumulator columns with tcgen05.mma.cta_group::2: block r of the pair holds rows 128 r .. 128 r + 127
-// of A and one half of B (128 weight rows) per K block, 32 KB per stage instead of 48, so six stages fit
-// and every weight byte enters shared memory once per 256 rows instead of once per 128.  The leader (block 0
-// of the pair) issues the MMAs for both; each block drains the 128 accumulator rows in its own tensor memory.
+// Two-SM form with the WEIGHTS on the M side.  A pair of blocks (a cluster of two) computes 256 weight rows x one
+// tile of N <= 256 rows of A, transposed: D^T[256, N] = W[256, K] . A[N, K]^T with tcgen05.mma.cta_group::2.  Block r
+// of the pair stages 128 weight rows and N / 2 rows of A per K block; the leader (block 0) issues the MMAs for both;
+// each block drains the 128 weight rows (= output columns) in its own tensor memory.
+//
+// Why this way round: the tile height of the instruction is fixed at 256 (or 128 in one block), its width N goes in
+// steps of 32.  With the rows of an expert on the M side every expert pads its last tile to 128 or 256 rows -- at
+// T = 8192 and balanced routing 1.25 x (128-row tiles) or 1.5 x (256) of the useful products, and with few rows per
+// expert nearly all of them -- while the weights, always whole multiples of 256 rows, pad nothing.  Here a tile costs
+// what its rows cost, rounded up to 32, and each weight byte enters shared memory once per up to 256 rows.
 //
 //   full[s]    leader only.  Completed by the TMA loads of BOTH blocks (cta_group::2 loads signal the
-//              leader's barrier), by the leader's gather threads and by the peer's forwarder.
-//   gdone[s]   peer only, gather mode: its gather threads' copies of a stage have landed; its forwarder
-//              (the peer's otherwise idle MMA warp) then arrives on the leader's full[s].
+//              leader's barrier).
 //   empty[s]   both blocks: the MMAs reading stage s have retired (tcgen05.commit, multicast to the pair).
 //   tfull[b]   both blocks: accumulator b is complete (commit, multicast).
 //   tempty[b]  leader only: the eight epilogue warps of each block have drained accumulator b.
 // No load uses cluster multicast: each block fetches its own operands.
 // ---------------------------------------------------------------------------
 constexpr int kStages2 = 6;
-constexpr int kStage2ABytes = kBM * kBK * 2;              // 16 KB: this block's 128 rows of A
-constexpr int kStage2BBytes = (kBN / 2) * kBK * 2;        // 16 KB: this block's half of B
+constexpr int kPairRows = 256;                            // rows of A per tile at most = accumulator columns of a buffer
+constexpr int kPlainBand = 8;                             // row tiles the units of a dense product walk together
+constexpr int kPairN = 256;                               // weight rows per unit (128 per block)
+constexpr int kStage2ABytes = 128 * kBK * 2;              // 16 KB: this block's 128 weight rows
+constexpr int kStage2BBytes = (kPairRows / 2) * kBK * 2;  // up to 16 KB: this block's half of the tile's rows
 constexpr int kStage2Bytes = kStage2ABytes + kStage2BBytes;
+constexpr int kGatherTableBytes = 32 * 16;                // per gather warp: token indices of 128 rows, in fours
 constexpr int kTc2BarrierBytes = 512;
+constexpr int kPairEpilogueWarps = 16;                    // four per quarter of the 128 TMEM lanes
+constexpr int kPairThreads = (4 + kPairEpilogueWarps) * 32;
+constexpr int kStoreStage2Bytes = 32 * 64;                // per epilogue warp: 32 rows x 32 BF16 outputs
 constexpr int kTc2SmemBytes = kStages2 * kStage2Bytes + 1024 /*alignment slack*/ + kTc2BarrierBytes +
-                              kEpilogueWarps * kStoreStageBytes;
+                              kPairEpilogueWarps * kStoreStage2Bytes + 2 * kGatherTableBytes;
 static_assert(kTc2SmemBytes <= 227 * 1024, "two-SM product kernel exceeds 227 KB of shared memory");
+
+struct TcPairMaps {
+  CUtensorMap w;        // weights: [rows, k] box 64 x 128, or the 5-D view of a gate_up tensor (make_gate_up_map)
+  CUtensorMap rows[4];  // A: boxes of 64 x 16, 32, 64 and 128 rows (any multiple of 16 rows is at most four loads);
+                        // gather: rows[0] is the box of one row
+};
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -550,15 +576,33 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Arrival on a barrier of either block, without cluster-scope release: what it orders are tensor-memory reads (complete
+// before it, tcgen05.wait::ld), and a release at that scope would first wait for every global store of the thread -- in
+// the epilogue, 3000 cycles per unit.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
 }
-// TMA tile load of one block of the pair; the bytes are accounted on the LEADER's barrier
+// TMA tile loads of one block of the pair; the bytes are accounted on the LEADER's barrier
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%2, %3}], [%4];"
       :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(leader_bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap* map, int x, int group, int expert,
+                                                 uint32_t leader_bar) {
+  const int zero = 0;
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %3, %4, %5}], [%6];"
+      :: "r"(dst), "l"(map), "r"(x), "r"(zero), "r"(group), "r"(expert), "r"(leader_bar) : "memory");
+}
+__device__ __forceinline__ void tma_gather4_pair(uint32_t dst, const CUtensorMap* map, int x, int r0, int r1, int r2,
+                                                 int r3, uint32_t leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+      :: "r"(dst), "l"(map), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(leader_bar) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -570,11 +614,10 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t colum
 }
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                                uint32_t idesc, uint32_t accumulate) {
-  const uint32_t zero = 0u;
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(zero) : "memory");
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // arrives on the barrier at the same shared-memory offset in both blocks of the pair once the MMAs issued so far retire
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
@@ -583,31 +626,155 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                :: "r"(bar), "h"(both) : "memory");
 }
 
-// D = F32, A = B = BF16, both K-major, M = 256 (128 rows per block), N = 256.
-constexpr uint32_t kInstrDesc2 =
-    (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kBN >> 3) << 17) |
-    (static_cast<uint32_t>((2 * kBM) >> 4) << 24);
+// D = F32, A = B = BF16, both K-major, M = 256 (128 weight rows per block), N = the tile's rows rounded up to 32
+__device__ __forceinline__ uint32_t pair_instr_desc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | ((256u >> 4) << 24);
+}
+__host__ __device__ inline int pair_width(int rows) { return (rows + 31) & ~31; }
+
+// 16 lanes x 32 columns of the accumulator in the fragment layout: v[4 i + 2 p + c] of thread t is lane t / 4 + 8 p,
+// column 8 i + 2 (t % 4) + c
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+// four 8 x 8 blocks of BF16 fragments, transposed: lane 8 m + j gives the address of row j of block m
+__device__ __forceinline__ void stmatrix_trans4(uint32_t smem_row, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+               :: "r"(smem_row), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  return static_cast<uint32_t>(float_to_bf16_bits(lo)) | (static_cast<uint32_t>(float_to_bf16_bits(hi)) << 16);
+}
+
+// One epilogue warp drains its share of D^T[128, rows]: TMEM lanes 32 q .. 32 q + 31 (output columns), every
+// `groups`-th 32-row batch of the tile.  Fragments of eight columns x eight rows are turned by stmatrix.trans into the
+// warp's own shared memory (16-byte pieces XOR-swizzled by the row: no bank conflicts on either side), from where a row
+// is written in whole 32- or 64-byte pieces.
+// `drained` is the leader's barrier for the accumulator: the warp arrives on it as soon as its last values are in
+// registers.
+template <int MODE>
+__device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcProblem& pb, uint32_t taddr, int rank,
+                                                 int q, int h, int lane, uint8_t* stage, int chunk, int row0, int rows,
+                                                 const float* scale, uint32_t drained) {
+  constexpr int kStep = 32 * (kPairEpilogueWarps / 4);
+  const uint32_t stage_s = smem_u32(stage);
+  auto release = [&]() {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cluster(drained);
+  };
+  if (32 * h >= rows) {
+    release();
+    return;
+  }
+  if (MODE == kGemmExpertGateUp) {
+    // lanes 0-15 of the quarter are gate columns, lanes 16-31 the up columns of the same sixteen outputs
+    __nv_bfloat16* dst = g.c + static_cast<size_t>(row0) * g.ldc + chunk * (kPairN / 2) + rank * 64 + 16 * q;
+#pragma unroll 1
+    for (int c0 = 32 * h; c0 < rows; c0 += kStep) {
+      uint32_t gr[16], ur[16];
+      tmem_ld_16x32(taddr + c0, gr);
+      tmem_ld_16x32(taddr + (16u << 16) + c0, ur);
+      tmem_ld_wait();
+      if (c0 + kStep >= rows) release();
+      uint32_t packed[8];         // [2 i + p]: rows 8 i .. 8 i + 7 of the batch, columns 8 p .. 8 p + 7
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float v[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const float gate = round_bf16(__uint_as_float(gr[2 * i + c]));
+          const float up = round_bf16(__uint_as_float(ur[2 * i + c]));
+          v[c] = __fmul_rn(round_bf16(det_silu(gate)), up);
+        }
+        packed[i] = pack_bf16(v[0], v[1]);
+      }
+      // 32 bytes per row: block m = 2 i' + p of a call holds rows 8 (2 call + i') .., piece p
+#pragma unroll
+      for (int call = 0; call < 2; ++call) {
+        const int row = 8 * (2 * call + (lane >> 4)) + (lane & 7);
+        const int piece = ((lane >> 3) & 1) ^ ((row >> 2) & 1);
+        stmatrix_trans4(stage_s + row * 32 + piece * 16, packed[4 * call], packed[4 * call + 1], packed[4 * call + 2],
+                        packed[4 * call + 3]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int row = 16 * i + (lane >> 1);
+        const uint4 w = *reinterpret_cast<const uint4*>(stage + row * 32 + (((lane & 1) ^ ((row >> 2) & 1)) * 16));
+        if (c0 + row < rows)
+          *reinterpret_cast<uint4*>(dst + static_cast<size_t>(c0 + row) * g.ldc + (lane & 1) * 8) = w;
+      }
+      __syncwarp();
+    }
+  } else {
+    const int col0 = chunk * kPairN + rank * 128 + 32 * q;
+    __nv_bfloat16* dst = g.c + static_cast<size_t>(row0) * g.ldc + col0;
+    const bool piece_ok = col0 + 8 * (lane & 3) < pb.n_valid;
+#pragma unroll
+    for (int b = 0; b < kPairRows / kStep; ++b) {
+      const int c0 = 32 * h + kStep * b;
+      if (c0 < rows) {
+        uint32_t r[32];           // [16 half + 4 i + 2 p + c]: column 16 half + 8 p + lane / 4, row 8 i + 2 (lane % 4) + c
+        tmem_ld_16x32(taddr + c0, r);
+        tmem_ld_16x32(taddr + (16u << 16) + c0, r + 16);
+        tmem_ld_wait();
+        if (c0 + kStep >= rows) release();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float s0 = 1.0f, s1 = 1.0f;
+          if (MODE == kGemmExpertDown) {
+            s0 = __shfl_sync(0xffffffffu, scale[b], 8 * i + 2 * (lane & 3));
+            s1 = __shfl_sync(0xffffffffu, scale[b], 8 * i + 2 * (lane & 3) + 1);
+          }
+          uint32_t packed[4];     // columns 8 m .. 8 m + 7 of rows 8 i .. 8 i + 7
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            float lo = __uint_as_float(r[16 * (m >> 1) + 4 * i + 2 * (m & 1)]);
+            float hi = __uint_as_float(r[16 * (m >> 1) + 4 * i + 2 * (m & 1) + 1]);
+            if (MODE == kGemmExpertDown) { lo = __fmul_rn(lo, s0); hi = __fmul_rn(hi, s1); }
+            packed[m] = pack_bf16(lo, hi);
+          }
+          const int row = 8 * i + (lane & 7);
+          stmatrix_trans4(stage_s + row * 64 + (((lane >> 3) ^ ((row >> 1) & 3)) * 16), packed[0], packed[1], packed[2], packed[3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = 8 * i + (lane >> 2);
+          const uint4 w = *reinterpret_cast<const uint4*>(stage + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) * 16));
+          if (c0 + row < rows && piece_ok)
+            *reinterpret_cast<uint4*>(dst + static_cast<size_t>(c0 + row) * g.ldc + (lane & 3) * 8) = w;
+        }
+        __syncwarp();
+      }
+    }
+  }
+}
 
 template <int MODE, bool kGather>
-__global__ void __launch_bounds__(kTcThreads, 1)
-grouped_gemm_tc2_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) {
-  static_assert(MODE == kGemmExpertGateUp || MODE == kGemmExpertDown, "two-SM form: the expert products");
-  constexpr bool kDual = (MODE == kGemmExpertGateUp);
+__global__ void __launch_bounds__(kPairThreads, 1)
+grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProblem pb) {
+  static_assert(MODE == kGemmExpertGateUp || MODE == kGemmExpertDown || MODE == kGemmPlain, "modes of the two-SM form");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + kStages2 * kStage2Bytes;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kStages2 + s); };
-  auto gdone_bar = [&](int s) { return bar_base + 8u * (2 * kStages2 + s); };
-  auto tfull_bar = [&](int b) { return bar_base + 8u * (3 * kStages2 + b); };
-  auto tempty_bar = [&](int b) { return bar_base + 8u * (3 * kStages2 + 2 + b); };
-  uint8_t* tail = smem_gen + kStages2 * kStage2Bytes + 8 * (3 * kStages2 + 4);
+  auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * kStages2 + b); };
+  auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * kStages2 + 2 + b); };
+  uint8_t* tail = smem_gen + kStages2 * kStage2Bytes + 8 * (2 * kStages2 + 4);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
   uint8_t* store_stage = smem_gen + kStages2 * kStage2Bytes + kTc2BarrierBytes;
+  uint8_t* gather_tables = store_stage + kPairEpilogueWarps * kStoreStage2Bytes;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // known to be the same in all lanes
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();          // 0: leader of the pair
   const bool leader = rank == 0;
@@ -615,13 +782,12 @@ grouped_gemm_tc2_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages2; ++s) {
-      mbar_init(full_bar(s), kGather ? 1 + kGatherThreads + 1 : 1);
+      mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
-      mbar_init(gdone_bar(s), kGatherThreads);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 2 * kEpilogueWarps);
+      mbar_init(tempty_bar(b), 2 * kPairEpilogueWarps);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -636,7 +802,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb)
 
   pdl_enter();
 
-  const int n_tiles = g.tile_count != nullptr ? *g.tile_count : g.max_tiles;
+  const int n_tiles = g.tile_count != nullptr ? *g.tile_count : (g.dense_rows + kPairRows - 1) / kPairRows;
   // as in the one-SM kernel; the leader samples the status for the pair
   volatile int* poison_slot = abort_flag + 1;
   if (threadIdx.x == 0 && leader) {
@@ -652,141 +818,205 @@ grouped_gemm_tc2_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb)
   const int pair = blockIdx.x >> 1;
   const int k_blocks = g.k / kBK;
 
-  // unit -> the tile's expert, this block's first row, its number of valid rows (0 .. 128) and the tile's last row
-  auto unit_tile = [&](int unit, int& chunk, int& expert, int& row0, int& rows, int& tile_last) {
-    const int tile = unit / pb.n_chunks;
-    chunk = unit - tile * pb.n_chunks;
-    expert = g.tile_expert[tile] - g.expert_base;
-    const int tile_rows = g.tile_rows[tile];
-    const int tile_row0 = g.tile_row0[tile];
-    tile_last = tile_row0 + tile_rows - 1;
-    row0 = tile_row0 + static_cast<int>(rank) * kBM;
-    rows = max(0, min(kBM, tile_rows - static_cast<int>(rank) * kBM));
+  // unit -> chunk of 256 weight rows, expert, first row and number of rows (1 .. 256) of the tile.  Every role asks for
+  // the unit after the one it works on (or later), so that these loads, and in the epilogue the two that follow from
+  // them, are never waited for between two units: in the down product, whose units are eight stages long, they cost
+  // half of a unit's time.
+  struct Unit {
+    int chunk, expert, row0, rows;
+  };
+  auto describe = [&](int unit) {
+    Unit u{0, 0, 0, 0};
+    if (unit >= total_units) return u;
+    if (MODE == kGemmPlain) {
+      // eight row tiles x all chunks at a time: the pairs that run together then share both operands in L2
+      const int band = unit / (kPlainBand * pb.n_chunks);
+      const int height = min(kPlainBand, n_tiles - band * kPlainBand);
+      const int within = unit - band * kPlainBand * pb.n_chunks;
+      u.chunk = within / height;
+      u.row0 = (band * kPlainBand + within - u.chunk * height) * kPairRows;
+      u.rows = min(kPairRows, g.dense_rows - u.row0);
+    } else {
+      const int tile = unit / pb.n_chunks;
+      u.chunk = unit - tile * pb.n_chunks;
+      u.expert = g.tile_expert[tile] - g.expert_base;
+      u.row0 = g.tile_row0[tile];
+      u.rows = g.tile_rows[tile];
+    }
+    return u;
   };
   auto timeout = [&]() { atomicCAS(pb.status, 0, kStatusTimeoutMbarrier); };
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both blocks) -----------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool alive = true;
-      for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
-        int chunk, expert, row0, rows, tile_last;
-        unit_tile(unit, chunk, expert, row0, rows, tile_last);
-        // this block's half of B: gate_up -- the leader takes the 128 gate rows of the chunk, the peer the 128
-        // up rows; down -- rows 128 r .. of the chunk's 256 output columns
-        const int b_row = kDual ? expert * pb.b_rows_per_expert + static_cast<int>(rank) * pb.up_row_offset + chunk * (kBN / 2)
-                                : expert * pb.b_rows_per_expert + chunk * kBN + static_cast<int>(rank) * (kBN / 2);
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          const uint32_t a_dst = smem_base + stage * kStage2Bytes;
-          const uint32_t b_dst = a_dst + kStage2ABytes;
-          if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
-          const uint32_t leader_full = map_to_rank(full_bar(stage), 0);
-          if (leader) mbar_arrive_expect_tx(full_bar(stage), 2 * (kGather ? kStage2BBytes : kStage2Bytes));
-          if (!kGather) tma_load_2d_pair(a_dst, &maps.a, kb * kBK, row0, leader_full);
-          tma_load_2d_pair(b_dst, &maps.b0, kb * kBK, b_row, leader_full);
-          if (++stage == kStages2) { stage = 0; phase ^= 1u; }
-        }
-      }
-    }
-  } else if (kGather && (warp == 2 || warp == 3)) {
-    // ------------------------------ A-row gather (both blocks) -----------------
-    const int lt = (warp - 2) * 32 + lane;
-    const int piece = lt & 7;
+    const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
     int stage = 0;
     uint32_t phase = 0;
     bool alive = true;
+    Unit next = describe(pair);
     for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
-      int chunk, expert, row0, rows, tile_last;
-      unit_tile(unit, chunk, expert, row0, rows, tile_last);
-      int source[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int r = (lt >> 3) + 8 * j;
-        // rows past the tile's end repeat its last row (a tile has at least one row)
-        const int token = g.sorted_rows[min(row0 + r, tile_last)] >> 3;
-        source[j] = token * g.lda + piece * 8;
-      }
+      const Unit u = next;
+      next = describe(unit + n_pairs);
+      const int half = pair_width(u.rows) / 2;      // a multiple of 16
+      const int my_row0 = u.row0 + static_cast<int>(rank) * half;
+      const int w_row = u.expert * pb.b_rows_per_expert + u.chunk * kPairN + static_cast<int>(rank) * 128;
+      // what both blocks fetch for a stage: weights, and the tile's rows (gathered: in fours per block)
+      uint32_t stage_bytes = 2 * (kStage2ABytes + half * kBK * 2);
+      if (kGather) stage_bytes = 2 * kStage2ABytes + ((min(half, u.rows) + 3) / 4 + (max(0, u.rows - half) + 3) / 4) * (4 * kBK * 2);
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
-        const uint32_t base = smem_base + stage * kStage2Bytes;
+        if (elect_one()) {
+          const uint32_t w_dst = smem_base + stage * kStage2Bytes;
+          const uint32_t leader_full = leader_full0 + 8u * stage;
+          if (leader) mbar_arrive_expect_tx(full_bar(stage), stage_bytes);
+          if (MODE == kGemmExpertGateUp)
+            tma_load_5d_pair(w_dst, &maps.w, kb * kBK, u.chunk * 8 + static_cast<int>(rank) * 4, u.expert, leader_full);
+          else
+            tma_load_2d_pair(w_dst, &maps.w, kb * kBK, w_row, leader_full);
+          if (!kGather) {
+            int done = 0;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int r = (lt >> 3) + 8 * j;
-          cp_async_16(base + r * 128 + ((piece ^ (r & 7)) << 4), g.gather_src + source[j] + kb * kBK);
+            for (int b = 3; b >= 0; --b) {
+              const int size = 16 << b;
+              if (half & size) {
+                tma_load_2d_pair(w_dst + kStage2ABytes + done * (kBK * 2), &maps.rows[b], kb * kBK, my_row0 + done, leader_full);
+                done += size;
+              }
+            }
+          }
         }
-        cp_async_arrive_noinc(leader ? full_bar(stage) : gdone_bar(stage));
+        __syncwarp();
         if (++stage == kStages2) { stage = 0; phase ^= 1u; }
       }
     }
-    cp_async_wait_all();
+  } else if (kGather && (warp == 2 || warp == 3)) {
+    // ------------------------------ row gather (both blocks) -------------------
+    // Rows by token index, four per TMA instruction (tile::gather4, a box of one row), the two warps in turn.  Only rows
+    // that exist are fetched, up to three repeats of the last one; what a stage holds beyond them ends in accumulator
+    // columns that nobody reads.  The tile's token indices wait in shared memory, one private copy per warp.
+    int4* table = reinterpret_cast<int4*>(gather_tables + (warp - 2) * kGatherTableBytes);
+    const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool alive = true;
+    // two units ahead: description; one unit ahead: token indices
+    auto tokens = [&](const Unit& u) {
+      const int half = pair_width(u.rows) / 2;
+      const int mine = max(0, min(half, u.rows - static_cast<int>(rank) * half));
+      int4 t = make_int4(0, 0, 0, 0);
+      if (4 * lane < mine) {
+        const int32_t* sorted = g.sorted_rows + u.row0 + static_cast<int>(rank) * half;
+        t.x = sorted[4 * lane];
+        t.y = sorted[min(4 * lane + 1, mine - 1)];
+        t.z = sorted[min(4 * lane + 2, mine - 1)];
+        t.w = sorted[min(4 * lane + 3, mine - 1)];
+      }
+      return t;
+    };
+    Unit next = describe(pair), later = describe(pair + n_pairs);
+    int4 next_tokens = tokens(next);
+    for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
+      const Unit u = next;
+      const int4 t4 = next_tokens;
+      next = later;
+      next_tokens = tokens(next);
+      later = describe(unit + 2 * n_pairs);
+      const int half = pair_width(u.rows) / 2;
+      const int fours = (max(0, min(half, u.rows - static_cast<int>(rank) * half)) + 3) / 4;
+      __syncwarp();
+      table[lane] = make_int4(t4.x >> 3, t4.y >> 3, t4.z >> 3, t4.w >> 3);
+      __syncwarp();
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        const uint32_t dst = smem_base + stage * kStage2Bytes + kStage2ABytes;
+        const uint32_t leader_full = leader_full0 + 8u * stage;
+        if (elect_one()) {
+#pragma unroll 4
+          for (int i = warp - 2; i < fours; i += 2) {
+            const int4 t = table[i];
+            tma_gather4_pair(dst + i * (4 * kBK * 2), &maps.rows[0], kb * kBK, t.x, t.y, t.z, t.w, leader_full);
+          }
+        }
+        __syncwarp();
+        if (++stage == kStages2) { stage = 0; phase ^= 1u; }
+      }
+    }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
       // ------------------------------ MMA issuer (leader) ------------------------
       int stage = 0;
       uint32_t phase = 0;
       int local = 0;
       bool alive = true;
+      Unit next = describe(pair);
       for (int unit = pair; unit < total_units && alive; unit += n_pairs, ++local) {
+        const uint32_t idesc = pair_instr_desc(pair_width(next.rows));
+        next = describe(unit + n_pairs);
         const int buf = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
         if (!mbar_wait_bounded(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kBN);
+        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kPairRows);
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait_bounded(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
-          if (kGather) fence_async_proxy();
           tc_fence_after();
-          const uint32_t a_addr = smem_base + stage * kStage2Bytes;
-          const uint32_t b_addr = a_addr + kStage2ABytes;
-          const uint64_t adesc = smem_desc_k_major_sw128(a_addr);
-          const uint64_t bdesc = smem_desc_k_major_sw128(b_addr);
+          if (elect_one()) {
+            const uint32_t w_addr = smem_base + stage * kStage2Bytes;
+            const uint64_t wdesc = smem_desc_k_major_sw128(w_addr);
+            const uint64_t rdesc = smem_desc_k_major_sw128(w_addr + kStage2ABytes);
 #pragma unroll
-          for (int k = 0; k < kBK / kUmmaK; ++k) {
-            umma_bf16_pair(tmem_d, adesc + static_cast<uint64_t>(k * 2), bdesc + static_cast<uint64_t>(k * 2),
-                           kInstrDesc2, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < kBK / kUmmaK; ++k) {
+              umma_bf16_pair(tmem_d, wdesc + static_cast<uint64_t>(k * 2), rdesc + static_cast<uint64_t>(k * 2),
+                             idesc, (kb | k) != 0 ? 1u : 0u);
+            }
+            umma_commit_pair(empty_bar(stage));
+            if (kb + 1 == k_blocks) umma_commit_pair(tfull_bar(buf));
           }
-          umma_commit_pair(empty_bar(stage));
-          if (++stage == kStages2) { stage = 0; phase ^= 1u; }
-        }
-        if (alive) umma_commit_pair(tfull_bar(buf));
-      }
-    } else if (lane == 0 && kGather) {
-      // ------------------------------ forwarder (peer) ---------------------------
-      // this block's gathered rows of a stage have landed: make them visible to the tensor cores and
-      // tell the leader, whose MMA reads them
-      int stage = 0;
-      uint32_t phase = 0;
-      bool alive = true;
-      for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded(gdone_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
-          fence_async_proxy();
-          mbar_arrive_cluster(map_to_rank(full_bar(stage), 0));
+          __syncwarp();
           if (++stage == kStages2) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp >= 4) {
     // ------------------------------ epilogue (both blocks) ---------------------
-    const int ew = (warp - 4) & 3;
-    const int eh = (warp - 4) >> 2;
+    const int q = (warp - 4) & 3;                  // TMEM lanes 32 q .. 32 q + 31
+    const int h = (warp - 4) >> 2;                 // which of the tile's 32-row batches
+    uint8_t* my_stage = store_stage + (warp - 4) * kStoreStage2Bytes;
     int local = 0;
     bool alive = true;
+    // three units ahead: description; two: the rows' flat indices; one: their scales
+    auto flats = [&](const Unit& u, int* flat) {
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const int r = 32 * h + 128 * b + lane;
+        flat[b] = (MODE == kGemmExpertDown && r < u.rows) ? g.sorted_rows[u.row0 + r] : -1;
+      }
+    };
+    auto scales = [&](const int* flat, float* scale) {
+#pragma unroll
+      for (int b = 0; b < 2; ++b) scale[b] = (MODE == kGemmExpertDown && flat[b] >= 0) ? g.row_scale[flat[b]] : 0.0f;
+    };
+    Unit u1 = describe(pair), u2 = describe(pair + n_pairs), u3 = describe(pair + 2 * n_pairs);
+    int flat[2];
+    float scale[2];
+    flats(u1, flat);
+    scales(flat, scale);
+    flats(u2, flat);
     for (int unit = pair; unit < total_units && alive; unit += n_pairs, ++local) {
-      int chunk, expert, row0, rows, tile_last;
-      unit_tile(unit, chunk, expert, row0, rows, tile_last);
+      const Unit u = u1;
+      const float scale_now[2] = {scale[0], scale[1]};
+      scales(flat, scale);
+      flats(u3, flat);
+      u1 = u2;
+      u2 = u3;
+      u3 = describe(unit + 3 * n_pairs);
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
       if (!mbar_wait_bounded(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
       tc_fence_after();
-      if (rows > 0)
-        drain_accumulator<MODE>(g, pb, tmem_base, buf, ew, eh, lane, store_stage + (warp - 4) * kStoreStageBytes,
-                                chunk, row0, rows);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_rank(tempty_bar(buf), 0));
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * kPairRows);
+      drain_transposed<MODE>(g, pb, taddr, static_cast<int>(rank), q, h, lane, my_stage, u.chunk, u.row0, u.rows,
+                             scale_now, map_to_rank(tempty_bar(buf), 0));
     }
   }
   tc_fence_before();
@@ -809,14 +1039,13 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// 2-D BF16 tensor [rows, cols] row-major, box 64 columns x box_rows rows (128 for tile loads,
-// 1 for gather4 loads), 128-byte swizzle.  A descriptor depends only on the base address and these
-// numbers, and a layer's weights and the workspace keep their addresses from bind to release, so the
-// encoded descriptors are kept: a prefill layer asks for 18 of them per call, always the same ones.
+// Descriptors of BF16 tensors, 128-byte swizzle.  A descriptor depends only on the base address and these numbers,
+// and a layer's weights and the workspace keep their addresses from bind to release, so the encoded descriptors are
+// kept: a prefill layer asks for about twenty of them per call, always the same ones.
 struct MapKey {
   const void* base;
   uint64_t rows, cols, pitch;
-  uint32_t box_rows;
+  uint32_t box_rows;        // rows of the tile; 0: the 5-D view of make_gate_up_map
   bool operator==(const MapKey& o) const {
     return base == o.base && rows == o.rows && cols == o.cols && pitch == o.pitch && box_rows == o.box_rows;
   }
@@ -830,11 +1059,10 @@ struct MapKeyHash {
   }
 };
 
-bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_elems,
-              uint32_t box_rows = kBM) {
+bool cached_map(CUtensorMap* map, const MapKey& key, cuuint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides,
+                const cuuint32_t* box) {
   static std::mutex mutex;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  const MapKey key{base, rows, cols, pitch_elems, box_rows};
   {
     std::lock_guard<std::mutex> lock(mutex);
     const auto hit = cache.find(key);
@@ -842,11 +1070,8 @@ bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, 
   }
   PFN_cuTensorMapEncodeTiled_v12000 encode = encode_fn();
   if (encode == nullptr) return false;
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {pitch_elems * 2};
-  const cuuint32_t box[2] = {kBK, box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+  const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(key.base), dims, strides, box, elem,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
@@ -854,6 +1079,25 @@ bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, 
   if (cache.size() >= 8192) cache.clear();      // a host that keeps binding new tensors: start over rather than grow
   cache.emplace(key, *map);
   return true;
+}
+
+// [rows, cols] row-major, box of 64 columns x box_rows rows
+bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_elems,
+              uint32_t box_rows = kBM) {
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {pitch_elems * 2};
+  const cuuint32_t box[2] = {kBK, box_rows};
+  return cached_map(map, MapKey{base, rows, cols, pitch_elems, box_rows}, 2, dims, strides, box);
+}
+
+// [experts, 2 (gate, up), n, k] seen as (k, 16 rows, gate / up, groups of 16 rows, expert); the box takes 64 columns of
+// four groups, gate and up: 128 rows that arrive as 16 gate rows, the 16 up rows that belong to them, 16 gate rows, ...,
+// so that one warp of the transposed epilogue holds both halves of its sixteen outputs.
+bool make_gate_up_map(CUtensorMap* map, const void* base, uint64_t experts, uint64_t n, uint64_t k) {
+  const cuuint64_t dims[5] = {k, 16, 2, n / 16, experts};
+  const cuuint64_t strides[4] = {k * 2, n * k * 2, 16 * k * 2, 2 * n * k * 2};
+  const cuuint32_t box[5] = {kBK, 16, 2, 4, 1};
+  return cached_map(map, MapKey{base, experts * 2 * n, k, k, 0}, 5, dims, strides, box);
 }
 
 template <int MODE, bool kGather = false>
@@ -865,12 +1109,12 @@ cudaError_t launch_mode(const TcMaps& maps, const TcProblem& pb, int grid, cudaS
 
 // two-SM form: clusters of two blocks, launched like launch_pdl
 template <int MODE, bool kGather>
-cudaError_t launch_pair_mode(const TcMaps& maps, const TcProblem& pb, int grid, cudaStream_t stream) {
-  const cudaError_t e = opt_in_dynamic_smem<grouped_gemm_tc2_kernel<MODE, kGather>>(kTc2SmemBytes);
+cudaError_t launch_pair_mode(const TcPairMaps& maps, const TcProblem& pb, int grid, cudaStream_t stream) {
+  const cudaError_t e = opt_in_dynamic_smem<grouped_gemm_pair_kernel<MODE, kGather>>(kTc2SmemBytes);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(grid & ~1);
-  config.blockDim = dim3(kTcThreads);
+  config.blockDim = dim3(kPairThreads);
   config.dynamicSmemBytes = kTc2SmemBytes;
   config.stream = stream;
   cudaLaunchAttribute attributes[2];
@@ -882,7 +1126,32 @@ cudaError_t launch_pair_mode(const TcMaps& maps, const TcProblem& pb, int grid, 
   attributes[1].val.programmaticStreamSerializationAllowed = t_pdl_relaxed ? 1 : 0;
   config.attrs = attributes;
   config.numAttrs = 2;
-  return cudaLaunchKernelEx(&config, grouped_gemm_tc2_kernel<MODE, kGather>, maps, pb);
+  return cudaLaunchKernelEx(&config, grouped_gemm_pair_kernel<MODE, kGather>, maps, pb);
+}
+
+cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extra, TcProblem pb, cudaStream_t stream) {
+  TcPairMaps maps;
+  const uint64_t experts = static_cast<uint64_t>(extra.experts_in_b);
+  const bool gather = mode == kGemmExpertGateUp && g.gather_src != nullptr;
+  bool ok = true;
+  if (mode == kGemmExpertGateUp) {
+    pb.n_chunks = g.n / (kPairN / 2);
+    ok = make_gate_up_map(&maps.w, g.b0, experts, g.n, g.k);
+  } else {
+    pb.n_chunks = (g.n + kPairN - 1) / kPairN;
+    pb.b_rows_per_expert = g.n;
+    ok = make_map(&maps.w, g.b0, (mode == kGemmExpertDown ? experts : 1) * static_cast<uint64_t>(g.n), g.k, g.k);
+  }
+  if (ok && gather) ok = make_map(&maps.rows[0], g.gather_src, extra.a_rows, g.k, g.lda, 1u);
+  for (int b = 0; ok && !gather && b < 4; ++b)
+    ok = make_map(&maps.rows[b], g.a, extra.a_rows, g.k, g.lda, 16u << b);
+  if (!ok) return cudaErrorNotSupported;
+  if (mode == kGemmExpertGateUp)
+    return gather ? launch_pair_mode<kGemmExpertGateUp, true>(maps, pb, extra.sm_count, stream)
+                  : launch_pair_mode<kGemmExpertGateUp, false>(maps, pb, extra.sm_count, stream);
+  if (mode == kGemmExpertDown) return launch_pair_mode<kGemmExpertDown, false>(maps, pb, extra.sm_count, stream);
+  if (mode == kGemmPlain) return launch_pair_mode<kGemmPlain, false>(maps, pb, extra.sm_count, stream);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace
@@ -891,15 +1160,15 @@ cudaError_t launch_grouped_gemm_tc(GemmMode mode, const GroupedGemm& g, const Tc
                                    cudaStream_t stream) {
   if (g.max_tiles <= 0) return cudaSuccess;
   if (g.k % kBK != 0 || extra.status == nullptr) return cudaErrorInvalidValue;
+  const bool gather = (mode == kGemmExpertGateUp && g.gather_src != nullptr);
+  if (gather && g.sorted_rows == nullptr) return cudaErrorInvalidValue;
   TcMaps maps;
   TcProblem pb{};
   pb.g = g;
   pb.status = extra.status;
   pb.n_valid = g.n;
-  const bool dual = (mode == kGemmExpertGateUp || mode == kGemmSharedGateUp);
+  if (extra.pair) return launch_pair(mode, g, extra, pb, stream);
   const uint64_t experts = static_cast<uint64_t>(extra.experts_in_b);
-  const bool gather = (mode == kGemmExpertGateUp && g.gather_src != nullptr);
-  if (gather && g.sorted_rows == nullptr) return cudaErrorInvalidValue;
   bool ok = make_map(&maps.a, gather ? g.gather_src : g.a, extra.a_rows, static_cast<uint64_t>(g.k),
                      static_cast<uint64_t>(g.lda), gather ? 1u : static_cast<uint32_t>(kBM));
   pb.a_rows = static_cast<int>(extra.a_rows);
@@ -921,16 +1190,8 @@ cudaError_t launch_grouped_gemm_tc(GemmMode mode, const GroupedGemm& g, const Tc
     ok = ok && make_map(&maps.b0, g.b0, (mode == kGemmExpertDown ? experts : 1) * static_cast<uint64_t>(g.n), g.k, g.k);
     maps.b1 = maps.b0;
   }
-  (void)dual;
   if (!ok) return cudaErrorNotSupported;
   const int grid = extra.sm_count;
-  if (extra.pair && g.tile_expert != nullptr && g.parts <= 1) {
-    if (mode == kGemmExpertGateUp)
-      return gather ? launch_pair_mode<kGemmExpertGateUp, true>(maps, pb, grid, stream)
-                    : launch_pair_mode<kGemmExpertGateUp, false>(maps, pb, grid, stream);
-    if (mode == kGemmExpertDown) return launch_pair_mode<kGemmExpertDown, false>(maps, pb, grid, stream);
-    return cudaErrorInvalidValue;      // the plan holds 256-row tiles: only the two-SM kernels can take them
-  }
   switch (mode) {
     case kGemmExpertGateUp:
       return gather ? launch_mode<kGemmExpertGateUp, true>(maps, pb, grid, stream)

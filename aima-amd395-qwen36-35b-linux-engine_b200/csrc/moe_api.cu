@@ -378,7 +378,7 @@ AIMA_EXPORT int aima_moe_prepare(const aima_moe_config* config, aima_moe_handle*
     handle->prefill.exact_router = (config->flags & AIMA_MOE_FLAG_EXACT_ROUTER) != 0;
     handle->prefill.router_audit_stride = (config->flags & AIMA_MOE_FLAG_AUDIT_ROUTER) != 0 ? 64 : 0;
     handle->prefill.fused_dispatch = (config->flags & AIMA_MOE_FLAG_MATERIALIZED_DISPATCH) == 0;
-    handle->prefill.pair_products = (config->flags & AIMA_MOE_FLAG_TWO_SM_PRODUCTS) != 0 && config->world == 1;
+    handle->prefill.pair_products = config->world == 1;
     handle->prefill.ep_parts = (config->flags & AIMA_MOE_FLAG_EP_PIPELINE_4)   ? 4
                                : (config->flags & AIMA_MOE_FLAG_EP_PIPELINE_2) ? 2
                                                                                : 1;
@@ -733,6 +733,7 @@ AIMA_EXPORT int aima_moe_gemm_bf16_launch(aima_moe_handle* handle, const void* a
   g.c = static_cast<__nv_bfloat16*>(d); g.ldc = static_cast<int>(n);
   TcExtra extra{};
   extra.status = handle->status; extra.sm_count = handle->sm_count; extra.a_rows = m; extra.experts_in_b = 1;
+  extra.pair = true;
   const cudaError_t error = launch_grouped_gemm_tc(kGemmPlain, g, extra, static_cast<cudaStream_t>(stream));
   if (error != cudaSuccess) return fail_cuda(error, "launch grouped_gemm_tc_kernel (plain)");
   handle->last_stream = static_cast<cudaStream_t>(stream);

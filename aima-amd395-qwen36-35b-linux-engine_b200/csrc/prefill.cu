@@ -498,6 +498,16 @@ plan_scan_kernel(int32_t* __restrict__ unit_counts, int units, int32_t* __restri
   if (lane == 0) expert_counts[e] = running;
 }
 
+// Rows per tile of an expert with `count` rows.  128-row tiles (one-SM products) are filled one after the other.  Tiles
+// of up to 256 rows (two-SM products, whose cost goes with the rows in steps of 32) are made equally large: 272 rows
+// are 160 + 112, not 256 + 16, so that the last tile does not stream the expert's weights for a handful of rows.  All
+// tiles but the last are full multiples of 32, and the last one is never empty (the tiles before it hold at most
+// 256 (n - 1) < count rows).
+__device__ __forceinline__ int rows_per_tile(int count, int n_tiles, int tile_cap) {
+  if (tile_cap <= kTileRows || n_tiles <= 1) return tile_cap;
+  return ((count + n_tiles - 1) / n_tiles + 31) & ~31;
+}
+
 // Exclusive offsets of the 256 experts from their counts, in shared memory (all 256 threads of a
 // block take part); thread 0 .. 255 returns with offsets[0 .. 256] and tile_base[0 .. 256] filled.
 __device__ __forceinline__ int expert_offsets_in_block(const int32_t* __restrict__ expert_counts, int tile_cap,
@@ -557,11 +567,12 @@ plan_scatter_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert
       *padded_rows = padded;
     }
     const int n_tiles = tile_base[e + 1] - tile_base[e];
+    const int height = rows_per_tile(count, n_tiles, tile_cap);
     for (int t = 0; t < n_tiles; ++t) {
       const int index = tile_base[e] + t;
       tile_expert[index] = e;
-      tile_row0[index] = offsets[e] + t * tile_cap;
-      tile_rows[index] = min(tile_cap, count - t * tile_cap);
+      tile_row0[index] = offsets[e] + t * height;
+      tile_rows[index] = min(height, count - t * height);
     }
   }
   const int warp = threadIdx.x >> 5;
@@ -1017,6 +1028,8 @@ __global__ void forced_routing_kernel(const int32_t* __restrict__ ids, const __n
   topk_scores[i] = 0.0f;
 }
 
+constexpr int kGatherMaxTokens = 3584;     // between the two sizes where the two dispatch forms cross
+
 int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStream_t stream,
                          int* launches, char* error, size_t error_bytes) {
   const int T = call.tokens;
@@ -1103,19 +1116,18 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   if ((code = cudaEventRecord(ws->join_event, side)) != cudaSuccess)
     return set_error(error, error_bytes, code, "join event of the shared-expert stream");
 
-  // Expert products: one block per 128-row tile; the two-SM form (a pair of blocks per 256-row tile) behind a
-  // flag.  Both stream every expert's weights once at T = 8192 and are bound by that stream -- 302 / 170 us
-  // (gate_up / down) against 308 / 218 us for the pair with materialised rows, and the pair's row gather has to
-  // cross to the leader's barrier, which doubles its gate_up time -- so the simpler form is the default.
+  // Expert products: the two-SM form with tiles of up to 256 rows (128-row tiles for the CUDA-core cross-check)
   const bool pair_products = ws->pair_products && !ws->use_simt_gemm;
   if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, stream, &count, pair_products ? 2 * kTileRows : kTileRows)) !=
       cudaSuccess)
     return set_error(error, error_bytes, code, "dispatch plan");
 
-  // Dispatch is fused into the gate_up kernel: two of its warps fetch each tile's rows by token index
-  // with asynchronous 16-byte copies (0.689 vs 0.745 ms per T = 8192 layer).  The materialised copy in
-  // expert order, read by tiled TMA loads, remains for the CUDA-core cross-check and behind a flag.
-  const bool fused_dispatch = ws->fused_dispatch && !ws->use_simt_gemm;
+  // Dispatch.  Up to kGatherMaxTokens the gate_up kernel fetches each tile's rows by token index itself (TMA gather4);
+  // with more tokens the rows are copied into expert order first and read by tile loads.  gather4 moves four rows per
+  // ~45 cycles, which the weight stream hides while a tile has few rows and not when it has 256: sustained us per layer,
+  // gather4 / copied rows, balanced routing: 331 / 348 at 1024 tokens, 379 / 420 at 2048, 451 / 468 at 3072, 518 / 505 at
+  // 4096, 645 / 610 at 6144, 855 / 771 at 8192.
+  const bool fused_dispatch = ws->fused_dispatch && !ws->use_simt_gemm && T <= kGatherMaxTokens;
   if (!fused_dispatch) {
     gather_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(call.h2), ws->sorted_rows, rows, ws->gathered);
