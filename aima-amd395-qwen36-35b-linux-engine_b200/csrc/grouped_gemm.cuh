@@ -69,12 +69,24 @@ struct GroupedGemm {
   int scatter_tokens_per_rank;
 };
 
+// The shared expert's half of an expert product, in the same launch of the two-SM form (rows = 0: none).  Same n, k and
+// ldc as the routed product; the rounding points are those of kGemmSharedGateUp / kGemmSharedDown.
+struct SharedProblem {
+  int rows;
+  const __nv_bfloat16* a;      // [rows, k]
+  const __nv_bfloat16* b0;     // gate matrix, or the down matrix
+  const __nv_bfloat16* b1;     // up matrix
+  __nv_bfloat16* c;
+  const float* row_scale;      // down: the sigmoid gate per row
+};
+
 // What the tensor-core launcher needs beyond the problem itself.
 struct TcExtra {
   int* status;          // device status word for bounded-wait expiry
   int sm_count;         // persistent grid size
   uint64_t a_rows;      // rows of the A allocation (TMA bounds; reads beyond are zero-filled)
   int experts_in_b;     // experts held in b0 (expert modes), else 1
+  SharedProblem shared = {};    // two-SM form, expert modes
   bool pair = false;    // expert modes: two-SM form; the plan's tiles then hold up to 256 rows
 };
 

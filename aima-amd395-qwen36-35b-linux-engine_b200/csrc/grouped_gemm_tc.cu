@@ -62,6 +62,10 @@ struct TcProblem {
   int n_valid;            // valid output columns (plain mode masks beyond)
   int a_rows;             // rows of the A tensor (fused dispatch: first out-of-range row index)
   int* status;            // device status word
+  // two-SM form
+  int dense_tile;         // dense modes: rows per tile
+  SharedProblem shared;   // expert modes: the shared expert's rows, in the same launch
+  int shared_tiles;
 };
 
 // ---- PTX wrappers ---------------------------------------------------------
@@ -557,6 +561,8 @@ static_assert(kTc2SmemBytes <= 227 * 1024, "two-SM product kernel exceeds 227 KB
 
 struct TcPairMaps {
   CUtensorMap w;        // weights: [rows, k] box 64 x 128, or the 5-D view of a gate_up tensor (make_gate_up_map)
+  CUtensorMap shared_w[2];     // the shared expert's gate and up matrices (box 64 x 16), or its down matrix (box 64 x 128)
+  CUtensorMap shared_rows[4];  // its rows, like `rows`
   CUtensorMap rows[4];  // A: boxes of 64 x 16, 32, 64 and 128 rows (any multiple of 16 rows is at most four loads);
                         // gather: rows[0] is the box of one row
 };
@@ -658,8 +664,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // registers.
 template <int MODE>
 __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcProblem& pb, uint32_t taddr, int rank,
-                                                 int q, int h, int lane, uint8_t* stage, int chunk, int row0, int rows,
-                                                 const float* scale, uint32_t drained) {
+                                                 int q, int h, int lane, uint8_t* stage, int chunk, bool shared, int row0,
+                                                 int rows, const float* scale, uint32_t drained) {
   constexpr int kStep = 32 * (kPairEpilogueWarps / 4);
   const uint32_t stage_s = smem_u32(stage);
   auto release = [&]() {
@@ -673,7 +679,7 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
   }
   if (MODE == kGemmExpertGateUp) {
     // lanes 0-15 of the quarter are gate columns, lanes 16-31 the up columns of the same sixteen outputs
-    __nv_bfloat16* dst = g.c + static_cast<size_t>(row0) * g.ldc + chunk * (kPairN / 2) + rank * 64 + 16 * q;
+    __nv_bfloat16* dst = (shared ? pb.shared.c : g.c) + static_cast<size_t>(row0) * g.ldc + chunk * (kPairN / 2) + rank * 64 + 16 * q;
 #pragma unroll 1
     for (int c0 = 32 * h; c0 < rows; c0 += kStep) {
       uint32_t gr[16], ur[16];
@@ -689,7 +695,8 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
         for (int c = 0; c < 2; ++c) {
           const float gate = round_bf16(__uint_as_float(gr[2 * i + c]));
           const float up = round_bf16(__uint_as_float(ur[2 * i + c]));
-          v[c] = __fmul_rn(round_bf16(det_silu(gate)), up);
+          const float s = det_silu(gate);
+          v[c] = __fmul_rn(shared ? s : round_bf16(s), up);
         }
         packed[i] = pack_bf16(v[0], v[1]);
       }
@@ -711,9 +718,24 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
       }
       __syncwarp();
     }
+  } else if (MODE == kGemmPlainF32) {
+    // FP32 as it is: a row's 32 columns are one 128-byte store
+    const int col0 = chunk * kPairN + rank * 128 + 32 * q;
+    float* dst = g.c_f32 + static_cast<size_t>(row0) * g.ldc + col0 + lane;
+#pragma unroll 1
+    for (int c0 = 32 * h; c0 < rows; c0 += kStep) {
+      uint32_t r[32];
+      tmem_ld32(taddr + c0, r);
+      tmem_ld_wait();
+      if (c0 + kStep >= rows) release();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (c0 + j < rows && col0 + lane < pb.n_valid) dst[static_cast<size_t>(c0 + j) * g.ldc] = __uint_as_float(r[j]);
+      }
+    }
   } else {
     const int col0 = chunk * kPairN + rank * 128 + 32 * q;
-    __nv_bfloat16* dst = g.c + static_cast<size_t>(row0) * g.ldc + col0;
+    __nv_bfloat16* dst = (MODE == kGemmExpertDown && shared ? pb.shared.c : g.c) + static_cast<size_t>(row0) * g.ldc + col0;
     const bool piece_ok = col0 + 8 * (lane & 3) < pb.n_valid;
 #pragma unroll
     for (int b = 0; b < kPairRows / kStep; ++b) {
@@ -736,7 +758,10 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
           for (int m = 0; m < 4; ++m) {
             float lo = __uint_as_float(r[16 * (m >> 1) + 4 * i + 2 * (m & 1)]);
             float hi = __uint_as_float(r[16 * (m >> 1) + 4 * i + 2 * (m & 1) + 1]);
-            if (MODE == kGemmExpertDown) { lo = __fmul_rn(lo, s0); hi = __fmul_rn(hi, s1); }
+            if (MODE == kGemmExpertDown) {
+              lo = __fmul_rn(shared ? round_bf16(lo) : lo, s0);
+              hi = __fmul_rn(shared ? round_bf16(hi) : hi, s1);
+            }
             packed[m] = pack_bf16(lo, hi);
           }
           const int row = 8 * i + (lane & 7);
@@ -759,7 +784,7 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
 template <int MODE, bool kGather>
 __global__ void __launch_bounds__(kPairThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProblem pb) {
-  static_assert(MODE == kGemmExpertGateUp || MODE == kGemmExpertDown || MODE == kGemmPlain, "modes of the two-SM form");
+  static_assert(MODE != kGemmSharedGateUp && MODE != kGemmSharedDown, "the shared expert runs inside the expert modes");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -802,7 +827,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
 
   pdl_enter();
 
-  const int n_tiles = g.tile_count != nullptr ? *g.tile_count : (g.dense_rows + kPairRows - 1) / kPairRows;
+  constexpr bool kDense = MODE == kGemmPlain || MODE == kGemmPlainF32;
+  const int n_tiles = kDense ? (g.dense_rows + pb.dense_tile - 1) / pb.dense_tile : pb.shared_tiles + *g.tile_count;
   // as in the one-SM kernel; the leader samples the status for the pair
   volatile int* poison_slot = abort_flag + 1;
   if (threadIdx.x == 0 && leader) {
@@ -818,7 +844,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   const int pair = blockIdx.x >> 1;
   const int k_blocks = g.k / kBK;
 
-  // unit -> chunk of 256 weight rows, expert, first row and number of rows (1 .. 256) of the tile.  Every role asks for
+  // unit -> chunk of 256 weight rows, expert (-1: the shared expert, whose tiles come first), first row and number of
+  // rows (1 .. 256) of the tile.  Every role asks for
   // the unit after the one it works on (or later), so that these loads, and in the epilogue the two that follow from
   // them, are never waited for between two units: in the down product, whose units are eight stages long, they cost
   // half of a unit's time.
@@ -828,20 +855,27 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   auto describe = [&](int unit) {
     Unit u{0, 0, 0, 0};
     if (unit >= total_units) return u;
-    if (MODE == kGemmPlain) {
+    if (kDense) {
       // eight row tiles x all chunks at a time: the pairs that run together then share both operands in L2
       const int band = unit / (kPlainBand * pb.n_chunks);
       const int height = min(kPlainBand, n_tiles - band * kPlainBand);
       const int within = unit - band * kPlainBand * pb.n_chunks;
       u.chunk = within / height;
-      u.row0 = (band * kPlainBand + within - u.chunk * height) * kPairRows;
-      u.rows = min(kPairRows, g.dense_rows - u.row0);
+      u.row0 = (band * kPlainBand + within - u.chunk * height) * pb.dense_tile;
+      u.rows = min(pb.dense_tile, g.dense_rows - u.row0);
     } else {
-      const int tile = unit / pb.n_chunks;
+      int tile = unit / pb.n_chunks;
       u.chunk = unit - tile * pb.n_chunks;
-      u.expert = g.tile_expert[tile] - g.expert_base;
-      u.row0 = g.tile_row0[tile];
-      u.rows = g.tile_rows[tile];
+      if (tile < pb.shared_tiles) {
+        u.expert = -1;
+        u.row0 = tile * pb.dense_tile;
+        u.rows = min(pb.dense_tile, pb.shared.rows - u.row0);
+      } else {
+        tile -= pb.shared_tiles;
+        u.expert = g.tile_expert[tile] - g.expert_base;
+        u.row0 = g.tile_row0[tile];
+        u.rows = g.tile_rows[tile];
+      }
     }
     return u;
   };
@@ -857,6 +891,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
       const Unit u = next;
       next = describe(unit + n_pairs);
+      const bool shared = !kDense && u.expert < 0;
       const int half = pair_width(u.rows) / 2;      // a multiple of 16
       const int my_row0 = u.row0 + static_cast<int>(rank) * half;
       const int w_row = u.expert * pb.b_rows_per_expert + u.chunk * kPairN + static_cast<int>(rank) * 128;
@@ -869,8 +904,16 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
           const uint32_t w_dst = smem_base + stage * kStage2Bytes;
           const uint32_t leader_full = leader_full0 + 8u * stage;
           if (leader) mbar_arrive_expect_tx(full_bar(stage), stage_bytes);
-          if (MODE == kGemmExpertGateUp)
+          if (MODE == kGemmExpertGateUp && shared) {
+            // two tensors: the interleaving of the 5-D view, sixteen rows at a time
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              tma_load_2d_pair(w_dst + i * (16 * kBK * 2), &maps.shared_w[i & 1], kb * kBK,
+                               u.chunk * (kPairN / 2) + static_cast<int>(rank) * 64 + 16 * (i >> 1), leader_full);
+          } else if (MODE == kGemmExpertGateUp)
             tma_load_5d_pair(w_dst, &maps.w, kb * kBK, u.chunk * 8 + static_cast<int>(rank) * 4, u.expert, leader_full);
+          else if (MODE == kGemmExpertDown && shared)
+            tma_load_2d_pair(w_dst, &maps.shared_w[0], kb * kBK, u.chunk * kPairN + static_cast<int>(rank) * 128, leader_full);
           else
             tma_load_2d_pair(w_dst, &maps.w, kb * kBK, w_row, leader_full);
           if (!kGather) {
@@ -879,7 +922,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
             for (int b = 3; b >= 0; --b) {
               const int size = 16 << b;
               if (half & size) {
-                tma_load_2d_pair(w_dst + kStage2ABytes + done * (kBK * 2), &maps.rows[b], kb * kBK, my_row0 + done, leader_full);
+                tma_load_2d_pair(w_dst + kStage2ABytes + done * (kBK * 2), shared ? &maps.shared_rows[b] : &maps.rows[b],
+                                 kb * kBK, my_row0 + done, leader_full);
                 done += size;
               }
             }
@@ -905,11 +949,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       const int mine = max(0, min(half, u.rows - static_cast<int>(rank) * half));
       int4 t = make_int4(0, 0, 0, 0);
       if (4 * lane < mine) {
-        const int32_t* sorted = g.sorted_rows + u.row0 + static_cast<int>(rank) * half;
-        t.x = sorted[4 * lane];
-        t.y = sorted[min(4 * lane + 1, mine - 1)];
-        t.z = sorted[min(4 * lane + 2, mine - 1)];
-        t.w = sorted[min(4 * lane + 3, mine - 1)];
+        const int first = u.row0 + static_cast<int>(rank) * half;
+        auto flat = [&](int r) { return u.expert < 0 ? (first + r) << 3 : g.sorted_rows[first + r]; };
+        t.x = flat(4 * lane);
+        t.y = flat(min(4 * lane + 1, mine - 1));
+        t.z = flat(min(4 * lane + 2, mine - 1));
+        t.w = flat(min(4 * lane + 3, mine - 1));
       }
       return t;
     };
@@ -984,17 +1029,23 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     uint8_t* my_stage = store_stage + (warp - 4) * kStoreStage2Bytes;
     int local = 0;
     bool alive = true;
+    constexpr int kSharedRow = 1 << 30;            // flat index of row 0 of the shared expert
     // three units ahead: description; two: the rows' flat indices; one: their scales
     auto flats = [&](const Unit& u, int* flat) {
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
         const int r = 32 * h + 128 * b + lane;
-        flat[b] = (MODE == kGemmExpertDown && r < u.rows) ? g.sorted_rows[u.row0 + r] : -1;
+        flat[b] = -1;
+        if (MODE == kGemmExpertDown && r < u.rows) flat[b] = u.expert < 0 ? kSharedRow + u.row0 + r : g.sorted_rows[u.row0 + r];
       }
     };
     auto scales = [&](const int* flat, float* scale) {
 #pragma unroll
-      for (int b = 0; b < 2; ++b) scale[b] = (MODE == kGemmExpertDown && flat[b] >= 0) ? g.row_scale[flat[b]] : 0.0f;
+      for (int b = 0; b < 2; ++b) {
+        scale[b] = 0.0f;
+        if (MODE == kGemmExpertDown && flat[b] >= 0)
+          scale[b] = flat[b] >= kSharedRow ? pb.shared.row_scale[flat[b] - kSharedRow] : g.row_scale[flat[b]];
+      }
     };
     Unit u1 = describe(pair), u2 = describe(pair + n_pairs), u3 = describe(pair + 2 * n_pairs);
     int flat[2];
@@ -1015,8 +1066,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       if (!mbar_wait_bounded(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * kPairRows);
-      drain_transposed<MODE>(g, pb, taddr, static_cast<int>(rank), q, h, lane, my_stage, u.chunk, u.row0, u.rows,
-                             scale_now, map_to_rank(tempty_bar(buf), 0));
+      drain_transposed<MODE>(g, pb, taddr, static_cast<int>(rank), q, h, lane, my_stage, u.chunk, u.expert < 0, u.row0,
+                             u.rows, scale_now, map_to_rank(tempty_bar(buf), 0));
     }
   }
   tc_fence_before();
@@ -1129,6 +1180,24 @@ cudaError_t launch_pair_mode(const TcPairMaps& maps, const TcProblem& pb, int gr
   return cudaLaunchKernelEx(&config, grouped_gemm_pair_kernel<MODE, kGather>, maps, pb);
 }
 
+// Rows per tile of a dense product over `chunks` chunks of 256 columns: the height whose last wave of units wastes
+// least.  A unit's time goes with its rows, in steps of 32, but not below what issuing a stage costs (about 128 rows);
+// smaller tiles then only help to spread a product over the chip.  Router logits (one chunk) at 1024 / 8192 rows: 32- /
+// 128-row tiles.
+int dense_tile_rows(int rows, int chunks, int pairs) {
+  int best = kPairRows;
+  long long best_cost = -1;
+  for (int height = kPairRows; height >= 32; height -= 32) {
+    const long long units = static_cast<long long>((rows + height - 1) / height) * chunks;
+    const long long cost = (units + pairs - 1) / pairs * ((height > 128 ? height : 128) + 16);
+    if (best_cost < 0 || cost < best_cost || (cost == best_cost && units <= pairs)) {
+      best = height;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extra, TcProblem pb, cudaStream_t stream) {
   TcPairMaps maps;
   const uint64_t experts = static_cast<uint64_t>(extra.experts_in_b);
@@ -1145,12 +1214,30 @@ cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extr
   if (ok && gather) ok = make_map(&maps.rows[0], g.gather_src, extra.a_rows, g.k, g.lda, 1u);
   for (int b = 0; ok && !gather && b < 4; ++b)
     ok = make_map(&maps.rows[b], g.a, extra.a_rows, g.k, g.lda, 16u << b);
+  const SharedProblem& shared = extra.shared;
+  if (mode == kGemmPlain || mode == kGemmPlainF32) {
+    pb.dense_tile = dense_tile_rows(g.dense_rows, pb.n_chunks, extra.sm_count / 2);
+  } else if (shared.rows > 0) {
+    // the shared expert's rows in equal tiles
+    const int tiles = (shared.rows + kPairRows - 1) / kPairRows;
+    pb.dense_tile = pair_width((shared.rows + tiles - 1) / tiles);
+    pb.shared_tiles = tiles;
+    pb.shared = shared;
+    if (mode == kGemmExpertGateUp) {
+      ok = ok && make_map(&maps.shared_w[0], shared.b0, g.n, g.k, g.k, 16) && make_map(&maps.shared_w[1], shared.b1, g.n, g.k, g.k, 16);
+    } else {
+      ok = ok && make_map(&maps.shared_w[0], shared.b0, g.n, g.k, g.k);
+    }
+    for (int b = 0; ok && !gather && b < 4; ++b)
+      ok = make_map(&maps.shared_rows[b], shared.a, shared.rows, g.k, g.k, 16u << b);
+  }
   if (!ok) return cudaErrorNotSupported;
   if (mode == kGemmExpertGateUp)
     return gather ? launch_pair_mode<kGemmExpertGateUp, true>(maps, pb, extra.sm_count, stream)
                   : launch_pair_mode<kGemmExpertGateUp, false>(maps, pb, extra.sm_count, stream);
   if (mode == kGemmExpertDown) return launch_pair_mode<kGemmExpertDown, false>(maps, pb, extra.sm_count, stream);
   if (mode == kGemmPlain) return launch_pair_mode<kGemmPlain, false>(maps, pb, extra.sm_count, stream);
+  if (mode == kGemmPlainF32) return launch_pair_mode<kGemmPlainF32, false>(maps, pb, extra.sm_count, stream);
   return cudaErrorInvalidValue;
 }
 

@@ -29,25 +29,29 @@ __device__ __forceinline__ float key_value(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// 8th largest of the 256 values a warp holds (8 per lane), counting repeats.
+// 8th largest of the 256 values a warp holds (8 per lane), counting repeats.  Every lane sorts its eight keys once
+// (Batcher's odd-even merge network), so that a round is one warp maximum and a shift on the lane that held it.
 __device__ __forceinline__ float warp_eighth_largest(const float* v, int lane) {
   uint32_t k[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) k[q] = order_key(v[q]);
+  constexpr int kPairs[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7}, {1, 2}, {5, 6},
+                                 {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
+#pragma unroll
+  for (int p = 0; p < 19; ++p) {
+    const uint32_t hi = max(k[kPairs[p][0]], k[kPairs[p][1]]);
+    k[kPairs[p][1]] = min(k[kPairs[p][0]], k[kPairs[p][1]]);
+    k[kPairs[p][0]] = hi;
+  }
   uint32_t best = 0;
 #pragma unroll
   for (int r = 0; r < kTopK; ++r) {
-    uint32_t local = k[0];
-#pragma unroll
-    for (int q = 1; q < 8; ++q) local = max(local, k[q]);
-    best = __reduce_max_sync(0xffffffffu, local);
-    const unsigned owners = __ballot_sync(0xffffffffu, local == best);
+    best = __reduce_max_sync(0xffffffffu, k[0]);
+    const unsigned owners = __ballot_sync(0xffffffffu, k[0] == best);
     if (lane == __ffs(owners) - 1) {
-      bool removed = false;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        if (!removed && k[q] == best) { k[q] = 0u; removed = true; }
-      }
+      for (int q = 0; q < 7; ++q) k[q] = k[q + 1];
+      k[7] = 0u;
     }
   }
   return key_value(best);
@@ -55,12 +59,11 @@ __device__ __forceinline__ float warp_eighth_largest(const float* v, int lane) {
 
 // The reference's prefill selection on the final (BF16-rounded) logits of one
 // token held as v[q] = logit of expert 32 q + lane: threshold, gather in expert
-// order, fixed bitonic network, softmax; lanes 0..7 write slot `lane`.
-__device__ __forceinline__ int route_token(const float* v, int lane, float* sel_v, int* sel_i,
+// order, fixed bitonic network, softmax; lanes 0..7 write slot `lane`.  `threshold` is the 8th largest of the values.
+__device__ __forceinline__ int route_token(const float* v, float threshold, int lane, float* sel_v, int* sel_i,
                                             size_t token, int32_t* __restrict__ ids,
                                             float* __restrict__ scores, float* __restrict__ weights,
                                             __nv_bfloat16* __restrict__ dbg_weights) {
-  const float threshold = warp_eighth_largest(v, lane);
   const unsigned lt_mask = (1u << lane) - 1u;
   int held = 0;
 #pragma unroll
@@ -227,8 +230,8 @@ prefill_router_kernel(const __nv_bfloat16* __restrict__ h2,
     v[q] = finish_logit(v[q], bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths);
     if (dbg_logits != nullptr) dbg_logits[static_cast<size_t>(token) * kExperts + 32 * q + lane] = v[q];
   }
-  route_token(v, lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token), ids, scores,
-              weights, dbg_weights);
+  route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
+              ids, scores, weights, dbg_weights);
   if (lane == 0) {
     shared_sigmoid[token] = round_bf16(det_sigmoid(round_bf16(gate_dot)));
   }
@@ -356,10 +359,12 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
     }
     acc0 = butterfly_sum(acc0);
     acc1 = butterfly_sum(acc1);
+    const float f0 = finish_logit(acc0, bias != nullptr ? __ldg(bias + e0) : 0.0f, quant_eighths);
+    const float f1 = finish_logit(acc1, bias != nullptr && e1 >= 0 ? __ldg(bias + e1) : 0.0f, quant_eighths);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      if (e0 == 32 * q + lane) v[q] = finish_logit(acc0, b[q], quant_eighths);
-      if (e1 == 32 * q + lane) v[q] = finish_logit(acc1, b[q], quant_eighths);
+      if (e0 == 32 * q + lane) v[q] = f0;
+      if (e1 == 32 * q + lane) v[q] = f1;
     }
   };
   // is the canonical value further from the tensor-core value than the bound the filter relied on?
@@ -388,7 +393,17 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
       exact_pair(e, e + 1, acc0, acc1);
     }
   }
-  const int certified_id = route_token(v, lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
+  // exactly eight candidates (nine tokens in ten): all are selected and the threshold is their smallest.  (A value at or
+  // below -inf in the order of the keys takes the general rule.)
+  uint32_t smallest = 0xffffffffu;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (upper[q] >= floor_value) smallest = min(smallest, order_key(v[q]));
+  }
+  smallest = __reduce_min_sync(0xffffffffu, smallest);
+  const float threshold = (recomputed == kTopK && !violated && smallest > order_key(-CUDART_INF_F))
+                              ? key_value(smallest) : warp_eighth_largest(v, lane);
+  const int certified_id = route_token(v, threshold, lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
                                        ids, scores, weights, dbg_weights);
   bool audited = false, audit_mismatch = false;
   if (audit_stride > 0 && token % audit_stride == 0 && !violated) {
@@ -396,7 +411,7 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
       float acc0, acc1;
       exact_pair(e, e + 1, acc0, acc1);
     }
-    const int exact_id = route_token(v, lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
+    const int exact_id = route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
                                      ids, scores, weights, dbg_weights);
     audited = true;
     audit_mismatch = __any_sync(0xffffffffu, lane < kTopK && exact_id != certified_id);
@@ -440,64 +455,8 @@ router_row_norms_kernel(const __nv_bfloat16* __restrict__ router, float* __restr
 }
 
 // ---------------------------------------------------------------------------
-// Dispatch plan: stable counting sort of the 8T routed rows by expert.
-// A "unit" is the 256 consecutive flat rows one warp owns.
+// Dispatch plan: stable counting sort of the 8T routed rows by expert, in one launch.
 // ---------------------------------------------------------------------------
-constexpr int kPlanWarps = 8;
-
-__global__ void __launch_bounds__(kPlanWarps * 32)
-plan_count_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int expert_hi,
-                  int32_t* __restrict__ unit_counts) {
-  __shared__ int cnt[kPlanWarps][kExperts];
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  for (int e = lane; e < kExperts; e += 32) cnt[warp][e] = 0;
-  __syncwarp();
-  pdl_enter();
-  const int unit = blockIdx.x * kPlanWarps + warp;
-  const int row0 = unit * kPlanRowsPerWarp;
-  if (row0 >= routed_rows) return;
-  for (int round = 0; round < kPlanRowsPerWarp / 32; ++round) {
-    const int row = row0 + round * 32 + lane;
-    // rows routed to experts held by another GPU are not part of this GPU's plan
-    const int e = row < routed_rows ? ids[row] : -1;
-    const bool valid = e >= expert_lo && e < expert_hi;
-    const unsigned active = __ballot_sync(0xffffffffu, valid);
-    if (valid) {
-      const unsigned same = __match_any_sync(active, e);
-      if ((same & ((1u << lane) - 1u)) == 0u) cnt[warp][e] += __popc(same);
-    }
-    __syncwarp();
-  }
-  for (int e = lane; e < kExperts; e += 32) {
-    unit_counts[static_cast<size_t>(unit) * kExperts + e] = cnt[warp][e];
-  }
-}
-
-// One warp per expert: exclusive prefix of that expert's counts over the units (in place) and the
-// expert's total.  Grid = 256 / kPlanWarps blocks.
-__global__ void __launch_bounds__(kPlanWarps * 32)
-plan_scan_kernel(int32_t* __restrict__ unit_counts, int units, int32_t* __restrict__ expert_counts) {
-  pdl_enter();
-  const int lane = threadIdx.x & 31;
-  const int e = blockIdx.x * kPlanWarps + (threadIdx.x >> 5);
-  int running = 0;
-  for (int u0 = 0; u0 < units; u0 += 32) {
-    const int u = u0 + lane;
-    const size_t index = static_cast<size_t>(u) * kExperts + e;
-    const int c = u < units ? unit_counts[index] : 0;
-    int inclusive = c;
-#pragma unroll
-    for (int d = 1; d < 32; d *= 2) {
-      const int up = __shfl_up_sync(0xffffffffu, inclusive, d);
-      if (lane >= d) inclusive += up;
-    }
-    if (u < units) unit_counts[index] = running + inclusive - c;
-    running += __shfl_sync(0xffffffffu, inclusive, 31);
-  }
-  if (lane == 0) expert_counts[e] = running;
-}
-
 // Rows per tile of an expert with `count` rows.  128-row tiles (one-SM products) are filled one after the other.  Tiles
 // of up to 256 rows (two-SM products, whose cost goes with the rows in steps of 32) are made equally large: 272 rows
 // are 160 + 112, not 256 + 16, so that the last tile does not stream the expert's weights for a handful of rows.  All
@@ -508,118 +467,153 @@ __device__ __forceinline__ int rows_per_tile(int count, int n_tiles, int tile_ca
   return ((count + n_tiles - 1) / n_tiles + 31) & ~31;
 }
 
-// Exclusive offsets of the 256 experts from their counts, in shared memory (all 256 threads of a
-// block take part); thread 0 .. 255 returns with offsets[0 .. 256] and tile_base[0 .. 256] filled.
-__device__ __forceinline__ int expert_offsets_in_block(const int32_t* __restrict__ expert_counts, int tile_cap,
-                                                       int* offsets, int* tile_base, int* warp_sums) {
-  const int e = threadIdx.x;
-  const int lane = e & 31, warp = e >> 5;
-  const int count = expert_counts[e];
-  int v0 = count, v1 = (count + tile_cap - 1) / tile_cap, v2 = (count + 31) / 32 * 32;
-  const int mine0 = v0, mine1 = v1;
-#pragma unroll
-  for (int d = 1; d < 32; d *= 2) {
-    const int a0 = __shfl_up_sync(0xffffffffu, v0, d);
-    const int a1 = __shfl_up_sync(0xffffffffu, v1, d);
-    const int a2 = __shfl_up_sync(0xffffffffu, v2, d);
-    if (lane >= d) { v0 += a0; v1 += a1; v2 += a2; }
-  }
-  if (lane == 31) { warp_sums[warp] = v0; warp_sums[8 + warp] = v1; warp_sums[16 + warp] = v2; }
-  __syncthreads();
-  int b0 = 0, b1 = 0, padded = 0;
-#pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    if (w < warp) { b0 += warp_sums[w]; b1 += warp_sums[8 + w]; }
-    padded += warp_sums[16 + w];
-  }
-  offsets[e] = b0 + v0 - mine0;
-  tile_base[e] = b1 + v1 - mine1;
-  if (e == kExperts - 1) { offsets[kExperts] = b0 + v0; tile_base[kExperts] = b1 + v1; }
-  __syncthreads();
-  return padded;
-}
+// One cluster of eight blocks, 256 warps; a warp owns a contiguous run of flat rows.  Count per warp and expert in shared
+// memory, prefix over a block's warps, over the blocks through distributed shared memory, over the experts; then each
+// warp scatters its run.  Block 0 also publishes the counts, the offsets, the tile list and the reference's block-32
+// padded row count.  Bound by latency (the ids are 256 KB at T = 8192): as three kernels -- count, scan, scatter -- it
+// took 28 us there, most of it between the kernels.
+constexpr int kPlanBlocks = 8;
+constexpr int kPlanWarps = 32;
+constexpr int kPlanRounds = 8;      // rounds of 32 rows whose ids are requested together
 
-// Stable scatter.  Every block first derives the expert offsets from the counts; block 0 also
-// publishes them together with the tile list and the reference's block-32 padded row count.
-__global__ void __launch_bounds__(kPlanWarps * 32)
-plan_scatter_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int expert_hi,
-                    const int32_t* __restrict__ unit_prefix,
-                    const int32_t* __restrict__ expert_counts,
-                    int32_t* __restrict__ expert_offsets,
-                    int32_t* __restrict__ tile_expert, int32_t* __restrict__ tile_row0,
-                    int32_t* __restrict__ tile_rows, int32_t* __restrict__ tile_count,
-                    int32_t* __restrict__ padded_rows,
-                    int32_t* __restrict__ sorted_rows, int32_t* __restrict__ row_position, int tile_cap) {
-  static_assert(kPlanWarps * 32 == kExperts, "one thread per expert in the prologue");
-  pdl_enter();
-  __shared__ int next[kPlanWarps][kExperts];
-  __shared__ int offsets[kExperts + 1];
-  __shared__ int tile_base[kExperts + 1];
-  __shared__ int warp_sums[24];
-  const int padded = expert_offsets_in_block(expert_counts, tile_cap, offsets, tile_base, warp_sums);
-  if (blockIdx.x == 0) {
-    const int e = threadIdx.x;
-    const int count = offsets[e + 1] - offsets[e];
-    expert_offsets[e] = offsets[e];
-    if (e == 0) {
-      expert_offsets[kExperts] = offsets[kExperts];
-      *tile_count = tile_base[kExperts];
-      *padded_rows = padded;
-    }
-    const int n_tiles = tile_base[e + 1] - tile_base[e];
-    const int height = rows_per_tile(count, n_tiles, tile_cap);
-    for (int t = 0; t < n_tiles; ++t) {
-      const int index = tile_base[e] + t;
-      tile_expert[index] = e;
-      tile_row0[index] = offsets[e] + t * height;
-      tile_rows[index] = min(height, count - t * height);
-    }
-  }
+__global__ void __cluster_dims__(kPlanBlocks, 1, 1) __launch_bounds__(kPlanWarps * 32)
+plan_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int expert_hi, int tile_cap,
+            int32_t* __restrict__ expert_counts, int32_t* __restrict__ expert_offsets,
+            int32_t* __restrict__ tile_expert, int32_t* __restrict__ tile_row0, int32_t* __restrict__ tile_rows,
+            int32_t* __restrict__ tile_count, int32_t* __restrict__ padded_rows,
+            int32_t* __restrict__ sorted_rows, int32_t* __restrict__ row_position) {
+  __shared__ int cnt[kPlanWarps][kExperts];      // a warp's counts, then its exclusive prefix, then its next positions
+  __shared__ int block_counts[kExperts];
+  __shared__ int base[kExperts];
+  __shared__ int warp_sums[3][kExperts / 32];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int unit = blockIdx.x * kPlanWarps + warp;
-  const int row0 = unit * kPlanRowsPerWarp;
-  if (row0 >= routed_rows) return;
-  for (int e = lane; e < kExperts; e += 32) {
-    next[warp][e] = offsets[e] + unit_prefix[static_cast<size_t>(unit) * kExperts + e];
-  }
+  const int block = blockIdx.x;                  // the grid is one cluster
+  for (int e = lane; e < kExperts; e += 32) cnt[warp][e] = 0;
   __syncwarp();
-  for (int round = 0; round < kPlanRowsPerWarp / 32; ++round) {
-    const int row = row0 + round * 32 + lane;
-    const int e = row < routed_rows ? ids[row] : -1;
-    const bool valid = e >= expert_lo && e < expert_hi;
-    const unsigned active = __ballot_sync(0xffffffffu, valid);
-    if (valid) {
-      const unsigned same = __match_any_sync(active, e);
-      const int rank = __popc(same & ((1u << lane) - 1u));
-      const int pos = next[warp][e] + rank;
-      sorted_rows[pos] = row;
-      row_position[row] = pos;
-      __syncwarp(active);
-      if (rank == 0) next[warp][e] += __popc(same);
+  pdl_enter();
+  const int run = ((routed_rows + kPlanBlocks * kPlanWarps - 1) / (kPlanBlocks * kPlanWarps) + 31) & ~31;
+  const int row_lo = min(routed_rows, (block * kPlanWarps + warp) * run);
+  const int row_hi = min(routed_rows, row_lo + run);
+  // rows routed to experts held by another GPU are not part of this GPU's plan
+  auto fetch = [&](int row0, int* e) {
+#pragma unroll
+    for (int i = 0; i < kPlanRounds; ++i) {
+      const int row = row0 + 32 * i + lane;
+      e[i] = row < row_hi ? ids[row] : -1;
+      if (e[i] < expert_lo || e[i] >= expert_hi) e[i] = -1;
     }
-    __syncwarp();
+  };
+  for (int row0 = row_lo; row0 < row_hi; row0 += 32 * kPlanRounds) {
+    int e[kPlanRounds];
+    fetch(row0, e);
+#pragma unroll
+    for (int i = 0; i < kPlanRounds; ++i) {
+      const unsigned same = __match_any_sync(0xffffffffu, e[i]);
+      if (e[i] >= 0 && (same & ((1u << lane) - 1u)) == 0u) cnt[warp][e[i]] += __popc(same);
+      __syncwarp();
+    }
   }
+  __syncthreads();
+  if (threadIdx.x < kExperts) {
+    int running = 0;
+#pragma unroll
+    for (int w = 0; w < kPlanWarps; ++w) {
+      const int c = cnt[w][threadIdx.x];
+      cnt[w][threadIdx.x] = running;
+      running += c;
+    }
+    block_counts[threadIdx.x] = running;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  int count = 0, before = 0, v0 = 0, v1 = 0, v2 = 0;
+  if (threadIdx.x < kExperts) {
+#pragma unroll
+    for (int b = 0; b < kPlanBlocks; ++b) {
+      uint32_t remote;
+      int c;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&block_counts[threadIdx.x])), "r"(b));
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(c) : "r"(remote) : "memory");
+      if (b < block) before += c;
+      count += c;
+    }
+    v0 = count;
+    v1 = (count + tile_cap - 1) / tile_cap;
+    v2 = (count + 31) / 32 * 32;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+      const int a0 = __shfl_up_sync(0xffffffffu, v0, d);
+      const int a1 = __shfl_up_sync(0xffffffffu, v1, d);
+      const int a2 = __shfl_up_sync(0xffffffffu, v2, d);
+      if (lane >= d) { v0 += a0; v1 += a1; v2 += a2; }
+    }
+    if (lane == 31) { warp_sums[0][warp] = v0; warp_sums[1][warp] = v1; warp_sums[2][warp] = v2; }
+  }
+  // this block has read the others' counts; they may leave once it has arrived (waited for at the end)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x < kExperts) {
+    const int e = threadIdx.x;
+    const int n_tiles = (count + tile_cap - 1) / tile_cap;
+    int offset = v0 - count, first_tile = v1 - n_tiles, total = 0, total_tiles = 0, padded = 0;
+#pragma unroll
+    for (int w = 0; w < kExperts / 32; ++w) {
+      if (w < warp) { offset += warp_sums[0][w]; first_tile += warp_sums[1][w]; }
+      total += warp_sums[0][w];
+      total_tiles += warp_sums[1][w];
+      padded += warp_sums[2][w];
+    }
+    base[e] = offset + before;
+    if (block == 0) {
+      expert_counts[e] = count;
+      expert_offsets[e] = offset;
+      if (e == 0) {
+        expert_offsets[kExperts] = total;
+        *tile_count = total_tiles;
+        *padded_rows = padded;
+      }
+      const int height = rows_per_tile(count, n_tiles, tile_cap);
+      for (int t = 0; t < n_tiles; ++t) {
+        tile_expert[first_tile + t] = e;
+        tile_row0[first_tile + t] = offset + t * height;
+        tile_rows[first_tile + t] = min(height, count - t * height);
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = lane; e < kExperts; e += 32) cnt[warp][e] += base[e];
+  __syncwarp();
+  for (int row0 = row_lo; row0 < row_hi; row0 += 32 * kPlanRounds) {
+    int e[kPlanRounds];
+    fetch(row0, e);
+#pragma unroll
+    for (int i = 0; i < kPlanRounds; ++i) {
+      const unsigned same = __match_any_sync(0xffffffffu, e[i]);
+      const int rank = __popc(same & ((1u << lane) - 1u));
+      int pos = 0;
+      if (e[i] >= 0) pos = cnt[warp][e[i]] + rank;
+      __syncwarp();
+      if (e[i] >= 0) {
+        const int row = row0 + 32 * i + lane;
+        sorted_rows[pos] = row;
+        row_position[row] = pos;
+        if (rank == 0) cnt[warp][e[i]] += __popc(same);
+      }
+      __syncwarp();
+    }
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Enqueues the dispatch plan for `rows` routed rows whose expert ids are `ids`.
 // tile_cap: rows per tile of the plan -- 128 for the one-SM product kernels, 256 for the two-SM form
 cudaError_t launch_plan(PrefillWorkspace* ws, const int32_t* ids, int rows, int expert_lo, int expert_hi,
                         cudaStream_t stream, int* launches, int tile_cap = kTileRows) {
-  const int units = (rows + kPlanRowsPerWarp - 1) / kPlanRowsPerWarp;
-  const int plan_blocks = (units + kPlanWarps - 1) / kPlanWarps;
-  cudaError_t code = launch_pdl(plan_count_kernel, dim3(plan_blocks), dim3(kPlanWarps * 32), 0, stream, ids, rows,
-                                expert_lo, expert_hi, ws->unit_counts);
-  if (code == cudaSuccess)
-    code = launch_pdl(plan_scan_kernel, dim3(kExperts / kPlanWarps), dim3(kPlanWarps * 32), 0, stream,
-                      ws->unit_counts, units, ws->expert_counts);
-  if (code == cudaSuccess)
-    code = launch_pdl(plan_scatter_kernel, dim3(plan_blocks), dim3(kPlanWarps * 32), 0, stream, ids, rows,
-                      expert_lo, expert_hi, ws->unit_counts, ws->expert_counts, ws->expert_offsets,
-                      ws->tile_expert, ws->tile_row0, ws->tile_rows, ws->tile_count, ws->padded_rows,
-                      ws->sorted_rows, ws->row_position, tile_cap);
-  *launches += 3;
-  return code;
+  *launches += 1;
+  return launch_pdl(plan_kernel, dim3(kPlanBlocks), dim3(kPlanWarps * 32), 0, stream, ids, rows, expert_lo, expert_hi,
+                    tile_cap, ws->expert_counts, ws->expert_offsets, ws->tile_expert, ws->tile_row0, ws->tile_rows,
+                    ws->tile_count, ws->padded_rows, ws->sorted_rows, ws->row_position);
 }
 
 // ---------------------------------------------------------------------------
@@ -652,7 +646,7 @@ combine_kernel(const __nv_bfloat16* __restrict__ expert_down,
                const __nv_bfloat16* __restrict__ next_norm_weight,
                __nv_bfloat16* __restrict__ next_norm_out, float eps) {
   __shared__ float group_sums[8];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // next layer's router product may set itself up
+  pdl_enter();
   const int token = blockIdx.x;
   const int t = threadIdx.x;
   float slot[kTopK][8];
@@ -892,7 +886,7 @@ int set_error(char* error, size_t error_bytes, cudaError_t code, const char* wha
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 struct Layout {
-  size_t ids, scores, weights, sigmoid, approx, stats, unit_counts, counts, offsets, sorted, position,
+  size_t ids, scores, weights, sigmoid, approx, stats, counts, offsets, sorted, position,
       tile_expert, tile_row0, tile_rows, tile_count, padded, gathered, act, down, shared_act,
       shared_scaled, x0, x1, h2, total;
 };
@@ -902,7 +896,6 @@ Layout layout_for(size_t T) {
   size_t cursor = 0;
   auto take = [&](size_t bytes) { const size_t at = cursor; cursor += align256(bytes); return at; };
   const size_t rows = T * kTopK;
-  const size_t units = (rows + kPlanRowsPerWarp - 1) / kPlanRowsPerWarp;
   const size_t tiles = static_cast<size_t>(max_tiles_for(static_cast<int>(T)));
   l.ids = take(rows * 4);
   l.scores = take(rows * 4);
@@ -910,7 +903,6 @@ Layout layout_for(size_t T) {
   l.sigmoid = take(T * 4);
   l.approx = take(T * kExperts * 4);
   l.stats = take(32);
-  l.unit_counts = take(units * kExperts * 4);
   l.counts = take(kExperts * 4);
   l.offsets = take((kExperts + 1) * 4);
   l.sorted = take(rows * 4);
@@ -974,7 +966,6 @@ int prefill_workspace_allocate(PrefillWorkspace* ws, uint32_t capacity_tokens, i
   ws->shared_sigmoid = reinterpret_cast<float*>(b + l.sigmoid);
   ws->approx_logits = reinterpret_cast<float*>(b + l.approx);
   ws->router_stats = reinterpret_cast<int32_t*>(b + l.stats);
-  ws->unit_counts = reinterpret_cast<int32_t*>(b + l.unit_counts);
   ws->expert_counts = reinterpret_cast<int32_t*>(b + l.counts);
   ws->expert_offsets = reinterpret_cast<int32_t*>(b + l.offsets);
   ws->sorted_rows = reinterpret_cast<int32_t*>(b + l.sorted);
@@ -1039,27 +1030,10 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   int count = 0;
   cudaError_t code;
 
-  // fork: the shared gate/up product needs only h2
-  cudaStream_t side = ws->side_stream;
-  if ((code = cudaEventRecord(ws->fork_event, stream)) != cudaSuccess ||
-      (code = cudaStreamWaitEvent(side, ws->fork_event, 0)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "fork of the shared-expert stream");
-  auto product = [&](GemmMode mode, const GroupedGemm& problem, const TcExtra& x, cudaStream_t on) {
-    return ws->use_simt_gemm ? launch_grouped_gemm_simt(mode, problem, on)
-                             : launch_grouped_gemm_tc(mode, problem, x, on);
-  };
-  GroupedGemm s{};
-  TcExtra shared_extra{};
-  shared_extra.status = ws->status; shared_extra.sm_count = ws->sm_count;
-  s.tile_expert = nullptr; s.tile_row0 = nullptr; s.tile_rows = nullptr; s.tile_count = nullptr;
-  s.max_tiles = (T + kTileRows - 1) / kTileRows; s.dense_rows = T;
-  s.a = static_cast<const __nv_bfloat16*>(call.h2); s.lda = kHidden; s.k = kHidden;
-  s.b0 = call.layer.shared_gate_proj; s.b1 = call.layer.shared_up_proj; s.b_expert_stride = 0;
-  s.n = kSharedInter; s.c = ws->shared_act; s.ldc = kSharedInter;
-  shared_extra.a_rows = static_cast<uint64_t>(T); shared_extra.experts_in_b = 1;
-  if ((code = product(kGemmSharedGateUp, s, shared_extra, side)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "grouped gemm shared gate_up");
-  ++count;
+  // Products: the two-SM tensor-core form, which takes the shared expert's rows along as tiles of their own, with tiles of
+  // up to 256 rows; or the CUDA-core cross-check, with 128-row tiles and the shared expert in launches of its own.
+  const bool simt = ws->use_simt_gemm;
+  const __nv_bfloat16* h2 = static_cast<const __nv_bfloat16*>(call.h2);
 
   const bool exact_router = ws->exact_router || (dbg != nullptr && dbg->router_logits != nullptr) ||
                             call.router_row_norms == nullptr;
@@ -1081,6 +1055,7 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
     r.b0 = call.layer.router; r.n = kExperts; r.c_f32 = ws->approx_logits; r.ldc = kExperts;
     TcExtra rx{};
     rx.status = ws->status; rx.sm_count = ws->sm_count; rx.a_rows = static_cast<uint64_t>(T); rx.experts_in_b = 1;
+    rx.pair = true;
     if ((code = launch_grouped_gemm_tc(kGemmPlainF32, r, rx, stream)) != cudaSuccess)
       return set_error(error, error_bytes, code, "router logits product");
     code = launch_pdl(prefill_router_certified_kernel, dim3((T + kCertWarps - 1) / kCertWarps), dim3(kCertWarps * 32),
@@ -1101,25 +1076,7 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
     ++count;
   }
 
-  // the shared down product scales by the sigmoid the router kernel wrote
-  if ((code = cudaEventRecord(ws->router_event, stream)) != cudaSuccess ||
-      (code = cudaStreamWaitEvent(side, ws->router_event, 0)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "router event of the shared-expert stream");
-  s.a = ws->shared_act; s.lda = kSharedInter; s.k = kSharedInter;
-  s.b0 = call.layer.shared_down_proj; s.b1 = nullptr;
-  s.n = kHidden; s.c = ws->shared_scaled; s.ldc = kHidden;
-  s.row_scale = ws->shared_sigmoid;
-  shared_extra.a_rows = static_cast<uint64_t>(ws->capacity);
-  if ((code = product(kGemmSharedDown, s, shared_extra, side)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "grouped gemm shared down");
-  ++count;
-  if ((code = cudaEventRecord(ws->join_event, side)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "join event of the shared-expert stream");
-
-  // Expert products: the two-SM form with tiles of up to 256 rows (128-row tiles for the CUDA-core cross-check)
-  const bool pair_products = ws->pair_products && !ws->use_simt_gemm;
-  if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, stream, &count, pair_products ? 2 * kTileRows : kTileRows)) !=
-      cudaSuccess)
+  if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, stream, &count, simt ? kTileRows : 2 * kTileRows)) != cudaSuccess)
     return set_error(error, error_bytes, code, "dispatch plan");
 
   // Dispatch.  Up to kGatherMaxTokens the gate_up kernel fetches each tile's rows by token index itself (TMA gather4);
@@ -1127,7 +1084,7 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   // ~45 cycles, which the weight stream hides while a tile has few rows and not when it has 256: sustained us per layer,
   // gather4 / copied rows, balanced routing: 331 / 348 at 1024 tokens, 379 / 420 at 2048, 451 / 468 at 3072, 518 / 505 at
   // 4096, 645 / 610 at 6144, 855 / 771 at 8192.
-  const bool fused_dispatch = ws->fused_dispatch && !ws->use_simt_gemm && T <= kGatherMaxTokens;
+  const bool fused_dispatch = ws->fused_dispatch && !simt && T <= kGatherMaxTokens;
   if (!fused_dispatch) {
     gather_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(call.h2), ws->sorted_rows, rows, ws->gathered);
@@ -1147,35 +1104,52 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   TcExtra extra{};
   extra.status = ws->status; extra.sm_count = ws->sm_count;
   extra.experts_in_b = call.experts_local;
-  extra.pair = pair_products;
+  extra.pair = !simt;
   if (fused_dispatch) {
-    g.gather_src = static_cast<const __nv_bfloat16*>(call.h2);
+    g.gather_src = h2;
     extra.a_rows = static_cast<uint64_t>(T);
   } else {
     extra.a_rows = static_cast<uint64_t>(ws->capacity) * kTopK;
   }
-  if ((code = product(kGemmExpertGateUp, g, extra, stream)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "grouped gemm expert gate_up");
+  extra.shared = SharedProblem{T, h2, call.layer.shared_gate_proj, call.layer.shared_up_proj, ws->shared_act, nullptr};
+  if (simt) {
+    GroupedGemm s{};
+    s.max_tiles = (T + kTileRows - 1) / kTileRows; s.dense_rows = T;
+    s.a = h2; s.lda = kHidden; s.k = kHidden;
+    s.b0 = call.layer.shared_gate_proj; s.b1 = call.layer.shared_up_proj;
+    s.n = kSharedInter; s.c = ws->shared_act; s.ldc = kSharedInter;
+    code = launch_grouped_gemm_simt(kGemmSharedGateUp, s, stream);
+    if (code == cudaSuccess) {
+      s.a = ws->shared_act; s.lda = kSharedInter; s.k = kSharedInter;
+      s.b0 = call.layer.shared_down_proj; s.b1 = nullptr;
+      s.n = kHidden; s.c = ws->shared_scaled; s.ldc = kHidden;
+      s.row_scale = ws->shared_sigmoid;
+      code = launch_grouped_gemm_simt(kGemmSharedDown, s, stream);
+    }
+    if (code == cudaSuccess) code = launch_grouped_gemm_simt(kGemmExpertGateUp, g, stream);
+    count += 2;
+  } else {
+    code = launch_grouped_gemm_tc(kGemmExpertGateUp, g, extra, stream);
+  }
+  if (code != cudaSuccess) return set_error(error, error_bytes, code, "grouped gemm expert gate_up");
   g.gather_src = nullptr;
   extra.a_rows = static_cast<uint64_t>(ws->capacity) * kTopK;
   g.a = ws->expert_act; g.lda = kInter; g.k = kInter;
   g.b0 = call.layer.expert_down; g.b_expert_stride = static_cast<size_t>(kHidden) * kInter;
   g.n = kHidden; g.c = ws->expert_down; g.ldc = kHidden;
   g.row_scale = ws->topk_weights; g.sorted_rows = ws->sorted_rows;
-  if ((code = product(kGemmExpertDown, g, extra, stream)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "grouped gemm expert down");
+  extra.shared = SharedProblem{T, ws->shared_act, call.layer.shared_down_proj, nullptr, ws->shared_scaled, ws->shared_sigmoid};
+  code = simt ? launch_grouped_gemm_simt(kGemmExpertDown, g, stream)
+              : launch_grouped_gemm_tc(kGemmExpertDown, g, extra, stream);
+  if (code != cudaSuccess) return set_error(error, error_bytes, code, "grouped gemm expert down");
   count += 2;
 
-  // join: the combine needs the shared expert's output
-  if ((code = cudaStreamWaitEvent(stream, ws->join_event, 0)) != cudaSuccess)
-    return set_error(error, error_bytes, code, "join of the shared-expert stream");
-  combine_kernel<<<T, 256, 0, stream>>>(ws->expert_down, ws->row_position, ws->shared_scaled,
-                                        static_cast<const __nv_bfloat16*>(call.residual),
-                                        static_cast<__nv_bfloat16*>(call.out),
-                                        dbg ? static_cast<__nv_bfloat16*>(dbg->routed) : nullptr,
-                                        static_cast<const __nv_bfloat16*>(call.next_norm_weight),
-                                        static_cast<__nv_bfloat16*>(call.next_norm_out), call.eps);
-  if ((code = cudaGetLastError()) != cudaSuccess) return set_error(error, error_bytes, code, "combine_kernel");
+  code = launch_pdl(combine_kernel, dim3(T), dim3(256), 0, stream, ws->expert_down, ws->row_position, ws->shared_scaled,
+                    static_cast<const __nv_bfloat16*>(call.residual), static_cast<__nv_bfloat16*>(call.out),
+                    dbg ? static_cast<__nv_bfloat16*>(dbg->routed) : nullptr,
+                    static_cast<const __nv_bfloat16*>(call.next_norm_weight),
+                    static_cast<__nv_bfloat16*>(call.next_norm_out), call.eps);
+  if (code != cudaSuccess) return set_error(error, error_bytes, code, "combine_kernel");
   ++count;
 
   if (dbg != nullptr) {

@@ -49,7 +49,6 @@ struct PrefillWorkspace {
                                       //     filter's bound (recomputed in full), tokens audited, audit mismatches
   int router_audit_stride = 0;        // qualification: every n-th token is also routed from all 256 canonical logits
   // dispatch plan
-  int32_t* unit_counts = nullptr;     // [units, 256] per-warp-unit histogram / prefix
   int32_t* expert_counts = nullptr;   // [256]
   int32_t* expert_offsets = nullptr;  // [257]
   int32_t* sorted_rows = nullptr;     // [8T]  flat (token*8+slot) rows grouped by expert
