@@ -255,6 +255,13 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
+// One lane of a converged warp, for issuing TMA and tcgen05 instructions: their operands live in the warp's uniform
+// registers, and inside a branch on `lane == 0` the compiler has to move every one of them there again under divergence.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+  return chosen != 0;
+}
 // global -> shared bulk copy; bytes % 16 == 0, both addresses 16-byte aligned.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src,
                                          uint32_t bytes, uint32_t bar) {

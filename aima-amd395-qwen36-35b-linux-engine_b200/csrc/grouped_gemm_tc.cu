@@ -76,6 +76,9 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "[%0], [%1, {%2, %3}], [%4];"
       :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
+// The producer and MMA loops below are run by their WHOLE warp and only the issuing instructions are guarded by
+// elect_one().  With a branch on lane == 0 around the loops a stage cost its TMA thread 680 cycles (two loads) and its MMA
+// thread 320 (four MMAs) of issue time -- more than the 512 cycles the tensor cores need for it.
 constexpr int kGatherThreads = 64;     // warps 2 and 3
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
@@ -107,16 +110,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// One lane of a converged warp.  The producer and MMA loops below are run by their WHOLE warp and only the issuing
-// instructions are guarded by this: the operands of TMA and tcgen05 instructions live in the warp's uniform registers,
-// and inside a branch on `lane == 0` the compiler has to move every one of them there again under divergence.  With
-// that branch around the loops a stage cost its TMA thread 680 cycles (two loads) and its MMA thread 320 (four MMAs)
-// of issue time -- more than the 512 cycles the tensor cores need for it.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t chosen;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
-  return chosen != 0;
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"

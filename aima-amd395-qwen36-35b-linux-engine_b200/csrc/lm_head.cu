@@ -16,7 +16,6 @@ namespace aima {
 namespace {
 
 constexpr int kLmThreads = 256;
-constexpr int kLmBoundBlocks = 256;
 constexpr int kResidualSafetyUlps = 8;
 constexpr int kHiddenSafetyUlps = 4;
 
@@ -79,7 +78,7 @@ lm_head_quantize_kernel(const __nv_bfloat16* __restrict__ source, int8_t* __rest
 
 // ---------------------------------------------------------------------------
 // Scan: approximate[row] = scale[row] * sum_c q[row, c] * hidden[c], FP32.
-// One warp per row at a time; lane l owns the 16-byte pieces l, l + 32, l + 64, l + 96 of the
+// Lane l owns the 16-byte pieces l, l + 32, l + 64, l + 96 of the
 // row (64 weights), multiplies them in ascending order into one accumulator, then the warp
 // butterfly (16, 8, 4, 2, 1).  The lane's 64 hidden values stay in registers for all its rows.
 // int8 -> FP32 without the conversion pipe: the byte, biased by 128, is placed in the mantissa
@@ -98,84 +97,28 @@ __device__ __forceinline__ float fma_word(uint32_t word, const float* x, float a
   return acc;
 }
 
-constexpr int kScanWarps = 4;
-
-__global__ void __launch_bounds__(kScanWarps * 32)
-lm_head_scan_kernel(const int8_t* __restrict__ q_weight, const float* __restrict__ scales,
-                    const __nv_bfloat16* __restrict__ hidden, float* __restrict__ logits, int rows) {
-  // the three short kernels after this one are placed while its last blocks drain (see pdl_enter)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int lane = threadIdx.x & 31;
-  const int warp_global = blockIdx.x * kScanWarps + (threadIdx.x >> 5);
-  const int warps_total = gridDim.x * kScanWarps;
-  float x[64];
+// ||hidden||_2 in FP64, rounded to FP32 and up 4 ULPs.  The order is that of 256 partials (partial t = elements t, t + 256,
+// ... in that order) folded by halving; lane l holds partials l + 32 j, so the halvings of width 128, 64 and 32 are its own
+// and the rest are lane exchanges.  Every warp of the scan evaluates it for itself while its first rows are on their way.
+__device__ __forceinline__ float hidden_norm_in_warp(const __nv_bfloat16* __restrict__ hidden, int lane) {
+  double q[8];
 #pragma unroll
-  for (int piece = 0; piece < 4; ++piece) {
-    // 16 weights of piece (32 piece + lane): hidden elements 16 (32 piece + lane) .. + 15
-    const uint4* src = reinterpret_cast<const uint4*>(hidden) + 2 * (32 * piece + lane);
-    unpack8(__ldg(src), x + 16 * piece);
-    unpack8(__ldg(src + 1), x + 16 * piece + 8);
-  }
-  // Two rows per trip, and the loads of the next trip are issued before the arithmetic of this one:
-  // eight to sixteen 16-byte loads per lane stay in flight.
-  auto load_pair = [&](int row, uint4* wa, uint4* wb) {
-    const int row_b = row + warps_total;
-    const uint4* qrow_a = reinterpret_cast<const uint4*>(q_weight + static_cast<size_t>(row) * kHidden) + lane;
-    const uint4* qrow_b = reinterpret_cast<const uint4*>(q_weight + static_cast<size_t>(row_b < rows ? row_b : row) * kHidden) + lane;
+  for (int j = 0; j < 8; ++j) {
+    q[j] = 0.0;
 #pragma unroll
-    for (int piece = 0; piece < 4; ++piece) wa[piece] = __ldcs(qrow_a + 32 * piece);
-#pragma unroll
-    for (int piece = 0; piece < 4; ++piece) wb[piece] = __ldcs(qrow_b + 32 * piece);
-  };
-  uint4 wa[4], wb[4];
-  if (warp_global < rows) load_pair(warp_global, wa, wb);
-  for (int row = warp_global; row < rows; row += 2 * warps_total) {
-    const int row_b = row + warps_total;
-    const int next = row + 2 * warps_total;
-    uint4 na[4], nb[4];
-    if (next < rows) load_pair(next, na, nb);
-    float acc_a = 0.0f, acc_b = 0.0f;
-#pragma unroll
-    for (int piece = 0; piece < 4; ++piece) {
-      acc_a = fma_word(wa[piece].x, x + 16 * piece, acc_a);
-      acc_a = fma_word(wa[piece].y, x + 16 * piece + 4, acc_a);
-      acc_a = fma_word(wa[piece].z, x + 16 * piece + 8, acc_a);
-      acc_a = fma_word(wa[piece].w, x + 16 * piece + 12, acc_a);
-      acc_b = fma_word(wb[piece].x, x + 16 * piece, acc_b);
-      acc_b = fma_word(wb[piece].y, x + 16 * piece + 4, acc_b);
-      acc_b = fma_word(wb[piece].z, x + 16 * piece + 8, acc_b);
-      acc_b = fma_word(wb[piece].w, x + 16 * piece + 12, acc_b);
-    }
-    acc_a = butterfly_sum(acc_a);
-    acc_b = butterfly_sum(acc_b);
-    if (lane == 0) {
-      logits[row] = __fmul_rn(acc_a, scales[row]);
-      if (row_b < rows) logits[row_b] = __fmul_rn(acc_b, scales[row_b]);
-    }
-    if (next < rows) {
-#pragma unroll
-      for (int piece = 0; piece < 4; ++piece) { wa[piece] = na[piece]; wb[piece] = nb[piece]; }
+    for (int i = 0; i < kHidden / 256; ++i) {
+      const double value = static_cast<double>(__bfloat162float(hidden[256 * i + 32 * j + lane]));
+      q[j] = __dadd_rn(q[j], __dmul_rn(value, value));
     }
   }
-}
-
-// ||hidden||_2 in FP64 (thread-strided partials, pairwise tree), rounded to FP32 and up 4 ULPs.
-// Every block of the bound kernel evaluates it for itself (2048 values) rather than waiting for
-// a kernel of its own.
-__device__ __forceinline__ float hidden_norm_in_block(const __nv_bfloat16* __restrict__ hidden, double* reduction) {
-  const int t = threadIdx.x;
-  double local = 0.0;
-  for (int index = t; index < kHidden; index += kLmThreads) {
-    const double value = static_cast<double>(__bfloat162float(hidden[index]));
-    local = __dadd_rn(local, __dmul_rn(value, value));
+#pragma unroll
+  for (int width = 4; width >= 1; width >>= 1) {
+#pragma unroll
+    for (int j = 0; j < width; ++j) q[j] = __dadd_rn(q[j], q[j + width]);
   }
-  reduction[t] = local;
-  __syncthreads();
-  for (int stride = kLmThreads / 2; stride != 0; stride >>= 1) {
-    if (t < stride) reduction[t] = __dadd_rn(reduction[t], reduction[t + stride]);
-    __syncthreads();
-  }
-  float norm = static_cast<float>(sqrt(reduction[0]));
+#pragma unroll
+  for (int s = 16; s >= 1; s >>= 1) q[0] = __dadd_rn(q[0], __shfl_xor_sync(0xffffffffu, q[0], s));
+  float norm = static_cast<float>(sqrt(q[0]));
   for (int step = 0; step < kHiddenSafetyUlps; ++step) norm = nextafterf(norm, CUDART_INF_F);
   return norm;
 }
@@ -184,114 +127,211 @@ __device__ __forceinline__ float row_error(float residual, float hidden_l2) {
   return nextafterf(__fmul_rn(residual, hidden_l2), CUDART_INF_F);
 }
 
-// largest lower bound over all rows, per block; block 0 also publishes the hidden norm and empties
-// the candidate list
-__global__ void __launch_bounds__(kLmThreads)
-lm_head_bound_kernel(const float* __restrict__ logits, const float* __restrict__ residual_l2,
-                     const __nv_bfloat16* __restrict__ hidden, aima_moe_lm_head_result* wire,
-                     float* __restrict__ partial, int rows) {
-  __shared__ double norm_reduction[kLmThreads];
-  __shared__ float reduction[kLmThreads];
-  pdl_enter();
-  const float hidden_l2 = hidden_norm_in_block(hidden, norm_reduction);
-  float local_max = -CUDART_INF_F;
-  for (int row = blockIdx.x * kLmThreads + threadIdx.x; row < rows; row += gridDim.x * kLmThreads) {
-    const float lower = nextafterf(__fsub_rn(logits[row], row_error(residual_l2[row], hidden_l2)), -CUDART_INF_F);
-    local_max = fmaxf(local_max, lower);
+constexpr int kScanWarps = 12;
+constexpr int kScanBuffers = 2;                     // per warp
+constexpr int kScanRows = 4;                        // per buffer: one 8 KB copy
+constexpr int kScanBufferBytes = kScanRows * kHidden;
+constexpr int kScanSmemBytes = kScanWarps * kScanBuffers * (kScanBufferBytes + 8) + 16;
+static_assert(32 % kScanRows == 0 && kScanRows % 2 == 0, "logits are finished 32 rows at a time");
+
+// The vocabulary is cut into one contiguous run of rows per warp of the chip.  A warp streams its run four rows (8 KB) at
+// a time through two buffers of its own with 1-D bulk copies -- no register holds a load in flight, so twelve warps keep
+// up to 192 KB per SM on the way -- and reads them back with conflict-free 16-byte loads.  Logits and bounds are finished
+// 32 rows at a time, one per lane.  Bound by HBM; the arithmetic (three instructions per weight, 42 us over the chip at
+// 248 320 rows) runs beside it.
+__global__ void __launch_bounds__(kScanWarps * 32, 1)
+lm_head_scan_kernel(const int8_t* __restrict__ q_weight, const float* __restrict__ scales,
+                    const float* __restrict__ residual_l2, const __nv_bfloat16* __restrict__ hidden,
+                    float* __restrict__ logits, aima_moe_lm_head_result* wire, LmHeadTop* top,
+                    float* __restrict__ partial, int rows) {
+  extern __shared__ __align__(16) uint8_t scan_smem[];
+  __shared__ float warp_max[kScanWarps];
+  // the kernel after this one is placed while its last blocks drain (see pdl_enter)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+  uint8_t* buffers = scan_smem + warp * kScanBuffers * kScanBufferBytes;
+  const uint32_t bars = smem_u32(scan_smem + kScanWarps * kScanBuffers * kScanBufferBytes) + warp * kScanBuffers * 8;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(scan_smem + kScanWarps * kScanBuffers * (kScanBufferBytes + 8));
+  if (lane == 0) {
+    for (int b = 0; b < kScanBuffers; ++b) mbar_init(bars + 8 * b, 1);
+    mbar_fence_init();
   }
-  reduction[threadIdx.x] = local_max;
+  if (threadIdx.x == 0) *abort_flag = 0;
   __syncthreads();
-  for (int stride = kLmThreads / 2; stride != 0; stride >>= 1) {
-    if (threadIdx.x < stride) reduction[threadIdx.x] = fmaxf(reduction[threadIdx.x], reduction[threadIdx.x + stride]);
-    __syncthreads();
+
+  const int warps_total = gridDim.x * kScanWarps;
+  const int run = ((rows + warps_total - 1) / warps_total + 1) & ~1;
+  const long long first = static_cast<long long>(blockIdx.x * kScanWarps + warp) * run;
+  const int lo = static_cast<int>(first < rows ? first : rows);
+  const int hi = min(rows, lo + run);
+  const int steps = (hi - lo + kScanRows - 1) / kScanRows;
+  auto request = [&](int p) {
+    const int row = lo + kScanRows * p;
+    const uint32_t bytes = min(kScanRows, hi - row) * kHidden;
+    const int b = p % kScanBuffers;
+    if (elect_one()) {
+      mbar_arrive_expect_tx(bars + 8 * b, bytes);
+      bulk_g2s(smem_u32(buffers + b * kScanBufferBytes), q_weight + static_cast<size_t>(row) * kHidden, bytes, bars + 8 * b);
+    }
+    __syncwarp();
+  };
+  for (int p = 0; p < min(steps, kScanBuffers); ++p) request(p);
+
+  float x[64];
+#pragma unroll
+  for (int piece = 0; piece < 4; ++piece) {
+    // 16 weights of piece (32 piece + lane): hidden elements 16 (32 piece + lane) .. + 15
+    const uint4* src = reinterpret_cast<const uint4*>(hidden) + 2 * (32 * piece + lane);
+    unpack8(__ldg(src), x + 16 * piece);
+    unpack8(__ldg(src + 1), x + 16 * piece + 8);
   }
-  if (threadIdx.x == 0) {
-    partial[blockIdx.x] = reduction[0];
-    if (blockIdx.x == 0) {
-      wire->hidden_l2 = hidden_l2;
-      wire->candidate_count = 0;
-      wire->overflow = 0;
+  const float hidden_l2 = hidden_norm_in_warp(hidden, lane);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    wire->hidden_l2 = hidden_l2;
+    wire->candidate_count = 0;
+    wire->overflow = 0;
+    top->best = 0;
+    top->blocks_done = 0;
+    top->failed = 0;
+  }
+
+  float best_lower = -CUDART_INF_F;
+  float mine = 0.0f, scale = 0.0f, residual = 0.0f;
+  for (int p = 0; p < steps; ++p) {
+    const int row = lo + kScanRows * p;
+    if (((kScanRows * p) & 31) == 0) {          // 32 rows from here on: this lane finishes row + lane
+      const int own = row + lane;
+      if (own < hi) { scale = __ldg(scales + own); residual = __ldg(residual_l2 + own); }
+    }
+    const int b = p % kScanBuffers;
+    if (!mbar_wait_bounded(bars + 8 * b, (p / kScanBuffers) & 1, abort_flag)) {
+      // the result is then reported as not certified; the copies under way have to land before the block leaves
+      if (lane == 0) top->failed = 1;
+      volatile int ignore = 0;
+      for (int q = p; q < min(steps, p + kScanBuffers); ++q)
+        mbar_wait_bounded(bars + 8 * (q % kScanBuffers), (q / kScanBuffers) & 1, &ignore);
+      break;
+    }
+    // (fewer rows left than the buffer holds: the rest of it are older rows, whose sums nobody takes)
+#pragma unroll
+    for (int r = 0; r < kScanRows; r += 2) {
+      const uint4* qa = reinterpret_cast<const uint4*>(buffers + b * kScanBufferBytes + r * kHidden) + lane;
+      const uint4* qb = qa + kHidden / 16;
+      float acc_a = 0.0f, acc_b = 0.0f;
+#pragma unroll
+      for (int piece = 0; piece < 4; ++piece) {
+        const uint4 wa = qa[32 * piece], wb = qb[32 * piece];
+        acc_a = fma_word(wa.x, x + 16 * piece, acc_a);
+        acc_b = fma_word(wb.x, x + 16 * piece, acc_b);
+        acc_a = fma_word(wa.y, x + 16 * piece + 4, acc_a);
+        acc_b = fma_word(wb.y, x + 16 * piece + 4, acc_b);
+        acc_a = fma_word(wa.z, x + 16 * piece + 8, acc_a);
+        acc_b = fma_word(wb.z, x + 16 * piece + 8, acc_b);
+        acc_a = fma_word(wa.w, x + 16 * piece + 12, acc_a);
+        acc_b = fma_word(wb.w, x + 16 * piece + 12, acc_b);
+      }
+      if (r + 2 == kScanRows) {
+        __syncwarp();                        // every lane has read the buffer
+        if (p + kScanBuffers < steps) request(p + kScanBuffers);
+      }
+      acc_a = butterfly_sum(acc_a);
+      acc_b = butterfly_sum(acc_b);
+      if (lane == ((kScanRows * p + r) & 31)) mine = acc_a;
+      if (lane == ((kScanRows * p + r + 1) & 31)) mine = acc_b;
+    }
+    if (((kScanRows * (p + 1)) & 31) == 0 || p + 1 == steps) {
+      const int own = lo + ((kScanRows * p) & ~31) + lane;
+      if (own < min(hi, row + kScanRows)) {
+        const float logit = __fmul_rn(mine, scale);
+        logits[own] = logit;
+        best_lower = fmaxf(best_lower, nextafterf(__fsub_rn(logit, row_error(residual, hidden_l2)), -CUDART_INF_F));
+      }
     }
   }
-}
-
-// every row whose upper bound reaches the largest lower bound is a candidate; each block first
-// reduces the 256 per-block maxima of the previous kernel
-__global__ void __launch_bounds__(kLmThreads)
-lm_head_collect_kernel(const float* __restrict__ logits, const float* __restrict__ residual_l2,
-                       const float* __restrict__ partial, aima_moe_lm_head_result* wire,
-                       uint32_t* __restrict__ candidate_ids, int rows) {
-  static_assert(kLmThreads == kLmBoundBlocks, "one thread per partial maximum");
-  __shared__ float reduction[kLmBoundBlocks];
-  pdl_enter();
-  reduction[threadIdx.x] = partial[threadIdx.x];
+#pragma unroll
+  for (int s = 16; s >= 1; s >>= 1) best_lower = fmaxf(best_lower, __shfl_xor_sync(0xffffffffu, best_lower, s));
+  if (lane == 0) warp_max[warp] = best_lower;
   __syncthreads();
-  for (int stride = kLmBoundBlocks / 2; stride != 0; stride >>= 1) {
-    if (threadIdx.x < stride) reduction[threadIdx.x] = fmaxf(reduction[threadIdx.x], reduction[threadIdx.x + stride]);
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kScanWarps; ++w) best_lower = fmaxf(best_lower, warp_max[w]);
+    partial[blockIdx.x] = best_lower;
   }
-  const float maximum_lower_bound = reduction[0];
-  if (blockIdx.x == 0 && threadIdx.x == 0) wire->maximum_lower_bound = maximum_lower_bound;
-  const int row = blockIdx.x * kLmThreads + threadIdx.x;
-  if (row >= rows) return;
-  const float upper = nextafterf(__fadd_rn(logits[row], row_error(residual_l2[row], wire->hidden_l2)), CUDART_INF_F);
-  if (upper < maximum_lower_bound) return;
-  const uint32_t slot = atomicAdd(&wire->candidate_count, 1u);
-  if (slot < AIMA_MOE_LM_HEAD_CANDIDATES) candidate_ids[slot] = static_cast<uint32_t>(row);
-  else wire->overflow = 1;
 }
 
-__device__ __forceinline__ bool better(float value, uint32_t index, float current, uint32_t current_index) {
-  return value > current || (value == current && index < current_index);
-}
-
-// One block: the exact BF16 logit of every candidate straight from the raw matrix (no gathered
-// copy) -- the canonical warp dot, rounded to BF16 like the reference's N = 1 GEMV provider -- then
-// the exact top-1 over them.  The exact logits replace the approximate ones in `logits`.
-constexpr int kExactWarps = 32;
-__global__ void __launch_bounds__(kExactWarps * 32)
-lm_head_exact_kernel(const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ hidden,
-                     aima_moe_lm_head_result* wire, const uint32_t* __restrict__ candidate_ids,
-                     float* __restrict__ logits) {
-  __shared__ float values[kExactWarps];
-  __shared__ uint32_t indices[kExactWarps];
+// Every row whose upper bound reaches the largest lower bound is a candidate.  The warp that finds one evaluates its
+// exact BF16 logit at once, straight from the raw matrix (no gathered copy, no list): the canonical warp dot, rounded to
+// BF16 like the reference's N = 1 GEMV provider.  The exact logit replaces the approximate one in `logits`; the largest --
+// equal ones: the lowest token id -- is kept in one 64-bit word, and the last block to finish publishes it.
+__global__ void __launch_bounds__(kLmThreads)
+lm_head_candidates_kernel(const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ hidden,
+                          const float* __restrict__ residual_l2, const float* __restrict__ partial, int partials,
+                          aima_moe_lm_head_result* wire, LmHeadTop* top, float* logits, int rows) {
+  __shared__ float reduction[kLmThreads / 32];
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
   pdl_enter();
-  const uint32_t count = min(wire->candidate_count, static_cast<uint32_t>(AIMA_MOE_LM_HEAD_CANDIDATES));
-  const uint4* xrow = reinterpret_cast<const uint4*>(hidden) + lane;
-  float local_value = -CUDART_INF_F;
-  uint32_t local_index = 0;
-  for (uint32_t candidate = warp; candidate < count; candidate += kExactWarps) {
-    const uint32_t token = candidate_ids[candidate];
+  const int row = blockIdx.x * kLmThreads + threadIdx.x;
+  const float logit = row < rows ? logits[row] : 0.0f;
+  const float residual = row < rows ? residual_l2[row] : 0.0f;
+  const float hidden_l2 = wire->hidden_l2;
+  float largest = -CUDART_INF_F;
+  for (int i = threadIdx.x; i < partials; i += kLmThreads) largest = fmaxf(largest, partial[i]);
+#pragma unroll
+  for (int s = 16; s >= 1; s >>= 1) largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, s));
+  if (lane == 0) reduction[threadIdx.x >> 5] = largest;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kLmThreads / 32; ++w) largest = fmaxf(largest, reduction[w]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) wire->maximum_lower_bound = largest;
+
+  bool candidate = false;
+  if (row < rows) {
+    const float upper = nextafterf(__fadd_rn(logit, row_error(residual, hidden_l2)), CUDART_INF_F);
+    candidate = !(upper < largest);
+  }
+  unsigned pending = __ballot_sync(0xffffffffu, candidate);
+  while (pending != 0u) {
+    const int owner = __ffs(pending) - 1;
+    pending &= pending - 1u;
+    const int token = __shfl_sync(0xffffffffu, row, owner);
+    uint32_t slot = 0;
+    if (lane == 0) slot = atomicAdd(&wire->candidate_count, 1u);
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+    if (slot >= AIMA_MOE_LM_HEAD_CANDIDATES) {
+      if (lane == 0) wire->overflow = 1;
+      continue;
+    }
     const uint4* wrow = reinterpret_cast<const uint4*>(weight + static_cast<size_t>(token) * kHidden) + lane;
+    const uint4* xrow = reinterpret_cast<const uint4*>(hidden) + lane;
+    uint4 w[kHidden / 256];
+#pragma unroll
+    for (int i = 0; i < kHidden / 256; ++i) w[i] = __ldg(wrow + i * 32);
     float acc = 0.0f;
 #pragma unroll
     for (int i = 0; i < kHidden / 256; ++i) {
       float xf[8];
       unpack8(__ldg(xrow + i * 32), xf);
-      acc = fma8(xf, __ldg(wrow + i * 32), acc);
+      acc = fma8(xf, w[i], acc);
     }
-    acc = butterfly_sum(acc);
-    const float value = round_bf16(acc);
-    if (lane == 0) logits[token] = value;
-    if (better(value, token, local_value, local_index)) { local_value = value; local_index = token; }
-  }
-  if (lane == 0) { values[warp] = local_value; indices[warp] = local_index; }
-  __syncthreads();
-  if (warp == 0) {
-    float value = values[lane];
-    uint32_t index = indices[lane];
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-      const float other_value = __shfl_xor_sync(0xffffffffu, value, offset);
-      const uint32_t other_index = __shfl_xor_sync(0xffffffffu, index, offset);
-      if (better(other_value, other_index, value, index)) { value = other_value; index = other_index; }
-    }
+    const float value = round_bf16(butterfly_sum(acc));
     if (lane == 0) {
-      wire->exact_top1_logit = value;
-      wire->exact_top1_token_id = index;
+      logits[token] = value;
+      if (value > -CUDART_INF_F) {       // neither -inf nor NaN ever wins
+        const uint32_t bits = __float_as_uint(value == 0.0f ? 0.0f : value);      // -0 ties with +0
+        const uint32_t key = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
+        atomicMax(&top->best, (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<uint32_t>(token)));
+      }
     }
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&top->blocks_done, 1u) + 1 == gridDim.x) {
+    __threadfence();
+    const unsigned long long best = atomicAdd(&top->best, 0ull);
+    const uint32_t token = best != 0 ? 0xffffffffu - static_cast<uint32_t>(best) : 0u;
+    wire->exact_top1_token_id = token;
+    wire->exact_top1_logit = best != 0 ? __ldcg(logits + token) : -CUDART_INF_F;
+    if (top->failed != 0) wire->overflow = 1;
   }
 }
 
@@ -308,20 +348,18 @@ cudaError_t lm_head_quantize(const void* weight, int rows, int8_t* q_weight, flo
 cudaError_t lm_head_certify(const LmHeadBuffers& b, const void* weight, const void* hidden, float* logits,
                             int rows, int sm_count, cudaStream_t stream, int* launches) {
   const __nv_bfloat16* h = static_cast<const __nv_bfloat16*>(hidden);
-  lm_head_scan_kernel<<<sm_count * 16, kScanWarps * 32, 0, stream>>>(b.q_weight, b.scales, h, logits, rows);
-  cudaError_t code = cudaGetLastError();
+  cudaError_t code = opt_in_dynamic_smem<lm_head_scan_kernel>(kScanSmemBytes);
+  if (code != cudaSuccess) return code;
+  const int blocks = sm_count < kLmMaxScanBlocks ? sm_count : kLmMaxScanBlocks;
+  lm_head_scan_kernel<<<blocks, kScanWarps * 32, kScanSmemBytes, stream>>>(b.q_weight, b.scales, b.residual_l2, h, logits,
+                                                                           b.wire, b.top, b.partial, rows);
+  code = cudaGetLastError();
   const PdlScope pdl_scope(true);
   if (code == cudaSuccess)
-    code = launch_pdl(lm_head_bound_kernel, dim3(kLmBoundBlocks), dim3(kLmThreads), 0, stream,
-                      static_cast<const float*>(logits), static_cast<const float*>(b.residual_l2), h, b.wire, b.partial, rows);
-  if (code == cudaSuccess)
-    code = launch_pdl(lm_head_collect_kernel, dim3((rows + kLmThreads - 1) / kLmThreads), dim3(kLmThreads), 0, stream,
-                      static_cast<const float*>(logits), static_cast<const float*>(b.residual_l2),
-                      static_cast<const float*>(b.partial), b.wire, b.candidate_ids, rows);
-  if (code == cudaSuccess)
-    code = launch_pdl(lm_head_exact_kernel, dim3(1), dim3(kExactWarps * 32), 0, stream,
-                      static_cast<const __nv_bfloat16*>(weight), h, b.wire, b.candidate_ids, logits);
-  *launches = 4;
+    code = launch_pdl(lm_head_candidates_kernel, dim3((rows + kLmThreads - 1) / kLmThreads), dim3(kLmThreads), 0, stream,
+                      static_cast<const __nv_bfloat16*>(weight), h, static_cast<const float*>(b.residual_l2),
+                      static_cast<const float*>(b.partial), blocks, b.wire, b.top, logits, rows);
+  *launches = 2;
   return code;
 }
 

@@ -6,19 +6,28 @@
 
 namespace aima {
 
+constexpr int kLmMaxScanBlocks = 256;
+
+// State of one launch beside the published result.
+struct LmHeadTop {
+  unsigned long long best;          // largest exact logit: order-preserving bits, then the complement of the token id
+  uint32_t blocks_done;             // blocks of the candidate kernel that have finished
+  uint32_t failed;                  // a bounded wait of the scan ran out
+};
+
 struct LmHeadBuffers {
   int8_t* q_weight;                 // [rows, 2048]
   float* scales;                    // [rows]
   float* residual_l2;               // [rows]
   aima_moe_lm_head_result* wire;    // device copy of the result
-  float* partial;                   // [256] per-block maxima of the lower bounds
-  uint32_t* candidate_ids;          // [AIMA_MOE_LM_HEAD_CANDIDATES]
+  LmHeadTop* top;
+  float* partial;                   // [kLmMaxScanBlocks] per-block maxima of the lower bounds
 };
 
 cudaError_t lm_head_quantize(const void* weight, int rows, int8_t* q_weight, float* scales, float* residual_l2,
                              cudaStream_t stream);
 
-// Enqueues the scan, the bounds, the candidate collection and the exact candidate logits with their arg-max.
+// Enqueues the scan with the bounds, and the candidates with their exact logits and arg-max.
 cudaError_t lm_head_certify(const LmHeadBuffers& buffers, const void* weight, const void* hidden, float* logits,
                             int rows, int sm_count, cudaStream_t stream, int* launches);
 

@@ -11,7 +11,8 @@ struct aima_moe_lm_head {
   int sm_count = 0;
   uint32_t rows = 0;
   const void* weight = nullptr;      // caller-owned raw BF16 matrix [rows, 2048]
-  void* allocation = nullptr;        // q | scales | residual_l2 | wire | partial | candidate ids
+  void* allocation = nullptr;        // q | scales | residual_l2 | wire | top | partial
+  aima_moe_lm_head_result* host_result = nullptr;      // pinned
   aima::LmHeadBuffers buffers{};
   cudaStream_t last_stream = nullptr;
   uint64_t launches = 0;
@@ -77,20 +78,22 @@ AIMA_EXPORT int aima_moe_lm_head_build(const void* weight_bf16, uint32_t rows, a
   handle->weight = weight_bf16;
   const size_t q_bytes = align256(static_cast<size_t>(rows) * aima::kHidden);
   const size_t row_bytes = align256(static_cast<size_t>(rows) * sizeof(float));
-  const size_t total = q_bytes + 2 * row_bytes + 256 + 1024 +
-                       align256(AIMA_MOE_LM_HEAD_CANDIDATES * sizeof(uint32_t));
+  const size_t total = q_bytes + 2 * row_bytes + 256 + 256 +
+                       aima::kLmMaxScanBlocks * sizeof(float);
   error = cudaMalloc(&handle->allocation, total);
+  if (error == cudaSuccess) error = cudaMallocHost(&handle->host_result, sizeof *handle->host_result);
   if (error != cudaSuccess) {
+    cudaFree(handle->allocation);
     delete handle;
-    return lm_fail_cuda(error, "cudaMalloc lm head");
+    return lm_fail_cuda(error, "allocation of the lm head");
   }
   uint8_t* cursor = static_cast<uint8_t*>(handle->allocation);
   handle->buffers.q_weight = reinterpret_cast<int8_t*>(cursor); cursor += q_bytes;
   handle->buffers.scales = reinterpret_cast<float*>(cursor); cursor += row_bytes;
   handle->buffers.residual_l2 = reinterpret_cast<float*>(cursor); cursor += row_bytes;
   handle->buffers.wire = reinterpret_cast<aima_moe_lm_head_result*>(cursor); cursor += 256;
-  handle->buffers.partial = reinterpret_cast<float*>(cursor); cursor += 1024;
-  handle->buffers.candidate_ids = reinterpret_cast<uint32_t*>(cursor);
+  handle->buffers.top = reinterpret_cast<aima::LmHeadTop*>(cursor); cursor += 256;
+  handle->buffers.partial = reinterpret_cast<float*>(cursor);
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
   error = cudaMemsetAsync(handle->buffers.wire, 0, 256, cuda_stream);
   if (error == cudaSuccess)
@@ -98,6 +101,7 @@ AIMA_EXPORT int aima_moe_lm_head_build(const void* weight_bf16, uint32_t rows, a
                                    handle->buffers.scales, handle->buffers.residual_l2, cuda_stream);
   if (error != cudaSuccess) {
     cudaFree(handle->allocation);
+    cudaFreeHost(handle->host_result);
     delete handle;
     return lm_fail_cuda(error, "lm head quantisation");
   }
@@ -139,10 +143,18 @@ AIMA_EXPORT int aima_moe_lm_head_read_result(aima_moe_lm_head* handle, aima_moe_
   if (handle == nullptr || result == nullptr)
     return lm_fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "lm head: handle or result is null");
   std::lock_guard<std::mutex> lock(handle->mutex);
-  cudaError_t error = cudaStreamSynchronize(handle->last_stream);
+  // On the handle's own device the copy goes through the legacy stream, which by itself waits for every ordinary stream; only a stream created
+  // non-blocking has to be waited for first.  Into pinned memory it is one request and one wait.
+  unsigned flags = 0;
+  int device = -1;
+  cudaError_t error = cudaGetDevice(&device);
+  if (error == cudaSuccess) error = cudaStreamGetFlags(handle->last_stream, &flags);
+  if (error == cudaSuccess && (device != handle->device || (flags & cudaStreamNonBlocking) != 0)) error = cudaStreamSynchronize(handle->last_stream);
   if (error != cudaSuccess) return lm_fail_cuda(error, "cudaStreamSynchronize");
-  error = cudaMemcpy(result, handle->buffers.wire, sizeof *result, cudaMemcpyDeviceToHost);
-  if (error != cudaSuccess) return lm_fail_cuda(error, "cudaMemcpy lm head result");
+  error = cudaMemcpyAsync(handle->host_result, handle->buffers.wire, sizeof *result, cudaMemcpyDeviceToHost, cudaStreamLegacy);
+  if (error == cudaSuccess) error = cudaStreamSynchronize(cudaStreamLegacy);
+  if (error != cudaSuccess) return lm_fail_cuda(error, "copy of the lm head result");
+  *result = *handle->host_result;
   if (result->overflow != 0)
     return lm_fail(AIMA_MOE_ERR_CAPACITY, "lm head: more than 1024 candidates, the top-1 is not certified");
   return AIMA_MOE_OK;
@@ -151,6 +163,7 @@ AIMA_EXPORT int aima_moe_lm_head_read_result(aima_moe_lm_head* handle, aima_moe_
 AIMA_EXPORT int aima_moe_lm_head_release(aima_moe_lm_head* handle) {
   if (handle == nullptr) return AIMA_MOE_OK;
   cudaFree(handle->allocation);
+  cudaFreeHost(handle->host_result);
   delete handle;
   return AIMA_MOE_OK;
 }

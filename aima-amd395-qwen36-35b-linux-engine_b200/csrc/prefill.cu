@@ -435,6 +435,83 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
   }
 }
 
+// ---------------------------------------------------------------------------
+// Router of a short call: all 256 canonical logits straight away, spread over the chip by EXPERT -- a block holds two
+// router rows in registers and walks the tokens -- then one warp per token selects.  The tensor-core filter needs the
+// whole router matrix in each 32-token tile and then a chain of dependent loads per token: 20 + 13 us at 16 tokens,
+// whatever their number, against 17 us for both here.
+// ---------------------------------------------------------------------------
+constexpr int kSmallRouterTokens = 128;
+
+__global__ void __launch_bounds__(256, 1)
+prefill_logits_small_kernel(const __nv_bfloat16* __restrict__ h2, const __nv_bfloat16* __restrict__ router,
+                            const __nv_bfloat16* __restrict__ shared_gate, int tokens, float* __restrict__ logits,
+                            float* __restrict__ shared_sigmoid) {
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const bool gate = blockIdx.x == kExperts / 2;              // the last block: the shared expert's gate row
+  pdl_enter();
+  const uint4* row0 = reinterpret_cast<const uint4*>(gate ? shared_gate : router + static_cast<size_t>(2 * blockIdx.x) * kHidden) + lane;
+  const uint4* row1 = gate ? row0 : row0 + kHidden / 8;
+  auto token_row = [&](int t) { return reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(t) * kHidden) + lane; };
+  uint4 next[8];
+  if (warp < tokens) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) next[i] = __ldg(token_row(warp) + i * 32);
+  }
+  float w0[64], w1[64];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    unpack8(__ldg(row0 + i * 32), w0 + 8 * i);
+    unpack8(__ldg(row1 + i * 32), w1 + 8 * i);
+  }
+  for (int t = warp; t < tokens; t += 8) {
+    uint4 x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = next[i];
+    if (t + 8 < tokens) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) next[i] = __ldg(token_row(t + 8) + i * 32);
+    }
+    float a = 0.0f, b = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      a = fma8(w0 + 8 * i, x[i], a);
+      b = fma8(w1 + 8 * i, x[i], b);
+    }
+    a = butterfly_sum(a);
+    b = butterfly_sum(b);
+    if (lane == 0) {
+      if (gate) shared_sigmoid[t] = round_bf16(det_sigmoid(round_bf16(a)));
+      else *reinterpret_cast<float2*>(logits + static_cast<size_t>(t) * kExperts + 2 * blockIdx.x) = make_float2(a, b);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kCertWarps * 32)
+prefill_select_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int quant_eighths, int tokens,
+                      int32_t* __restrict__ ids, float* __restrict__ scores, float* __restrict__ weights,
+                      __nv_bfloat16* __restrict__ dbg_weights, int32_t* __restrict__ stats) {
+  __shared__ float sel_v_s[kCertWarps * 8];
+  __shared__ int sel_i_s[kCertWarps * 8];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int token = blockIdx.x * kCertWarps + warp;
+  pdl_enter();
+  if (token >= tokens) return;
+  float v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    v[q] = finish_logit(logits[static_cast<size_t>(token) * kExperts + 32 * q + lane],
+                        bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths);
+  route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
+              ids, scores, weights, dbg_weights);
+  if (lane == 0) {
+    atomicAdd(stats, kExperts);
+    atomicAdd(stats + 1, 1);
+  }
+}
+
 // Euclidean norms of the 256 router rows, rounded up a little; one warp per row.
 __global__ void __launch_bounds__(256)
 router_row_norms_kernel(const __nv_bfloat16* __restrict__ router, float* __restrict__ norms) {
@@ -476,7 +553,7 @@ constexpr int kPlanBlocks = 8;
 constexpr int kPlanWarps = 32;
 constexpr int kPlanRounds = 8;      // rounds of 32 rows whose ids are requested together
 
-__global__ void __cluster_dims__(kPlanBlocks, 1, 1) __launch_bounds__(kPlanWarps * 32)
+__global__ void __cluster_dims__(kPlanBlocks, 1, 1) __launch_bounds__(kPlanWarps * 32, 1)
 plan_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int expert_hi, int tile_cap,
             int32_t* __restrict__ expert_counts, int32_t* __restrict__ expert_offsets,
             int32_t* __restrict__ tile_expert, int32_t* __restrict__ tile_row0, int32_t* __restrict__ tile_rows,
@@ -1047,6 +1124,16 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
         dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr);
     if ((code = cudaGetLastError()) != cudaSuccess) return set_error(error, error_bytes, code, "prefill_router_kernel");
     ++count;
+  } else if (T <= kSmallRouterTokens && ws->router_audit_stride == 0) {
+    code = launch_pdl(prefill_logits_small_kernel, dim3(kExperts / 2 + 1), dim3(256), 0, stream, h2, call.layer.router,
+                      call.layer.shared_gate, T, ws->approx_logits, ws->shared_sigmoid);
+    if (code == cudaSuccess)
+      code = launch_pdl(prefill_select_kernel, dim3((T + kCertWarps - 1) / kCertWarps), dim3(kCertWarps * 32), 0, stream,
+                        static_cast<const float*>(ws->approx_logits), call.router_bias, call.quant_eighths, T,
+                        ws->topk_ids, ws->topk_scores, ws->topk_weights,
+                        dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr, ws->router_stats);
+    if (code != cudaSuccess) return set_error(error, error_bytes, code, "router of a short call");
+    count += 2;
   } else {
     // tensor-core logits for the candidate filter, then exact recomputation of the candidates
     GroupedGemm r{};

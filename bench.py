@@ -748,7 +748,7 @@ def run_lm_head(args) -> None:
                      "traffic": None, "peak_source": kind, "bytes_per_step": step_bytes},
         "e2e": {"value": 1.0e3 / e2e_ms, "unit": "tokens/s", "h2d_bytes_per_step": HIDDEN * 2,
                 "d2h_bytes_per_step": 24},
-        "candidates_last_step": int(result.candidate_count), "gpu_launches": 4 * steps, "clocks": clocks,
+        "candidates_last_step": int(result.candidate_count), "gpu_launches": 2 * steps, "clocks": clocks,
         **({"cpu_baseline": baseline} if baseline is not None else {})}))
 
 
