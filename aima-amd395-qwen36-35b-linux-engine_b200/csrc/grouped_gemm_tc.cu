@@ -7,12 +7,16 @@
 // (:384-402), and the five hipBLASLt plans of the shared expert with their
 // pointwise kernels (:790-826) -- the epilogues are fused.
 //
+// Two kernels.  The two-SM one (grouped_gemm_pair_kernel, below) runs the expert, shared-expert, dense and router-logits
+// products of one GPU.  The one-SM one, described here, serves expert parallelism (its epilogue stores to peers, and its
+// launches can be split into parts).
+//
 // Work unit = one 128-row tile of one expert x one 256-wide slice of the output
 // columns.  D[128, 256] (FP32) lives in tensor memory, two buffers of 256
 // columns, so the epilogue of a unit overlaps the main loop of the next.
 //   warp 0   TMA producer: per 64-wide K block one 128x64 tile of A and two
 //            128x64 tiles of B into a 4-stage shared-memory ring (128-byte swizzle)
-//   warp 1   one thread issues tcgen05.mma (M128 N256 K16, 4 per K block) and
+//   warp 1   issues tcgen05.mma (M128 N256 K16, 4 per K block) and
 //            commits to the ring's "empty" barriers / the accumulator's "full" barrier
 //   warp 2   allocates and frees the 512 tensor-memory columns
 //   warps 2-3 with fused dispatch (gate_up only): gather the tile's 128 activation rows BY TOKEN
@@ -630,6 +634,8 @@ __device__ __forceinline__ uint32_t pair_instr_desc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | ((256u >> 4) << 24);
 }
 __host__ __device__ inline int pair_width(int rows) { return (rows + 31) & ~31; }
+// groups of four rows a block gathers for `rows` rows of its own (<= 0: none): one for each gather warp at least
+__device__ __forceinline__ int gather_fours(int rows) { return max(2, (rows + 3) / 4); }
 
 // 16 lanes x 32 columns of the accumulator in the fragment layout: v[4 i + 2 p + c] of thread t is lane t / 4 + 8 p,
 // column 8 i + 2 (t % 4) + c
@@ -890,7 +896,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       const int w_row = u.expert * pb.b_rows_per_expert + u.chunk * kPairN + static_cast<int>(rank) * 128;
       // what both blocks fetch for a stage: weights, and the tile's rows (gathered: in fours per block)
       uint32_t stage_bytes = 2 * (kStage2ABytes + half * kBK * 2);
-      if (kGather) stage_bytes = 2 * kStage2ABytes + ((min(half, u.rows) + 3) / 4 + (max(0, u.rows - half) + 3) / 4) * (4 * kBK * 2);
+      if (kGather) stage_bytes = 2 * kStage2ABytes + (gather_fours(min(half, u.rows)) + gather_fours(u.rows - half)) * (4 * kBK * 2);
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
         if (elect_one()) {
@@ -929,8 +935,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   } else if (kGather && (warp == 2 || warp == 3)) {
     // ------------------------------ row gather (both blocks) -------------------
     // Rows by token index, four per TMA instruction (tile::gather4, a box of one row), the two warps in turn.  Only rows
-    // that exist are fetched, up to three repeats of the last one; what a stage holds beyond them ends in accumulator
-    // columns that nobody reads.  The tile's token indices wait in shared memory, one private copy per warp.
+    // that exist are fetched, the last group filled up with repeats; what a stage holds beyond them ends in accumulator
+    // columns that nobody reads.  Each warp fetches at least one group per stage, an unneeded one if the tile has no row
+    // for it: a stage then always waits for both, so that neither can fall behind the ring or run ahead of it by a whole
+    // round, which a barrier's parity would not tell.  (One warp for all groups, or the warp that loads the weights, is
+    // slower: 456 against 380 us per layer at 2048 tokens.)  The tile's token indices wait in shared memory, one private
+    // copy per warp.
     int4* table = reinterpret_cast<int4*>(gather_tables + (warp - 2) * kGatherTableBytes);
     const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
     int stage = 0;
@@ -941,10 +951,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       const int half = pair_width(u.rows) / 2;
       const int mine = max(0, min(half, u.rows - static_cast<int>(rank) * half));
       int4 t = make_int4(0, 0, 0, 0);
-      if (4 * lane < mine) {
+      if (mine > 0 && lane < gather_fours(mine)) {
         const int first = u.row0 + static_cast<int>(rank) * half;
         auto flat = [&](int r) { return u.expert < 0 ? (first + r) << 3 : g.sorted_rows[first + r]; };
-        t.x = flat(4 * lane);
+        t.x = flat(min(4 * lane, mine - 1));
         t.y = flat(min(4 * lane + 1, mine - 1));
         t.z = flat(min(4 * lane + 2, mine - 1));
         t.w = flat(min(4 * lane + 3, mine - 1));
@@ -960,7 +970,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       next_tokens = tokens(next);
       later = describe(unit + 2 * n_pairs);
       const int half = pair_width(u.rows) / 2;
-      const int fours = (max(0, min(half, u.rows - static_cast<int>(rank) * half)) + 3) / 4;
+      const int fours = gather_fours(min(half, u.rows - static_cast<int>(rank) * half));
       __syncwarp();
       table[lane] = make_int4(t4.x >> 3, t4.y >> 3, t4.z >> 3, t4.w >> 3);
       __syncwarp();
