@@ -85,9 +85,8 @@ typedef struct aima_moe_config {
  * FP32 dot instead of filtering candidates with tensor-core logits first. */
 #define AIMA_MOE_FLAG_EXACT_ROUTER 2u
 /* Prefill, for A/B timing and qualification: copy the routed activation rows into expert order first
- * (one materialised copy read by tiled TMA loads) instead of letting the gate_up tensor-core kernel
- * gather them by token index itself.  Same bits; the default (fused dispatch) saves the copy kernel
- * and 0.5 GB of traffic per T = 8192 layer. */
+ * (one materialised copy read by tiled TMA loads) for every call.  By default the gate_up tensor-core kernel
+ * gathers them by token index itself in calls of up to 3584 tokens; longer calls copy.  Same bits. */
 #define AIMA_MOE_FLAG_MATERIALIZED_DISPATCH 8u
 /* Expert-parallel prefill: split the plan's tiles into 2 (or 4) parts and, with copy kernels on two more
  * streams, put the rows of one part into expert order / store the results of another back to their owners
@@ -100,10 +99,8 @@ typedef struct aima_moe_config {
  * the reference's certified LM head, native/src/native_lm_head_certificate.hip.cpp:33-39, applied to
  * the router; the reference's own router has no filter to audit.) */
 #define AIMA_MOE_FLAG_AUDIT_ROUTER 256u
-/* Prefill, for A/B timing and qualification: run the expert products in the two-SM form
- * (tcgen05.mma.cta_group::2, a pair of blocks per 256-row tile, each block staging its 128 rows and its half
- * of the weights) instead of the default one-SM form (128-row tiles, one block per tile).  Same bits; on the
- * measured workloads the default is as fast or faster.  Single GPU only. */
+/* Accepted and without effect: with one GPU the expert products always run in the two-SM form
+ * (tcgen05.mma.cta_group::2); expert parallelism uses the one-SM form.  Same bits in both. */
 #define AIMA_MOE_FLAG_TWO_SM_PRODUCTS 512u
 /* Decode, for A/B timing and qualification: do not predict the next layer's experts (its router applied
  * to the current layer's input) and do not request their rows ahead of the routing.  Same bits either
