@@ -1289,7 +1289,7 @@ cudaError_t launch_grouped_gemm_tc(GemmMode mode, const GroupedGemm& g, const Tc
     case kGemmSharedGateUp: return launch_mode<kGemmSharedGateUp>(maps, pb, grid, stream);
     case kGemmExpertDown: return launch_mode<kGemmExpertDown>(maps, pb, grid, stream);
     case kGemmSharedDown: return launch_mode<kGemmSharedDown>(maps, pb, grid, stream);
-    case kGemmPlain: return launch_mode<kGemmPlain>(maps, pb, grid, stream);
+    case kGemmPlain: break;              // two-SM form only
     case kGemmPlainF32: return launch_mode<kGemmPlainF32>(maps, pb, grid, stream);
   }
   return cudaErrorInvalidValue;
