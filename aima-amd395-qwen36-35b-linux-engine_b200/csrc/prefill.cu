@@ -59,7 +59,8 @@ __device__ __forceinline__ float warp_eighth_largest(const float* v, int lane) {
 
 // The reference's prefill selection on the final (BF16-rounded) logits of one
 // token held as v[q] = logit of expert 32 q + lane: threshold, gather in expert
-// order, fixed bitonic network, softmax; lanes 0..7 write slot `lane`.  `threshold` is the 8th largest of the values.
+// order, fixed bitonic network, softmax; lanes 0..7 write slot `lane`.  `threshold` is the 8th largest of the values, none
+// of which may be a NaN (selectable): then at least eight of them reach it and every slot is written.
 __device__ __forceinline__ int route_token(const float* v, float threshold, int lane, float* sel_v, int* sel_i,
                                             size_t token, int32_t* __restrict__ ids,
                                             float* __restrict__ scores, float* __restrict__ weights,
@@ -141,13 +142,18 @@ __device__ __forceinline__ int route_token(const float* v, float threshold, int 
   return selected;
 }
 
-// logit transform shared by both router kernels: optional harness hooks, then
+// logit transform shared by the router kernels: optional harness hooks, then
 // the BF16 rounding the reference's router GEMM applies
 __device__ __forceinline__ float finish_logit(float x, float bias, int quant_eighths) {
   x = __fadd_rn(x, bias);
   if (quant_eighths) x = __fmul_rn(rintf(__fmul_rn(x, 8.0f)), 0.125f);
   return round_bf16(x);
 }
+
+// What the selection sees of a logit.  A NaN compares false with every threshold, so route_token would leave slots
+// unwritten and the plan would lose rows; counted as -inf it loses to every number, and a token with fewer than eight
+// numbers still gets eight valid experts (the lowest ids among the rest).
+__device__ __forceinline__ float selectable(float logit) { return logit == logit ? logit : -CUDART_INF_F; }
 
 // ---------------------------------------------------------------------------
 // Router: canonical FP32 logits of all 256 experts (+ the shared-expert gate
@@ -229,6 +235,7 @@ prefill_router_kernel(const __nv_bfloat16* __restrict__ h2,
   for (int q = 0; q < 8; ++q) {
     v[q] = finish_logit(v[q], bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths);
     if (dbg_logits != nullptr) dbg_logits[static_cast<size_t>(token) * kExperts + 32 * q + lane] = v[q];
+    v[q] = selectable(v[q]);
   }
   route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
               ids, scores, weights, dbg_weights);
@@ -359,8 +366,8 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
     }
     acc0 = butterfly_sum(acc0);
     acc1 = butterfly_sum(acc1);
-    const float f0 = finish_logit(acc0, bias != nullptr ? __ldg(bias + e0) : 0.0f, quant_eighths);
-    const float f1 = finish_logit(acc1, bias != nullptr && e1 >= 0 ? __ldg(bias + e1) : 0.0f, quant_eighths);
+    const float f0 = selectable(finish_logit(acc0, bias != nullptr ? __ldg(bias + e0) : 0.0f, quant_eighths));
+    const float f1 = selectable(finish_logit(acc1, bias != nullptr && e1 >= 0 ? __ldg(bias + e1) : 0.0f, quant_eighths));
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       if (e0 == 32 * q + lane) v[q] = f0;
@@ -502,8 +509,8 @@ prefill_select_kernel(const float* __restrict__ logits, const float* __restrict_
   float v[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q)
-    v[q] = finish_logit(logits[static_cast<size_t>(token) * kExperts + 32 * q + lane],
-                        bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths);
+    v[q] = selectable(finish_logit(logits[static_cast<size_t>(token) * kExperts + 32 * q + lane],
+                                   bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths));
   route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
               ids, scores, weights, dbg_weights);
   if (lane == 0) {
@@ -694,14 +701,15 @@ cudaError_t launch_plan(PrefillWorkspace* ws, const int32_t* ids, int rows, int 
 }
 
 // ---------------------------------------------------------------------------
-// Gather of h2 rows into expert order; one warp per routed row.
+// Gather of h2 rows into expert order; one warp per routed row.  It ends where the plan does (expert_offsets[256]):
+// beyond that sorted_rows would hold what an earlier call left there.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const __nv_bfloat16* __restrict__ h2, const int32_t* __restrict__ sorted_rows,
-                   int routed_rows, __nv_bfloat16* __restrict__ gathered) {
+                   const int32_t* __restrict__ expert_offsets, __nv_bfloat16* __restrict__ gathered) {
   const int lane = threadIdx.x & 31;
   const int pos = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (pos >= routed_rows) return;
+  if (pos >= expert_offsets[kExperts]) return;
   const int token = sorted_rows[pos] >> 3;
   const uint4* src = reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(token) * kHidden);
   uint4* dst = reinterpret_cast<uint4*>(gathered + static_cast<size_t>(pos) * kHidden);
@@ -1174,7 +1182,7 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   const bool fused_dispatch = ws->fused_dispatch && !simt && T <= kGatherMaxTokens;
   if (!fused_dispatch) {
     gather_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(call.h2), ws->sorted_rows, rows, ws->gathered);
+        static_cast<const __nv_bfloat16*>(call.h2), ws->sorted_rows, ws->expert_offsets, ws->gathered);
     if ((code = cudaGetLastError()) != cudaSuccess) return set_error(error, error_bytes, code, "gather_rows_kernel");
     ++count;
   }

@@ -119,3 +119,49 @@ def test_lm_head_rows_at_the_ends_of_copies_and_runs(package, oracle, rows):
             assert torch.equal(logits.cpu(), want["logits"])
     finally:
         head.release()
+
+
+@pytest.mark.parametrize("flag", [None, "FLAG_MATERIALIZED_DISPATCH", "FLAG_EXACT_ROUTER"])
+def test_nan_logits_of_a_short_call_stay_in_their_row(package, oracle, gpu_layers, synth, flag):
+    """After a longer call on the same handle: a row of NaN gets the eight lowest experts (all its logits count as -inf) and
+    leaves its neighbours' bits alone; a router row with a NaN, one logit of every token, is as good as -inf there."""
+    device = torch.device("cuda", 0)
+    weights = gpu_layers(0)["cuda"]
+    broken = dict(weights, router=weights["router"].clone())
+    broken["router"][77, 5] = float("nan")
+    tokens, bad, longer = 40, 7, 300
+    h2 = synth.activations(SEED, longer, "input", 0).to(device)
+    resid = synth.activations(SEED, longer, "residual", 0).to(device)
+    with_nan = h2[:tokens].clone()
+    with_nan[bad] = float("nan")
+    provider = package.MoeProvider(layers=2, max_prefill_tokens=longer, flags=getattr(package.provider, flag) if flag else 0)
+    try:
+        provider.bind_layer(0, weights)
+        provider.bind_layer(1, broken)
+
+        def call(x, layer=0):
+            views, dbg = provider.make_debug(len(x), prefill=True, with_logits=False)
+            out = provider.launch_selected_moe(post_attention=x, residual_hidden=resid[:len(x)], model_layer=layer, debug=views)
+            provider.sync_metrics()
+            return out, dbg
+
+        clean, clean_dbg = call(h2[:tokens])
+        call(h2)
+        got, dbg = call(with_nan)
+        others = [t for t in range(tokens) if t != bad]
+        assert torch.equal(got[others], clean[others])
+        assert torch.equal(dbg["topk_ids"][others], clean_dbg["topk_ids"][others])
+        assert sorted(dbg["topk_ids"][bad].tolist()) == list(range(8))      # (the fixed network permutes equal scores)
+        assert torch.isnan(got[bad]).all()
+        assert int(dbg["expert_offsets"][256]) == tokens * 8
+        assert torch.equal(dbg["sorted_rows"].sort().values.cpu(), torch.arange(tokens * 8, dtype=torch.int32))
+        call(h2)
+        _, dbg = call(h2[:tokens], layer=1)
+    finally:
+        provider.release()
+    bias = torch.zeros(256)
+    bias[77] = float("-inf")
+    want = oracle.router_prefill(h2[:tokens].cpu(), oracle.OracleLayer(gpu_layers(0)["cpu"], router_bias=bias))
+    assert torch.equal(dbg["topk_ids"].cpu(), want["ids"])
+    assert torch.equal(dbg["topk_scores"].cpu(), want["scores"])
+    assert torch.equal(dbg["topk_weights"].cpu(), want["weights"])
