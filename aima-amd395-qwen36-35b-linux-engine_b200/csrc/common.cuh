@@ -315,6 +315,27 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   return mbar_wait_bounded_slow(bar, parity, abort_flag, diag);
 }
 
+// The same for a converged warp whose 32 lanes go on together (elect.sync, tcgen05 and shuffles with a full mask follow):
+// every look at the barrier, the flag and the clock is a vote, so all lanes leave with one verdict.  A wait that each lane
+// decided for itself could end true in some and false in others when the phase completes while the limit runs out, and the
+// two groups would then wait for each other without one.  One probe inline: it suspends the warp for up to 4 us by itself.
+static __device__ __noinline__ bool mbar_wait_bounded_warp_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                                unsigned long long limit_ns) {
+  const unsigned long long start = global_timer_ns();
+  while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
+    if (__any_sync(0xffffffffu, *abort_flag != 0 || global_timer_ns() - start > limit_ns)) {
+      *abort_flag = kStatusTimeoutMbarrier;
+      return false;
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool mbar_wait_bounded_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                       unsigned long long limit_ns = kWaitBudgetNs) {
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  return mbar_wait_bounded_warp_slow(bar, parity, abort_flag, limit_ns);
+}
+
 // Programmatic dependent launch.  A kernel launched with launch_pdl may have its blocks placed
 // while the kernel before it in the stream is still running; it must call pdl_enter() before its
 // first access to global memory: that waits until the predecessor has completed and its writes are

@@ -402,7 +402,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
         b1_row = b0_row + kBN / 2;
       }
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
         if (elect_one()) {
           const uint32_t a_dst = smem_base + stage * kStageBytes;
           const uint32_t b_dst = a_dst + kStageABytes;
@@ -472,11 +472,11 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
       // the epilogue must have drained this accumulator buffer (first use: free)
-      if (!mbar_wait_bounded(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+      if (!mbar_wait_bounded_warp(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
       tc_fence_after();
       const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kBN);
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
         if (kGather) fence_async_proxy();     // rows written by cp.async are read through the async proxy
         tc_fence_after();
         if (elect_one()) {
@@ -507,7 +507,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
       unit_tile(unit, tile, chunk, expert, row0, rows);
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
-      if (!mbar_wait_bounded(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
+      if (!mbar_wait_bounded_warp(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
       tc_fence_after();
       drain_accumulator<MODE>(g, pb, tmem_base, buf, ew, eh, lane,
                               smem_gen + kStages * kStageBytes + 256 + (warp - 4) * kStoreStageBytes, chunk, row0, rows);
@@ -898,7 +898,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       uint32_t stage_bytes = 2 * (kStage2ABytes + half * kBK * 2);
       if (kGather) stage_bytes = 2 * kStage2ABytes + (gather_fours(min(half, u.rows)) + gather_fours(u.rows - half)) * (4 * kBK * 2);
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
         if (elect_one()) {
           const uint32_t w_dst = smem_base + stage * kStage2Bytes;
           const uint32_t leader_full = leader_full0 + 8u * stage;
@@ -975,7 +975,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       table[lane] = make_int4(t4.x >> 3, t4.y >> 3, t4.z >> 3, t4.w >> 3);
       __syncwarp();
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
         const uint32_t dst = smem_base + stage * kStage2Bytes + kStage2ABytes;
         const uint32_t leader_full = leader_full0 + 8u * stage;
         if (elect_one()) {
@@ -1002,11 +1002,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
         next = describe(unit + n_pairs);
         const int buf = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
-        if (!mbar_wait_bounded(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kPairRows);
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
+          if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
           tc_fence_after();
           if (elect_one()) {
             const uint32_t w_addr = smem_base + stage * kStage2Bytes;
@@ -1066,7 +1066,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       u3 = describe(unit + 3 * n_pairs);
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
-      if (!mbar_wait_bounded(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
+      if (!mbar_wait_bounded_warp(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * kPairRows);
       drain_transposed<MODE>(g, pb, taddr, static_cast<int>(rank), q, h, lane, my_stage, u.chunk, u.expert < 0, u.row0,

@@ -205,12 +205,12 @@ lm_head_scan_kernel(const int8_t* __restrict__ q_weight, const float* __restrict
       if (own < hi) { scale = __ldg(scales + own); residual = __ldg(residual_l2 + own); }
     }
     const int b = p % kScanBuffers;
-    if (!mbar_wait_bounded(bars + 8 * b, (p / kScanBuffers) & 1, abort_flag)) {
+    if (!mbar_wait_bounded_warp(bars + 8 * b, (p / kScanBuffers) & 1, abort_flag)) {
       // the result is then reported as not certified; the copies under way have to land before the block leaves
       if (lane == 0) top->failed = 1;
       volatile int ignore = 0;
       for (int q = p; q < min(steps, p + kScanBuffers); ++q)
-        mbar_wait_bounded(bars + 8 * (q % kScanBuffers), (q / kScanBuffers) & 1, &ignore);
+        mbar_wait_bounded_warp(bars + 8 * (q % kScanBuffers), (q / kScanBuffers) & 1, &ignore);
       break;
     }
     // (fewer rows left than the buffer holds: the rest of it are older rows, whose sums nobody takes)
