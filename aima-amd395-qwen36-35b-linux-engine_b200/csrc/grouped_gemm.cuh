@@ -87,7 +87,8 @@ struct TcExtra {
   uint64_t a_rows;      // rows of the A allocation (TMA bounds; reads beyond are zero-filled)
   int experts_in_b;     // experts held in b0 (expert modes), else 1
   SharedProblem shared = {};    // two-SM form, expert modes
-  bool pair = false;    // expert modes: two-SM form; the plan's tiles then hold up to 256 rows
+  bool pair = false;    // two-SM form; in the expert modes the plan's tiles then hold up to 256 rows
+  unsigned long long wait_limit_ns = kWaitBudgetNs;    // limit of each wait of the kernel
 };
 
 // tcgen05 / TMEM / TMA implementation (grouped_gemm_tc.cu).

@@ -66,6 +66,7 @@ struct TcProblem {
   int n_valid;            // valid output columns (plain mode masks beyond)
   int a_rows;             // rows of the A tensor (fused dispatch: first out-of-range row index)
   int* status;            // device status word
+  unsigned long long wait_limit_ns;
   // two-SM form
   int dense_tile;         // dense modes: rows per tile
   SharedProblem shared;   // expert modes: the shared expert's rows, in the same launch
@@ -402,7 +403,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
         b1_row = b0_row + kBN / 2;
       }
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         if (elect_one()) {
           const uint32_t a_dst = smem_base + stage * kStageBytes;
           const uint32_t b_dst = a_dst + kStageABytes;
@@ -472,11 +473,11 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
       // the epilogue must have drained this accumulator buffer (first use: free)
-      if (!mbar_wait_bounded_warp(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+      if (!mbar_wait_bounded_warp(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
       tc_fence_after();
       const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kBN);
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         if (kGather) fence_async_proxy();     // rows written by cp.async are read through the async proxy
         tc_fence_after();
         if (elect_one()) {
@@ -507,7 +508,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
       unit_tile(unit, tile, chunk, expert, row0, rows);
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
-      if (!mbar_wait_bounded_warp(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
+      if (!mbar_wait_bounded_warp(tfull_bar(buf), use & 1u, abort_flag, pb.wait_limit_ns)) { alive = false; if (lane == 0) timeout(); break; }
       tc_fence_after();
       drain_accumulator<MODE>(g, pb, tmem_base, buf, ew, eh, lane,
                               smem_gen + kStages * kStageBytes + 256 + (warp - 4) * kStoreStageBytes, chunk, row0, rows);
@@ -795,6 +796,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   uint8_t* tail = smem_gen + kStages2 * kStage2Bytes + 8 * (2 * kStages2 + 4);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
+  volatile int* issued_stages = reinterpret_cast<volatile int*>(tail + 16);      // by the producer and the two gather warps
+  const uint32_t drain_bar = smem_u32(tail + 32);
   uint8_t* store_stage = smem_gen + kStages2 * kStage2Bytes + kTc2BarrierBytes;
   uint8_t* gather_tables = store_stage + kPairEpilogueWarps * kStoreStage2Bytes;
 
@@ -813,6 +816,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       mbar_init(tfull_bar(b), 1);
       mbar_init(tempty_bar(b), 2 * kPairEpilogueWarps);
     }
+    mbar_init(drain_bar, 1);
+    for (int i = 0; i < 3; ++i) issued_stages[i] = 0;
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -878,13 +883,21 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     }
     return u;
   };
-  auto timeout = [&]() { atomicCAS(pb.status, 0, kStatusTimeoutMbarrier); };
+  // a wait ran out in this warp (or it saw the flag of one that did): both blocks of the pair stop
+  auto timeout = [&]() {
+    if (lane == 0) {
+      atomicCAS(pb.status, 0, kStatusTimeoutMbarrier);
+      asm volatile("st.shared::cluster.u32 [%0], %1;"
+                   :: "r"(map_to_rank(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u)), "r"(kStatusTimeoutMbarrier) : "memory");
+    }
+  };
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both blocks) -----------------
     const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
     int stage = 0;
     uint32_t phase = 0;
+    int issued = 0;
     bool alive = true;
     Unit next = describe(pair);
     for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
@@ -898,7 +911,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       uint32_t stage_bytes = 2 * (kStage2ABytes + half * kBK * 2);
       if (kGather) stage_bytes = 2 * kStage2ABytes + (gather_fours(min(half, u.rows)) + gather_fours(u.rows - half)) * (4 * kBK * 2);
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         if (elect_one()) {
           const uint32_t w_dst = smem_base + stage * kStage2Bytes;
           const uint32_t leader_full = leader_full0 + 8u * stage;
@@ -929,9 +942,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
           }
         }
         __syncwarp();
+        ++issued;
         if (++stage == kStages2) { stage = 0; phase ^= 1u; }
       }
     }
+    if (lane == 0) issued_stages[0] = issued;
   } else if (kGather && (warp == 2 || warp == 3)) {
     // ------------------------------ row gather (both blocks) -------------------
     // Rows by token index, four per TMA instruction (tile::gather4, a box of one row), the two warps in turn.  Only rows
@@ -945,6 +960,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
     int stage = 0;
     uint32_t phase = 0;
+    int issued = 0;
     bool alive = true;
     // two units ahead: description; one unit ahead: token indices
     auto tokens = [&](const Unit& u) {
@@ -975,7 +991,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       table[lane] = make_int4(t4.x >> 3, t4.y >> 3, t4.z >> 3, t4.w >> 3);
       __syncwarp();
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         const uint32_t dst = smem_base + stage * kStage2Bytes + kStage2ABytes;
         const uint32_t leader_full = leader_full0 + 8u * stage;
         if (elect_one()) {
@@ -986,9 +1002,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
           }
         }
         __syncwarp();
+        ++issued;
         if (++stage == kStages2) { stage = 0; phase ^= 1u; }
       }
     }
+    if (lane == 0) issued_stages[warp - 1] = issued;
   } else if (warp == 1) {
     if (leader) {
       // ------------------------------ MMA issuer (leader) ------------------------
@@ -1002,11 +1020,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
         next = describe(unit + n_pairs);
         const int buf = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
-        if (!mbar_wait_bounded_warp(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kPairRows);
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag)) { alive = false; timeout(); break; }
+          if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
           tc_fence_after();
           if (elect_one()) {
             const uint32_t w_addr = smem_base + stage * kStage2Bytes;
@@ -1066,7 +1084,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       u3 = describe(unit + 3 * n_pairs);
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
-      if (!mbar_wait_bounded_warp(tfull_bar(buf), use & 1u, abort_flag)) { alive = false; if (lane == 0) timeout(); break; }
+      if (!mbar_wait_bounded_warp(tfull_bar(buf), use & 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * kPairRows);
       drain_transposed<MODE>(g, pb, taddr, static_cast<int>(rank), q, h, lane, my_stage, u.chunk, u.expert < 0, u.row0,
@@ -1076,6 +1094,30 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                 // neither block leaves while the other may still signal it or read its memory
+  if (*abort_flag != 0) {
+    // Raised in both blocks, before the barrier above.  Nothing is issued any more; what is under way has to land before
+    // shared memory and tensor memory are given up: the MMAs (a last commit, to both blocks) and the loads of the last
+    // round of the ring (the leader's full barriers).  A stage that not every loader got to never completes; its wait gives
+    // the copies that were issued the whole budget.
+    volatile int ignore = 0;
+    if (warp == 1 && leader && elect_one()) umma_commit_pair(drain_bar);
+    if (threadIdx.x == 0) {
+      mbar_wait_bounded(drain_bar, 0, &ignore);
+      if (leader) {
+        int last = 0;
+        for (int i = 0; i < 3; ++i) {
+          int theirs;
+          asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(theirs) : "r"(map_to_rank(smem_u32(const_cast<int*>(issued_stages + i)), 1)) : "memory");
+          last = max(last, max(theirs, static_cast<int>(issued_stages[i])));
+        }
+        for (int j = max(0, last - kStages2); j < last; ++j) {
+          if (!mbar_wait_bounded(full_bar(j % kStages2), (j / kStages2) & 1, &ignore)) break;
+        }
+      }
+    }
+    __syncthreads();
+    cluster_sync_all();
+  }
   if (warp == 2) tmem_dealloc_pair(tmem_base, kTmemColumns);
 }
 
@@ -1256,6 +1298,7 @@ cudaError_t launch_grouped_gemm_tc(GemmMode mode, const GroupedGemm& g, const Tc
   TcProblem pb{};
   pb.g = g;
   pb.status = extra.status;
+  pb.wait_limit_ns = extra.wait_limit_ns;
   pb.n_valid = g.n;
   if (extra.pair) return launch_pair(mode, g, extra, pb, stream);
   const uint64_t experts = static_cast<uint64_t>(extra.experts_in_b);
