@@ -142,7 +142,7 @@ static_assert(32 % kScanRows == 0 && kScanRows % 2 == 0, "logits are finished 32
 __global__ void __launch_bounds__(kScanWarps * 32, 1)
 lm_head_scan_kernel(const int8_t* __restrict__ q_weight, const float* __restrict__ scales,
                     const float* __restrict__ residual_l2, const __nv_bfloat16* __restrict__ hidden,
-                    float* __restrict__ logits, aima_moe_lm_head_result* wire, LmHeadTop* top,
+                    float* __restrict__ logits, LmHeadWire* wire, LmHeadTop* top,
                     float* __restrict__ partial, int rows) {
   extern __shared__ __align__(16) uint8_t scan_smem[];
   __shared__ float warp_max[kScanWarps];
@@ -188,12 +188,11 @@ lm_head_scan_kernel(const int8_t* __restrict__ q_weight, const float* __restrict
   }
   const float hidden_l2 = hidden_norm_in_warp(hidden, lane);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    wire->hidden_l2 = hidden_l2;
-    wire->candidate_count = 0;
-    wire->overflow = 0;
+    wire->result.hidden_l2 = hidden_l2;
+    wire->result.candidate_count = 0;
+    wire->result.overflow = 0;
     top->best = 0;
     top->blocks_done = 0;
-    top->failed = 0;
   }
 
   float best_lower = -CUDART_INF_F;
@@ -206,7 +205,7 @@ lm_head_scan_kernel(const int8_t* __restrict__ q_weight, const float* __restrict
     }
     const int b = p % kScanBuffers;
     if (!mbar_wait_bounded_warp(bars + 8 * b, (p / kScanBuffers) & 1, abort_flag)) {
-      // the result is then reported as not certified; the copies under way have to land before the block leaves
+      // read_result then reports the timeout; the copies under way have to land before the block leaves
       if (lane == 0) top->failed = 1;
       volatile int ignore = 0;
       for (int q = p; q < min(steps, p + kScanBuffers); ++q)
@@ -266,14 +265,14 @@ lm_head_scan_kernel(const int8_t* __restrict__ q_weight, const float* __restrict
 __global__ void __launch_bounds__(kLmThreads)
 lm_head_candidates_kernel(const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ hidden,
                           const float* __restrict__ residual_l2, const float* __restrict__ partial, int partials,
-                          aima_moe_lm_head_result* wire, LmHeadTop* top, float* logits, int rows) {
+                          LmHeadWire* wire, LmHeadTop* top, float* logits, int rows) {
   __shared__ float reduction[kLmThreads / 32];
   const int lane = threadIdx.x & 31;
   pdl_enter();
   const int row = blockIdx.x * kLmThreads + threadIdx.x;
   const float logit = row < rows ? logits[row] : 0.0f;
   const float residual = row < rows ? residual_l2[row] : 0.0f;
-  const float hidden_l2 = wire->hidden_l2;
+  const float hidden_l2 = wire->result.hidden_l2;
   float largest = -CUDART_INF_F;
   for (int i = threadIdx.x; i < partials; i += kLmThreads) largest = fmaxf(largest, partial[i]);
 #pragma unroll
@@ -282,7 +281,7 @@ lm_head_candidates_kernel(const __nv_bfloat16* __restrict__ weight, const __nv_b
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kLmThreads / 32; ++w) largest = fmaxf(largest, reduction[w]);
-  if (blockIdx.x == 0 && threadIdx.x == 0) wire->maximum_lower_bound = largest;
+  if (blockIdx.x == 0 && threadIdx.x == 0) wire->result.maximum_lower_bound = largest;
 
   bool candidate = false;
   if (row < rows) {
@@ -295,10 +294,10 @@ lm_head_candidates_kernel(const __nv_bfloat16* __restrict__ weight, const __nv_b
     pending &= pending - 1u;
     const int token = __shfl_sync(0xffffffffu, row, owner);
     uint32_t slot = 0;
-    if (lane == 0) slot = atomicAdd(&wire->candidate_count, 1u);
+    if (lane == 0) slot = atomicAdd(&wire->result.candidate_count, 1u);
     slot = __shfl_sync(0xffffffffu, slot, 0);
     if (slot >= AIMA_MOE_LM_HEAD_CANDIDATES) {
-      if (lane == 0) wire->overflow = 1;
+      if (lane == 0) wire->result.overflow = 1;
       continue;
     }
     const uint4* wrow = reinterpret_cast<const uint4*>(weight + static_cast<size_t>(token) * kHidden) + lane;
@@ -329,9 +328,10 @@ lm_head_candidates_kernel(const __nv_bfloat16* __restrict__ weight, const __nv_b
     __threadfence();
     const unsigned long long best = atomicAdd(&top->best, 0ull);
     const uint32_t token = best != 0 ? 0xffffffffu - static_cast<uint32_t>(best) : 0u;
-    wire->exact_top1_token_id = token;
-    wire->exact_top1_logit = best != 0 ? __ldcg(logits + token) : -CUDART_INF_F;
-    if (top->failed != 0) wire->overflow = 1;
+    wire->result.exact_top1_token_id = token;
+    wire->result.exact_top1_logit = best != 0 ? __ldcg(logits + token) : -CUDART_INF_F;
+    wire->failed = top->failed;
+    top->failed = 0;
   }
 }
 

@@ -12,14 +12,22 @@ constexpr int kLmMaxScanBlocks = 256;
 struct LmHeadTop {
   unsigned long long best;          // largest exact logit: order-preserving bits, then the complement of the token id
   uint32_t blocks_done;             // blocks of the candidate kernel that have finished
-  uint32_t failed;                  // a bounded wait of the scan ran out
+  // a bounded wait of the scan ran out.  Any block of the scan may set it, so none of them clears it: that is done when the
+  // head is built and by the last block of the candidate kernel, after it has published it.
+  uint32_t failed;
+};
+
+// What read_result copies to the host.
+struct LmHeadWire {
+  aima_moe_lm_head_result result;
+  uint32_t failed;
 };
 
 struct LmHeadBuffers {
   int8_t* q_weight;                 // [rows, 2048]
   float* scales;                    // [rows]
   float* residual_l2;               // [rows]
-  aima_moe_lm_head_result* wire;    // device copy of the result
+  LmHeadWire* wire;                 // device copy of the result
   LmHeadTop* top;
   float* partial;                   // [kLmMaxScanBlocks] per-block maxima of the lower bounds
 };

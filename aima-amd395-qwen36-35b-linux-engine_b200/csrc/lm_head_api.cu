@@ -12,7 +12,7 @@ struct aima_moe_lm_head {
   uint32_t rows = 0;
   const void* weight = nullptr;      // caller-owned raw BF16 matrix [rows, 2048]
   void* allocation = nullptr;        // q | scales | residual_l2 | wire | top | partial
-  aima_moe_lm_head_result* host_result = nullptr;      // pinned
+  aima::LmHeadWire* host_result = nullptr;      // pinned
   aima::LmHeadBuffers buffers{};
   cudaStream_t last_stream = nullptr;
   uint64_t launches = 0;
@@ -91,11 +91,11 @@ AIMA_EXPORT int aima_moe_lm_head_build(const void* weight_bf16, uint32_t rows, a
   handle->buffers.q_weight = reinterpret_cast<int8_t*>(cursor); cursor += q_bytes;
   handle->buffers.scales = reinterpret_cast<float*>(cursor); cursor += row_bytes;
   handle->buffers.residual_l2 = reinterpret_cast<float*>(cursor); cursor += row_bytes;
-  handle->buffers.wire = reinterpret_cast<aima_moe_lm_head_result*>(cursor); cursor += 256;
+  handle->buffers.wire = reinterpret_cast<aima::LmHeadWire*>(cursor); cursor += 256;
   handle->buffers.top = reinterpret_cast<aima::LmHeadTop*>(cursor); cursor += 256;
   handle->buffers.partial = reinterpret_cast<float*>(cursor);
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
-  error = cudaMemsetAsync(handle->buffers.wire, 0, 256, cuda_stream);
+  error = cudaMemsetAsync(handle->buffers.wire, 0, 512, cuda_stream);      // wire and top
   if (error == cudaSuccess)
     error = aima::lm_head_quantize(weight_bf16, static_cast<int>(rows), handle->buffers.q_weight,
                                    handle->buffers.scales, handle->buffers.residual_l2, cuda_stream);
@@ -143,18 +143,21 @@ AIMA_EXPORT int aima_moe_lm_head_read_result(aima_moe_lm_head* handle, aima_moe_
   if (handle == nullptr || result == nullptr)
     return lm_fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "lm head: handle or result is null");
   std::lock_guard<std::mutex> lock(handle->mutex);
-  // On the handle's own device the copy goes through the legacy stream, which by itself waits for every ordinary stream; only a stream created
-  // non-blocking has to be waited for first.  Into pinned memory it is one request and one wait.
+  // On the handle's own device the copy goes through the legacy stream, which by itself waits for every ordinary stream;
+  // only a stream created non-blocking has to be waited for first.  Into pinned memory it is one request and one wait.
   unsigned flags = 0;
   int device = -1;
   cudaError_t error = cudaGetDevice(&device);
   if (error == cudaSuccess) error = cudaStreamGetFlags(handle->last_stream, &flags);
-  if (error == cudaSuccess && (device != handle->device || (flags & cudaStreamNonBlocking) != 0)) error = cudaStreamSynchronize(handle->last_stream);
+  if (error == cudaSuccess && (device != handle->device || (flags & cudaStreamNonBlocking) != 0))
+    error = cudaStreamSynchronize(handle->last_stream);
   if (error != cudaSuccess) return lm_fail_cuda(error, "cudaStreamSynchronize");
-  error = cudaMemcpyAsync(handle->host_result, handle->buffers.wire, sizeof *result, cudaMemcpyDeviceToHost, cudaStreamLegacy);
+  error = cudaMemcpyAsync(handle->host_result, handle->buffers.wire, sizeof *handle->host_result, cudaMemcpyDeviceToHost, cudaStreamLegacy);
   if (error == cudaSuccess) error = cudaStreamSynchronize(cudaStreamLegacy);
   if (error != cudaSuccess) return lm_fail_cuda(error, "copy of the lm head result");
-  *result = *handle->host_result;
+  *result = handle->host_result->result;
+  if (handle->host_result->failed != 0)
+    return lm_fail(AIMA_MOE_ERR_TIMEOUT, "lm head: a bounded wait of the scan ran out, the result is incomplete");
   if (result->overflow != 0)
     return lm_fail(AIMA_MOE_ERR_CAPACITY, "lm head: more than 1024 candidates, the top-1 is not certified");
   return AIMA_MOE_OK;

@@ -393,13 +393,14 @@ uint32_t aima_moe_abi_version(void);
  * reference; any row count here).  The library allocates rows x 2048 int8 + 2 x rows floats and
  * quantises on `stream`; the raw matrix stays caller-owned and must outlive the handle (the exact
  * candidate logits are read from it).
- * launch: hidden_bf16 [2048] (the final-norm output), logits_f32 [rows].  Enqueues four kernels:
+ * launch: hidden_bf16 [2048] (the final-norm output), logits_f32 [rows].  Enqueues two kernels:
  * the int8 scan writes approximate logits; rows whose upper bound reaches the largest lower bound
  * become candidates (at most AIMA_MOE_LM_HEAD_CANDIDATES); their exact BF16 logits overwrite the
  * approximate ones in logits_f32; the exact top-1 (equal logits -> lowest token id) goes to the
  * result.  Asynchronous and allocation-free.
  * read_result: synchronises the last stream and copies the result; returns AIMA_MOE_ERR_CAPACITY
- * when more than 1024 rows were candidates (top-1 not certified), as the reference's assert does. */
+ * when more than 1024 rows were candidates (top-1 not certified), as the reference's assert does, and
+ * AIMA_MOE_ERR_TIMEOUT when a bounded wait of the scan ran out (result incomplete). */
 #define AIMA_MOE_LM_HEAD_CANDIDATES 1024
 typedef struct aima_moe_lm_head aima_moe_lm_head;
 typedef struct aima_moe_lm_head_result {

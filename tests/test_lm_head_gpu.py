@@ -4,6 +4,8 @@ set, the same exact top-1; at the reference's vocabulary size the certified toke
 arg-max of the full exact BF16 GEMV."""
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
@@ -87,4 +89,36 @@ def test_lm_head_full_vocabulary_agrees_with_the_exact_gemv(package):
             assert float((logits - exact).abs().max()) < 0.05
     finally:
         provider.release()
+        head.release()
+
+
+def test_a_wait_that_ran_out_in_the_scan_is_reported_as_a_timeout(package, oracle):
+    """The scan's failure flag, set before its first block could have run, is neither lost nor taken for too many candidates,
+    and the launch after it is clean."""
+    rows = 4099
+    generator = torch.Generator().manual_seed(SEED)
+    weight = (torch.randn(rows, 2048, generator=generator) * 0.02).to(torch.bfloat16)
+    hidden = torch.randn(2048, generator=generator).to(torch.bfloat16)
+    want = oracle.lm_head_certify(weight, *oracle.lm_head_quantize(weight), hidden)
+    head = package.LmHead(weight.to("cuda"))
+    try:
+        residual = ctypes.c_void_p()
+        head.lib.check(head.lib.aima_moe_lm_head_views(head.handle, None, None, ctypes.byref(residual)))
+        state = residual.value + (rows * 4 + 255) // 256 * 256 + 256       # behind the residual norms and the result
+
+        class _Word:
+            __cuda_array_interface__ = {"shape": (1,), "typestr": "<i4", "data": (state + 12, False), "version": 2}
+
+        failed = torch.as_tensor(_Word(), device="cuda")
+        assert failed.item() == 0
+        failed.fill_(1)
+        head.launch(hidden.to("cuda"))
+        with pytest.raises(package.AimaMoeError) as error:
+            head.result()
+        assert error.value.status == -5                                    # AIMA_MOE_ERR_TIMEOUT
+        head.launch(hidden.to("cuda"))
+        result = head.result()
+        assert (result.exact_top1_token_id, result.exact_top1_logit) == (want["top1_token"], want["top1_logit"])
+        assert result.overflow == 0 and failed.item() == 0
+    finally:
         head.release()
