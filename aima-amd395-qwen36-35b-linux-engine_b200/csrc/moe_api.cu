@@ -754,14 +754,14 @@ AIMA_EXPORT int aima_moe_sync_metrics(aima_moe_handle* handle, aima_moe_metrics*
     error = cudaMemcpy(&handle->metrics.last_padded_routed_rows, handle->prefill.padded_rows,
                        sizeof(int32_t), cudaMemcpyDeviceToHost);
     if (error != cudaSuccess) return fail_cuda(error, "cudaMemcpy padded row count");
-    int32_t stats[5] = {0, 0, 0, 0, 0};
+    unsigned long long stats[5] = {0, 0, 0, 0, 0};
     error = cudaMemcpy(stats, handle->prefill.router_stats, sizeof stats, cudaMemcpyDeviceToHost);
     if (error != cudaSuccess) return fail_cuda(error, "cudaMemcpy router statistics");
-    handle->metrics.router_candidates = static_cast<uint64_t>(static_cast<uint32_t>(stats[0]));
-    handle->metrics.router_tokens = static_cast<uint64_t>(static_cast<uint32_t>(stats[1]));
-    handle->metrics.router_bound_violations = static_cast<uint64_t>(static_cast<uint32_t>(stats[2]));
-    handle->metrics.router_audited_tokens = static_cast<uint64_t>(static_cast<uint32_t>(stats[3]));
-    handle->metrics.router_audit_mismatches = static_cast<uint64_t>(static_cast<uint32_t>(stats[4]));
+    handle->metrics.router_candidates = stats[0];
+    handle->metrics.router_tokens = stats[1];
+    handle->metrics.router_bound_violations = stats[2];
+    handle->metrics.router_audited_tokens = stats[3];
+    handle->metrics.router_audit_mismatches = stats[4];
   }
   if (metrics != nullptr) {
     if (metrics->struct_bytes != sizeof(aima_moe_metrics))

@@ -290,7 +290,7 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
                                 const float* __restrict__ bias, int quant_eighths, int tokens,
                                 int32_t* __restrict__ ids, float* __restrict__ scores,
                                 float* __restrict__ weights, float* __restrict__ shared_sigmoid,
-                                __nv_bfloat16* __restrict__ dbg_weights, int32_t* __restrict__ stats,
+                                __nv_bfloat16* __restrict__ dbg_weights, unsigned long long* __restrict__ stats,
                                 int audit_stride) {
   __shared__ float sel_v_s[kCertWarps * 8];
   __shared__ int sel_i_s[kCertWarps * 8];
@@ -432,11 +432,11 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
     if (lane == 0) {
       shared_sigmoid[token] = round_bf16(det_sigmoid(round_bf16(acc)));
       if (stats != nullptr) {
-        atomicAdd(stats, recomputed);
-        atomicAdd(stats + 1, 1);
-        if (violated) atomicAdd(stats + 2, 1);
-        if (audited) atomicAdd(stats + 3, 1);
-        if (audit_mismatch) atomicAdd(stats + 4, 1);
+        atomicAdd(stats, static_cast<unsigned long long>(recomputed));
+        atomicAdd(stats + 1, 1ull);
+        if (violated) atomicAdd(stats + 2, 1ull);
+        if (audited) atomicAdd(stats + 3, 1ull);
+        if (audit_mismatch) atomicAdd(stats + 4, 1ull);
       }
     }
   }
@@ -498,7 +498,7 @@ prefill_logits_small_kernel(const __nv_bfloat16* __restrict__ h2, const __nv_bfl
 __global__ void __launch_bounds__(kCertWarps * 32)
 prefill_select_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int quant_eighths, int tokens,
                       int32_t* __restrict__ ids, float* __restrict__ scores, float* __restrict__ weights,
-                      __nv_bfloat16* __restrict__ dbg_weights, int32_t* __restrict__ stats) {
+                      __nv_bfloat16* __restrict__ dbg_weights) {
   __shared__ float sel_v_s[kCertWarps * 8];
   __shared__ int sel_i_s[kCertWarps * 8];
   const int warp = threadIdx.x >> 5;
@@ -513,10 +513,6 @@ prefill_select_kernel(const float* __restrict__ logits, const float* __restrict_
                                    bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths));
   route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
               ids, scores, weights, dbg_weights);
-  if (lane == 0) {
-    atomicAdd(stats, kExperts);
-    atomicAdd(stats + 1, 1);
-  }
 }
 
 // Euclidean norms of the 256 router rows, rounded up a little; one warp per row.
@@ -987,7 +983,7 @@ Layout layout_for(size_t T) {
   l.weights = take(rows * 4);
   l.sigmoid = take(T * 4);
   l.approx = take(T * kExperts * 4);
-  l.stats = take(32);
+  l.stats = take(5 * sizeof(unsigned long long));
   l.counts = take(kExperts * 4);
   l.offsets = take((kExperts + 1) * 4);
   l.sorted = take(rows * 4);
@@ -1050,7 +1046,7 @@ int prefill_workspace_allocate(PrefillWorkspace* ws, uint32_t capacity_tokens, i
   ws->topk_weights = reinterpret_cast<float*>(b + l.weights);
   ws->shared_sigmoid = reinterpret_cast<float*>(b + l.sigmoid);
   ws->approx_logits = reinterpret_cast<float*>(b + l.approx);
-  ws->router_stats = reinterpret_cast<int32_t*>(b + l.stats);
+  ws->router_stats = reinterpret_cast<unsigned long long*>(b + l.stats);
   ws->expert_counts = reinterpret_cast<int32_t*>(b + l.counts);
   ws->expert_offsets = reinterpret_cast<int32_t*>(b + l.offsets);
   ws->sorted_rows = reinterpret_cast<int32_t*>(b + l.sorted);
@@ -1139,7 +1135,7 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
       code = launch_pdl(prefill_select_kernel, dim3((T + kCertWarps - 1) / kCertWarps), dim3(kCertWarps * 32), 0, stream,
                         static_cast<const float*>(ws->approx_logits), call.router_bias, call.quant_eighths, T,
                         ws->topk_ids, ws->topk_scores, ws->topk_weights,
-                        dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr, ws->router_stats);
+                        dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr);
     if (code != cudaSuccess) return set_error(error, error_bytes, code, "router of a short call");
     count += 2;
   } else {

@@ -44,8 +44,9 @@ struct PrefillWorkspace {
   float* topk_weights = nullptr;      // [T, 8] BF16-rounded, stored as FP32
   float* shared_sigmoid = nullptr;    // [T]    bf16(sigmoid(bf16 gate logit)) as FP32
   float* approx_logits = nullptr;     // [T, 256] tensor-core router logits (candidate filter only)
-  int32_t* router_stats = nullptr;    // [5] candidates recomputed exactly, tokens routed, tokens whose candidates broke the
-                                      //     filter's bound (recomputed in full), tokens audited, audit mismatches
+  // [5] of the certified router: candidates recomputed exactly, tokens routed, tokens whose candidates broke the filter's
+  //     bound (recomputed in full), tokens audited, audit mismatches
+  unsigned long long* router_stats = nullptr;
   int router_audit_stride = 0;        // qualification: every n-th token is also routed from all 256 canonical logits
   // dispatch plan
   int32_t* expert_counts = nullptr;   // [256]

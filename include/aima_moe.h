@@ -166,7 +166,8 @@ typedef struct aima_moe_metrics {
   int32_t device_status;         /* last device status word read              */
   uint64_t router_candidates;    /* experts recomputed exactly by the certified
                                     prefill router since prepare()             */
-  uint64_t router_tokens;        /* tokens it routed                           */
+  uint64_t router_tokens;        /* tokens it routed (calls of up to 128 tokens
+                                    evaluate all 256 instead and do not count) */
   uint64_t router_bound_violations; /* tokens one of whose candidates lay further
                                     from its tensor-core logit than the filter's
                                     bound allows; such a token is routed from all

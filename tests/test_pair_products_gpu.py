@@ -165,3 +165,20 @@ def test_nan_logits_of_a_short_call_stay_in_their_row(package, oracle, gpu_layer
     assert torch.equal(dbg["topk_ids"].cpu(), want["ids"])
     assert torch.equal(dbg["topk_scores"].cpu(), want["scores"])
     assert torch.equal(dbg["topk_weights"].cpu(), want["weights"])
+
+
+def test_calls_that_do_not_filter_leave_the_filter_statistics_alone(package, gpu_layers, synth):
+    device = torch.device("cuda", 0)
+    provider = package.MoeProvider(layers=1, max_prefill_tokens=129)
+    try:
+        provider.bind_layer(0, gpu_layers(0)["cuda"])
+        h2 = synth.activations(SEED, 129, "input", 0).to(device)
+        seen = []
+        for tokens in (129, 128, 1):
+            provider.launch_selected_moe(post_attention=h2[:tokens], residual_hidden=h2[:tokens], model_layer=0)
+            metrics = provider.sync_metrics()
+            seen.append((metrics.router_tokens, metrics.router_candidates))
+        assert seen[0][0] == 129 and 8 * 129 <= seen[0][1] <= 64 * 129
+        assert seen[1:] == seen[:1] * 2
+    finally:
+        provider.release()
