@@ -69,6 +69,7 @@ struct TcProblem {
   unsigned long long wait_limit_ns;
   // two-SM form
   int dense_tile;         // dense modes: rows per tile
+  int copied_above;       // gather: tiles of more rows are read from the copied rows
   SharedProblem shared;   // expert modes: the shared expert's rows, in the same launch
   int shared_tiles;
 };
@@ -561,8 +562,8 @@ struct TcPairMaps {
   CUtensorMap w;        // weights: [rows, k] box 64 x 128, or the 5-D view of a gate_up tensor (make_gate_up_map)
   CUtensorMap shared_w[2];     // the shared expert's gate and up matrices (box 64 x 16), or its down matrix (box 64 x 128)
   CUtensorMap shared_rows[4];  // its rows, like `rows`
-  CUtensorMap rows[4];  // A: boxes of 64 x 16, 32, 64 and 128 rows (any multiple of 16 rows is at most four loads);
-                        // gather: rows[0] is the box of one row
+  CUtensorMap rows[4];  // A: boxes of 64 x 16, 32, 64 and 128 rows (any multiple of 16 rows is at most four loads)
+  CUtensorMap one_row;  // gather: the box of one row of the rows by token
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -884,6 +885,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     return u;
   };
   // a wait ran out in this warp (or it saw the flag of one that did): both blocks of the pair stop
+  // gather: whether the tile's rows lie one after the other all the same -- the shared expert's in the input, a tall
+  // tile's where they were copied -- and come by tile loads.  (Both gather warps then have a box of 16 rows at least.)
+  auto tiled = [&](const Unit& u) { return u.rows > 32 && (u.expert < 0 || u.rows > pb.copied_above); };
   auto timeout = [&]() {
     if (lane == 0) {
       atomicCAS(pb.status, 0, kStatusTimeoutMbarrier);
@@ -909,7 +913,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       const int w_row = u.expert * pb.b_rows_per_expert + u.chunk * kPairN + static_cast<int>(rank) * 128;
       // what both blocks fetch for a stage: weights, and the tile's rows (gathered: in fours per block)
       uint32_t stage_bytes = 2 * (kStage2ABytes + half * kBK * 2);
-      if (kGather) stage_bytes = 2 * kStage2ABytes + (gather_fours(min(half, u.rows)) + gather_fours(u.rows - half)) * (4 * kBK * 2);
+      if (kGather && !tiled(u)) stage_bytes = 2 * kStage2ABytes + (gather_fours(min(half, u.rows)) + gather_fours(u.rows - half)) * (4 * kBK * 2);
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         if (elect_one()) {
@@ -949,13 +953,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     if (lane == 0) issued_stages[0] = issued;
   } else if (kGather && (warp == 2 || warp == 3)) {
     // ------------------------------ row gather (both blocks) -------------------
-    // Rows by token index, four per TMA instruction (tile::gather4, a box of one row), the two warps in turn.  Only rows
-    // that exist are fetched, the last group filled up with repeats; what a stage holds beyond them ends in accumulator
-    // columns that nobody reads.  Each warp fetches at least one group per stage, an unneeded one if the tile has no row
-    // for it: a stage then always waits for both, so that neither can fall behind the ring or run ahead of it by a whole
-    // round, which a barrier's parity would not tell.  (One warp for all groups, or the warp that loads the weights, is
-    // slower: 456 against 380 us per layer at 2048 tokens.)  The tile's token indices wait in shared memory, one private
-    // copy per warp.
+    // Rows by token index, four per TMA instruction (tile::gather4, a box of one row), the two warps in turn; those of a
+    // tile whose rows lie in order (tiled) by tile loads, one part of the block's half per warp.  Only rows that exist are
+    // gathered, the last group filled up with repeats; what a stage holds beyond them ends in accumulator columns that
+    // nobody reads.  Each warp fetches at least one group per stage, an unneeded one if the tile has no row for it: a stage
+    // then always waits for both, so that neither can fall behind the ring or run ahead of it by a whole round, which a
+    // barrier's parity would not tell.  (One warp for all groups, or the warp that loads the weights, is slower: 456 against
+    // 380 us per layer at 2048 tokens.)  Why tall tiles are not gathered: 256 rows are 1440 cycles of gather4 a stage against
+    // 512 of tensor time; with the shared expert's tiles read by tile loads a layer of 1024 tokens went from 324 to 314 us.
+    // The tile's token indices wait in shared memory, one private copy per warp.
     int4* table = reinterpret_cast<int4*>(gather_tables + (warp - 2) * kGatherTableBytes);
     const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
     int stage = 0;
@@ -986,6 +992,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       next_tokens = tokens(next);
       later = describe(unit + 2 * n_pairs);
       const int half = pair_width(u.rows) / 2;
+      const bool by_tile = tiled(u);
+      // boxes of 16 rows of this block's half: the first warp takes the larger part
+      const int my_boxes = (half / 16 + 3 - warp) / 2;
+      const int my_first = warp == 2 ? 0 : half - 16 * my_boxes;
       const int fours = gather_fours(min(half, u.rows - static_cast<int>(rank) * half));
       __syncwarp();
       table[lane] = make_int4(t4.x >> 3, t4.y >> 3, t4.z >> 3, t4.w >> 3);
@@ -995,10 +1005,22 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
         const uint32_t dst = smem_base + stage * kStage2Bytes + kStage2ABytes;
         const uint32_t leader_full = leader_full0 + 8u * stage;
         if (elect_one()) {
+          if (by_tile) {
+            int done = my_first;
+#pragma unroll
+            for (int b = 2; b >= 0; --b) {
+              if (my_boxes & (1 << b)) {
+                tma_load_2d_pair(dst + done * (kBK * 2), u.expert < 0 ? &maps.shared_rows[b] : &maps.rows[b], kb * kBK,
+                                 u.row0 + static_cast<int>(rank) * half + done, leader_full);
+                done += 16 << b;
+              }
+            }
+          } else {
 #pragma unroll 4
-          for (int i = warp - 2; i < fours; i += 2) {
-            const int4 t = table[i];
-            tma_gather4_pair(dst + i * (4 * kBK * 2), &maps.rows[0], kb * kBK, t.x, t.y, t.z, t.w, leader_full);
+            for (int i = warp - 2; i < fours; i += 2) {
+              const int4 t = table[i];
+              tma_gather4_pair(dst + i * (4 * kBK * 2), &maps.one_row, kb * kBK, t.x, t.y, t.z, t.w, leader_full);
+            }
           }
         }
         __syncwarp();
@@ -1256,9 +1278,11 @@ cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extr
     pb.b_rows_per_expert = g.n;
     ok = make_map(&maps.w, g.b0, (mode == kGemmExpertDown ? experts : 1) * static_cast<uint64_t>(g.n), g.k, g.k);
   }
-  if (ok && gather) ok = make_map(&maps.rows[0], g.gather_src, extra.a_rows, g.k, g.lda, 1u);
-  for (int b = 0; ok && !gather && b < 4; ++b)
-    ok = make_map(&maps.rows[b], g.a, extra.a_rows, g.k, g.lda, 16u << b);
+  if (ok && gather) ok = make_map(&maps.one_row, g.gather_src, extra.a_rows, g.k, g.lda, 1u);
+  pb.copied_above = extra.copied_above;
+  const bool tiles = !gather || extra.copied_above < kPairRows;
+  for (int b = 0; ok && tiles && b < (gather ? 3 : 4); ++b)
+    ok = make_map(&maps.rows[b], g.a, gather ? extra.a_copied_rows : extra.a_rows, g.k, g.lda, 16u << b);
   const SharedProblem& shared = extra.shared;
   if (mode == kGemmPlain || mode == kGemmPlainF32) {
     pb.dense_tile = dense_tile_rows(g.dense_rows, pb.n_chunks, extra.sm_count / 2);
@@ -1273,7 +1297,7 @@ cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extr
     } else {
       ok = ok && make_map(&maps.shared_w[0], shared.b0, g.n, g.k, g.k);
     }
-    for (int b = 0; ok && !gather && b < 4; ++b)
+    for (int b = 0; ok && b < (gather ? 3 : 4); ++b)
       ok = make_map(&maps.shared_rows[b], shared.a, shared.rows, g.k, g.k, 16u << b);
   }
   if (!ok) return cudaErrorNotSupported;

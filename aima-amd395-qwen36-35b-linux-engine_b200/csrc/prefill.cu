@@ -697,16 +697,26 @@ cudaError_t launch_plan(PrefillWorkspace* ws, const int32_t* ids, int rows, int 
 }
 
 // ---------------------------------------------------------------------------
-// Gather of h2 rows into expert order; one warp per routed row.  It ends where the plan does (expert_offsets[256]):
-// beyond that sorted_rows would hold what an earlier call left there.
+// Copy of h2 rows into expert order, one warp per routed row: the rows of tiles with more than `copied_above` rows (0: all
+// of them); the product kernel gathers the others by token.  It ends where the plan does (expert_offsets[256]): beyond
+// that sorted_rows would hold what an earlier call left there.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const __nv_bfloat16* __restrict__ h2, const int32_t* __restrict__ sorted_rows,
-                   const int32_t* __restrict__ expert_offsets, __nv_bfloat16* __restrict__ gathered) {
+gather_rows_kernel(const __nv_bfloat16* __restrict__ h2, const int32_t* __restrict__ ids, const int32_t* __restrict__ sorted_rows,
+                   const int32_t* __restrict__ expert_counts, const int32_t* __restrict__ expert_offsets, int tile_cap,
+                   int copied_above, __nv_bfloat16* __restrict__ gathered) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int pos = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (pos >= expert_offsets[kExperts]) return;
-  const int token = sorted_rows[pos] >> 3;
+  const int flat = sorted_rows[pos];
+  if (copied_above > 0) {
+    const int e = ids[flat];
+    const int count = expert_counts[e];
+    const int height = rows_per_tile(count, (count + tile_cap - 1) / tile_cap, tile_cap);
+    if (min(height, count - (pos - expert_offsets[e]) / height * height) <= copied_above) return;
+  }
+  const int token = flat >> 3;
   const uint4* src = reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(token) * kHidden);
   uint4* dst = reinterpret_cast<uint4*>(gathered + static_cast<size_t>(pos) * kHidden);
 #pragma unroll
@@ -1100,7 +1110,10 @@ __global__ void forced_routing_kernel(const int32_t* __restrict__ ids, const __n
   topk_scores[i] = 0.0f;
 }
 
-constexpr int kGatherMaxTokens = 3584;     // between the two sizes where the two dispatch forms cross
+// dispatch of the routed rows (prefill_layer_launch)
+constexpr int kCopyMinTokens = 1024;
+constexpr int kGatherMaxTokens = 3584;
+constexpr int kCopiedAbove = 96;
 
 int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStream_t stream,
                          int* launches, char* error, size_t error_bytes) {
@@ -1167,19 +1180,27 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
     ++count;
   }
 
-  if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, stream, &count, simt ? kTileRows : 2 * kTileRows)) != cudaSuccess)
+  const int tile_cap = simt ? kTileRows : 2 * kTileRows;
+  if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, stream, &count, tile_cap)) != cudaSuccess)
     return set_error(error, error_bytes, code, "dispatch plan");
 
-  // Dispatch.  Up to kGatherMaxTokens the gate_up kernel fetches each tile's rows by token index itself (TMA gather4);
-  // with more tokens the rows are copied into expert order first and read by tile loads.  gather4 moves four rows per
-  // ~45 cycles, which the weight stream hides while a tile has few rows and not when it has 256: sustained us per layer,
-  // gather4 / copied rows, balanced routing: 331 / 348 at 1024 tokens, 379 / 420 at 2048, 451 / 468 at 3072, 518 / 505 at
-  // 4096, 645 / 610 at 6144, 855 / 771 at 8192.
+  // Dispatch.  Rows come to the gate_up product by token index, gathered by the kernel itself (TMA gather4), or from a copy
+  // in expert order, read by tile loads.  gather4 moves four rows per ~45 cycles, which the weight stream hides while a tile
+  // has few rows and not when it has many, so what decides is the rows of a TILE: those with more than kCopiedAbove are
+  // copied and read, the others gathered.  (The shared expert's rows lie in order anyway and are never gathered.)
+  //   up to kCopyMinTokens   nothing is copied: the copy kernel, which finds its tiles by itself, costs balanced routing more
+  //                          than a tall tile loses (balanced routing at 1024 tokens 314 us, 319 with the launch)
+  //   above kGatherMaxTokens everything is copied: nearly all tiles are tall
+  // us per layer, all gathered / by tile / all copied: eight hot experts 147 / 127 / 127 at 1536 tokens, 182 / 157 / 157 at
+  // 2048, 303 / 267 / 273 at 3584; Zipf 322 / 293 / 303 at 1536, 343 / 334 / 340 at 2048, 510 / 475 / 451 at 3584; balanced
+  // 331 / 336 / 355 at 1536, 350 / 348 / 374 at 2048, 442 / 436 / 431 at 3072, 468 / 460 / 459 at 3584.  A crossing of 64
+  // rows is slower at 2048 balanced tokens (363), 128 to 192 are as good as 96.
   const bool fused_dispatch = ws->fused_dispatch && !simt && T <= kGatherMaxTokens;
-  if (!fused_dispatch) {
-    gather_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(call.h2), ws->sorted_rows, ws->expert_offsets, ws->gathered);
-    if ((code = cudaGetLastError()) != cudaSuccess) return set_error(error, error_bytes, code, "gather_rows_kernel");
+  const int copied_above = !fused_dispatch ? 0 : T > kCopyMinTokens ? kCopiedAbove : tile_cap;
+  if (copied_above < tile_cap) {
+    code = launch_pdl(gather_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, h2, ws->topk_ids, ws->sorted_rows,
+                      ws->expert_counts, ws->expert_offsets, tile_cap, copied_above, ws->gathered);
+    if (code != cudaSuccess) return set_error(error, error_bytes, code, "gather_rows_kernel");
     ++count;
   }
 
@@ -1199,6 +1220,8 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   if (fused_dispatch) {
     g.gather_src = h2;
     extra.a_rows = static_cast<uint64_t>(T);
+    extra.copied_above = copied_above;
+    extra.a_copied_rows = static_cast<uint64_t>(ws->capacity) * kTopK;
   } else {
     extra.a_rows = static_cast<uint64_t>(ws->capacity) * kTopK;
   }

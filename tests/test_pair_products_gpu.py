@@ -182,3 +182,36 @@ def test_calls_that_do_not_filter_leave_the_filter_statistics_alone(package, gpu
         assert seen[1:] == seen[:1] * 2
     finally:
         provider.release()
+
+
+@pytest.mark.parametrize("tokens", [1025, 1100, 3584, 3585])
+def test_copied_and_gathered_tiles_give_the_same_bits(package, gpu_layers, synth, tokens):
+    """Calls in which some tiles are copied into expert order and others gathered by token: row counts on both sides of the
+    crossing (96) and of its halves and doubles, against the form that copies everything."""
+    device = torch.device("cuda", 0)
+    edges = [1, 31, 33, 64, 95, 96, 97, 128, 160, 161, 192, 193, 256, 257, 320, 321, 353, 449, 513, 577]
+    rows = tokens * 8
+    ids = torch.full((rows,), 200, dtype=torch.int32)
+    at = 0
+    for index, count in enumerate(edges):
+        ids[at:at + count] = 3 + 7 * index
+        at += count
+    generator = torch.Generator().manual_seed(SEED + tokens)
+    ids = ids[torch.randperm(rows, generator=generator)].reshape(tokens, 8).to(device)
+    routing = torch.rand(tokens, 8, generator=generator).to(torch.bfloat16).to(device)
+    h2 = synth.activations(SEED, tokens, "input", 0).to(device)
+    resid = synth.activations(SEED, tokens, "residual", 0).to(device)
+    results = []
+    for flags in (0, package.provider.FLAG_MATERIALIZED_DISPATCH):
+        provider = package.MoeProvider(layers=1, max_prefill_tokens=tokens, flags=flags)
+        try:
+            provider.bind_layer(0, gpu_layers(0)["cuda"])
+            provider.set_forced_routing(ids, routing)
+            views, dbg = provider.make_debug(tokens, prefill=True, with_logits=False, with_slot_rows=True)
+            out = provider.launch_selected_moe(post_attention=h2, residual_hidden=resid, model_layer=0, debug=views)
+            provider.sync_metrics()
+            results.append((out, dbg["slot_rows"], dbg["shared_scaled"]))
+        finally:
+            provider.release()
+    for mixed, copied in zip(*results):
+        assert torch.equal(mixed, copied)
