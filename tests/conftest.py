@@ -66,6 +66,33 @@ def built_library(package):
     return build.build()
 
 
+@pytest.fixture(scope="session")
+def product_probe(tmp_path_factory):
+    """tests/product_probe.cu: the product kernels with operands, form and limit of the waits chosen by the test."""
+    import ctypes
+    import shutil
+    import subprocess
+
+    library = tmp_path_factory.mktemp("products") / "libproduct_probe.so"
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    subprocess.run([nvcc, "-std=c++17", "-O3", "-shared", "-Xcompiler", "-fPIC", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "-I", str(PACKAGE_DIR / "csrc"), "-o", str(library), str(ROOT / "tests" / "product_probe.cu")], check=True)
+    probe = ctypes.CDLL(str(library))
+
+    class Operands(ctypes.Structure):
+        _fields_ = ([(name, ctypes.c_void_p) for name in (
+            "x", "gate_up", "down", "shared_gate", "shared_up", "shared_down", "tile_expert", "tile_row0", "tile_rows",
+            "tile_count", "sorted_rows", "row_scale", "shared_scale", "act", "out", "shared_act", "shared_out")] +
+            [(name, ctypes.c_longlong) for name in ("tokens", "rows", "experts", "max_tiles")])
+
+    def operands(**values):
+        """The caller keeps the tensors alive."""
+        return Operands(**{name: value if isinstance(value, int) else value.data_ptr() for name, value in values.items()})
+
+    probe.operands = operands
+    return probe
+
+
 SEED = 1234
 
 

@@ -3,6 +3,8 @@ all-ones known answer, agreement with an FP32 torch reference, and agreement of 
 layer with the CUDA-core cross-check kernel at a size the CPU oracle cannot reach."""
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
@@ -88,35 +90,58 @@ def test_prefill_tensor_core_products_match_cuda_core_products(package, gpu_laye
 
 
 @pytest.mark.parametrize("tokens,regime", [(300, "zipf"), (1024, "uniform"), (2048, "zipf"), (8192, "hot")])
-def test_two_sm_products_equal_one_sm_products(package, gpu_layers, synth, tokens, regime):
-    """The expert products in the two-SM form (tcgen05.mma.cta_group::2, a pair of blocks per 256-row tile)
-    against the one-SM form (128-row tiles): same operands in the same K order, so the same bits -- with
-    experts of fewer than 128 rows (the second block of the pair idle), of 129 .. 256 rows and of many
-    tiles, and the dispatch plan identical apart from the tile size."""
+def test_two_sm_products_equal_one_sm_products(product_probe, gpu_layers, synth, tokens, regime):
+    """The two product kernels on the same operands: the two-SM form of one GPU (weights on the M side, tiles of up to 256
+    rows, the shared expert in the same launch) and the one-SM form of expert parallelism (rows on the M side, 128-row tiles,
+    the shared expert in launches of its own).  Same products in the same K order, so the same bits -- with experts of one
+    row, of fewer than 128, of 129 .. 256 and of many tiles."""
     device = torch.device("cuda", 0)
     weights = gpu_layers(0)["cuda"]
     h2 = synth.activations(SEED + 5 + tokens, tokens, "input", 0).to(device)
-    resid = synth.activations(SEED + 5 + tokens, tokens, "residual", 0).to(device)
-    bias = {"zipf": synth.zipf_router_bias(SEED), "hot": synth.hot_expert_bias(range(3, 256, 32)), "uniform": None}[regime]
+    logits = h2.float() @ weights["router"].float().T
+    if regime != "uniform":
+        logits += {"zipf": synth.zipf_router_bias(SEED), "hot": synth.hot_expert_bias(range(3, 256, 32))}[regime].to(device)
+    top = logits.topk(8, dim=1)
+    flat = top.indices.reshape(-1)
+    routing = torch.softmax(top.values, dim=1).to(torch.bfloat16).float().reshape(-1).contiguous()
+    gate = torch.sigmoid(h2.float() @ weights["shared_gate"].float().reshape(-1)).to(torch.bfloat16).float().contiguous()
+    sorted_rows = torch.sort(flat, stable=True).indices.to(torch.int32)
+    counts = torch.bincount(flat, minlength=256).tolist()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    status = torch.zeros(1, dtype=torch.int32, device=device)
     results = []
-    for flags in (0, package.provider.FLAG_TWO_SM_PRODUCTS):
-        provider = package.MoeProvider(layers=1, max_prefill_tokens=tokens, flags=flags)
-        try:
-            provider.bind_layer(0, weights)
-            provider.set_router_hooks(None if bias is None else bias.to(device), quantize_eighths=False)
-            views, tensors = provider.make_debug(tokens, prefill=True, with_logits=False)
-            out = provider.launch_selected_moe(post_attention=h2, residual_hidden=resid, model_layer=0, debug=views)
-            provider.sync_metrics()
-            results.append((out.clone(), {k: v.clone() for k, v in tensors.items()}))
-        finally:
-            provider.release()
-    (out_one, dbg_one), (out_pair, dbg_pair) = results
-    for name in ("topk_ids", "sorted_rows", "expert_counts", "expert_offsets"):
-        assert torch.equal(dbg_pair[name], dbg_one[name]), name
-    assert torch.equal(dbg_pair["routed"], dbg_one["routed"])
-    assert torch.equal(dbg_pair["shared_scaled"], dbg_one["shared_scaled"])
-    assert torch.equal(out_pair, out_one)
-    assert torch.isfinite(out_pair.float()).all()
+    for pair, cap in ((0, 128), (1, 256)):
+        tiles, at = [], 0
+        for expert, count in enumerate(counts):
+            parts = -(-count // cap)
+            height = cap if cap == 128 or parts <= 1 else -(-(-(-count // parts)) // 32) * 32
+            tiles += [(expert, at + t * height, min(height, count - t * height)) for t in range(parts)]
+            at += count
+        assert sum(rows for _, _, rows in tiles) == tokens * 8
+        columns = [torch.tensor(column, dtype=torch.int32, device=device) for column in zip(*tiles)]
+        held = dict(tile_expert=columns[0], tile_row0=columns[1], tile_rows=columns[2],
+                    tile_count=torch.tensor([len(tiles)], dtype=torch.int32, device=device))
+        outputs = dict(act=torch.zeros(tokens * 8, 512, dtype=torch.bfloat16, device=device),
+                       out=torch.zeros(tokens * 8, 2048, dtype=torch.bfloat16, device=device),
+                       shared_act=torch.zeros(tokens, 512, dtype=torch.bfloat16, device=device),
+                       shared_out=torch.zeros(tokens, 2048, dtype=torch.bfloat16, device=device))
+        operands = product_probe.operands(
+            x=h2, gate_up=weights["expert_gate_up"], down=weights["expert_down"], shared_gate=weights["shared_gate_proj"],
+            shared_up=weights["shared_up_proj"], shared_down=weights["shared_down_proj"], sorted_rows=sorted_rows,
+            row_scale=routing, shared_scale=gate, tokens=tokens, rows=tokens * 8, experts=256, max_tiles=len(tiles),
+            **held, **outputs)
+        limit = ctypes.c_uint64(2_000_000_000)
+        pointer = ctypes.c_void_p(status.data_ptr())
+        torch.cuda.synchronize()
+        assert product_probe.run_gate_up(ctypes.byref(operands), pair, 1, sms, pointer, limit) == 0
+        assert product_probe.run_down(ctypes.byref(operands), pair, sms, pointer, limit) == 0
+        torch.cuda.synchronize()
+        assert status.item() == 0
+        results.append(outputs)
+    one, two = results
+    for name in one:
+        assert one[name].float().abs().amax() > 0, name
+        assert torch.equal(one[name], two[name]), name
 
 
 def test_certified_router_equals_exact_router_at_full_size(package, gpu_layers, synth):

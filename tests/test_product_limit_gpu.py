@@ -3,28 +3,14 @@ both blocks of every pair, lets its copies and MMAs land, returns with a status,
 from __future__ import annotations
 
 import ctypes
-import shutil
-import subprocess
 import time
-from pathlib import Path
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-ROOT = Path(__file__).resolve().parents[1]
-CSRC = ROOT / "aima-amd395-qwen36-35b-linux-engine_b200" / "csrc"
 NO_LIMIT = 2_000_000_000
-
-
-@pytest.fixture(scope="module")
-def probe(tmp_path_factory):
-    library = tmp_path_factory.mktemp("limit") / "libproduct_limit_probe.so"
-    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    subprocess.run([nvcc, "-std=c++17", "-O3", "-shared", "-Xcompiler", "-fPIC", "-gencode", "arch=compute_100a,code=sm_100a",
-                    "-I", str(CSRC), "-o", str(library), str(ROOT / "tests" / "product_limit_probe.cu")], check=True)
-    return ctypes.CDLL(str(library))
 
 
 def _p(tensor: torch.Tensor) -> ctypes.c_void_p:
@@ -56,19 +42,19 @@ def _check(launch, out: torch.Tensor, limit_ns: int, must_run_out: bool) -> None
 
 
 @pytest.mark.parametrize("limit_ns", [0, 6_000, 20_000, 5_000_000])
-def test_dense_product_stops_and_recovers(probe, limit_ns):
+def test_dense_product_stops_and_recovers(product_probe, limit_ns):
     m, n, k = 4096, 2048, 8192         # a unit is 128 stages, more than 30 us
     generator = torch.Generator(device="cuda").manual_seed(3)
     a = torch.randn(m, k, generator=generator, device="cuda").to(torch.bfloat16)
     b = torch.randn(n, k, generator=generator, device="cuda").to(torch.bfloat16)
     out = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    _check(lambda status, limit: probe.run_dense(_p(a), _p(b), _p(out), m, n, k, sms, _p(status), limit), out, limit_ns,
+    _check(lambda status, limit: product_probe.run_dense(_p(a), _p(b), _p(out), m, n, k, sms, _p(status), limit), out, limit_ns,
            must_run_out=limit_ns <= 20_000)
 
 
 @pytest.mark.parametrize("limit_ns", [0, 4_000, 12_000, 5_000_000])
-def test_gathered_product_stops_and_recovers(probe, limit_ns):
+def test_gathered_product_stops_and_recovers(product_probe, limit_ns):
     tokens, experts = 1024, 24
     generator = torch.Generator(device="cuda").manual_seed(4)
     x = torch.randn(tokens, 2048, generator=generator, device="cuda").to(torch.bfloat16)
@@ -84,6 +70,8 @@ def test_gathered_product_stops_and_recovers(probe, limit_ns):
     sorted_rows = torch.randint(0, tokens * 8, (total,), generator=torch.Generator().manual_seed(5), dtype=torch.int32).cuda()
     out = torch.empty(total, 512, dtype=torch.bfloat16, device="cuda")
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    _check(lambda status, limit: probe.run_gate_up(_p(x), tokens, _p(weights), experts, _p(tile_expert), _p(row0), _p(rows),
-                                                   _p(count), len(tiles), _p(sorted_rows), _p(out), sms, _p(status), limit),
+    operands = product_probe.operands(x=x, gate_up=weights, tile_expert=tile_expert, tile_row0=row0, tile_rows=rows,
+                                      tile_count=count, sorted_rows=sorted_rows, act=out, tokens=tokens, rows=total,
+                                      experts=experts, max_tiles=len(tiles))
+    _check(lambda status, limit: product_probe.run_gate_up(ctypes.byref(operands), 1, 0, sms, _p(status), limit),
            out, limit_ns, must_run_out=limit_ns == 0)
