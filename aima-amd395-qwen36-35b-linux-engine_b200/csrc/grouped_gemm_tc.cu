@@ -64,7 +64,6 @@ struct TcProblem {
   int b_rows_per_expert;  // rows between experts in b0 / b1
   int up_row_offset;      // row offset of the "up" half inside an expert (gate_up modes)
   int n_valid;            // valid output columns (plain mode masks beyond)
-  int a_rows;             // rows of the A tensor (fused dispatch: first out-of-range row index)
   int* status;            // device status word
   unsigned long long wait_limit_ns;
   // two-SM form
@@ -238,8 +237,7 @@ __device__ __forceinline__ void drain_accumulator(const GroupedGemm& g, const Tc
   } else if (MODE != kGemmPlainF32) {
     float scale = 1.0f;
     if (row_ok) {
-      if (MODE == kGemmExpertDown) scale = g.row_scale[g.sorted_rows[row]];
-      if (MODE == kGemmSharedDown) scale = g.row_scale[row];
+      scale = g.row_scale[MODE == kGemmExpertDown ? g.sorted_rows[row] : row];
     }
     const int col_base = chunk * kBN;
     __nv_bfloat16* dst = g.c + static_cast<size_t>(row0 + ew * 32) * g.ldc + col_base;
@@ -271,9 +269,7 @@ __device__ __forceinline__ void drain_accumulator(const GroupedGemm& g, const Tc
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const float acc = __uint_as_float(ar[j]);
-          if (MODE == kGemmExpertDown) v[j] = __fmul_rn(acc, scale);
-          else if (MODE == kGemmSharedDown) v[j] = __fmul_rn(scale, round_bf16(acc));
-          else v[j] = acc;
+          v[j] = (MODE == kGemmExpertDown) ? __fmul_rn(acc, scale) : __fmul_rn(scale, round_bf16(acc));
         }
         stage_32(stage, lane, half, v);
       }
@@ -1318,7 +1314,7 @@ cudaError_t launch_grouped_gemm_tc(GemmMode mode, const GroupedGemm& g, const Tc
   if (g.k % kBK != 0 || extra.status == nullptr) return cudaErrorInvalidValue;
   const bool gather = (mode == kGemmExpertGateUp && g.gather_src != nullptr);
   if (gather && g.sorted_rows == nullptr) return cudaErrorInvalidValue;
-  TcMaps maps;
+  TcMaps maps{};
   TcProblem pb{};
   pb.g = g;
   pb.status = extra.status;
@@ -1326,9 +1322,8 @@ cudaError_t launch_grouped_gemm_tc(GemmMode mode, const GroupedGemm& g, const Tc
   pb.n_valid = g.n;
   if (extra.pair) return launch_pair(mode, g, extra, pb, stream);
   const uint64_t experts = static_cast<uint64_t>(extra.experts_in_b);
-  bool ok = make_map(&maps.a, gather ? g.gather_src : g.a, extra.a_rows, static_cast<uint64_t>(g.k),
-                     static_cast<uint64_t>(g.lda), gather ? 1u : static_cast<uint32_t>(kBM));
-  pb.a_rows = static_cast<int>(extra.a_rows);
+  // (gathered rows are copied one by one, without a descriptor)
+  bool ok = gather || make_map(&maps.a, g.a, extra.a_rows, static_cast<uint64_t>(g.k), static_cast<uint64_t>(g.lda));
   if (mode == kGemmExpertGateUp) {
     pb.n_chunks = g.n / (kBN / 2);
     pb.b_rows_per_expert = 2 * g.n;

@@ -734,7 +734,7 @@ AIMA_EXPORT int aima_moe_gemm_bf16_launch(aima_moe_handle* handle, const void* a
   extra.status = handle->status; extra.sm_count = handle->sm_count; extra.a_rows = m; extra.experts_in_b = 1;
   extra.pair = true;
   const cudaError_t error = launch_grouped_gemm_tc(kGemmPlain, g, extra, static_cast<cudaStream_t>(stream));
-  if (error != cudaSuccess) return fail_cuda(error, "launch grouped_gemm_tc_kernel (plain)");
+  if (error != cudaSuccess) return fail_cuda(error, "launch grouped_gemm_pair_kernel (plain)");
   handle->last_stream = static_cast<cudaStream_t>(stream);
   handle->metrics.kernel_launches += 1;
   return AIMA_MOE_OK;

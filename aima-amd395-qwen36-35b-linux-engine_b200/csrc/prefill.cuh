@@ -7,7 +7,6 @@
 namespace aima {
 
 constexpr int kTileRows = 128;      // rows of one grouped-GEMM tile (one expert)
-constexpr int kPlanRowsPerWarp = 256;
 
 // Device buffers owned by a handle for prefill calls of up to `capacity` tokens.
 struct PrefillWorkspace {
@@ -19,8 +18,9 @@ struct PrefillWorkspace {
   bool exact_router = false;          // qualification: all 256 logits with the canonical dot
   bool fused_dispatch = true;         // gate_up kernel gathers its rows itself (no materialised copy)
   uint8_t* base = nullptr;
-  // The shared expert does not depend on the routing: it runs on a second stream, forked from and
-  // joined to the caller's stream with events, next to the router, the plan and the row gather.
+  // Expert parallelism: the shared expert does not depend on the routing and runs on a second stream, forked from and
+  // joined to the caller's stream with events, next to the router, the exchanges and the plan.  (On one GPU its rows are
+  // tiles of the expert products.)
   cudaStream_t side_stream = nullptr;
   cudaEvent_t fork_event = nullptr;     // caller's stream: inputs of this call are ready
   cudaEvent_t router_event = nullptr;   // caller's stream: sigmoid of the shared gate is written
