@@ -347,9 +347,12 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 // Whether launch_pdl relaxes the serialisation is the calling thread's choice for the span of one
-// host call (PdlScope): overlapping the kernel boundaries gains 3-4 % on a prefill layer of up to
-// 2048 tokens, where the gaps between its ten kernels weigh most, and loses 2-3 % at 4096 and 8192
-// tokens, so the prefill entry points relax it only up to pdl_max_tokens().
+// host call (PdlScope).  Overlapping the boundaries of a prefill layer's six or seven kernels gains most where they are short
+// and loses at the top, where kernels of 100 us and more compete with blocks that wait; the prefill entry points relax the
+// order up to pdl_max_tokens().  us per layer, plain order / relaxed, balanced routing: 133 / 121 at 16 tokens, 298 / 289
+// at 333, 318 / 310 at 1024, 350 / 339 at 2048, 416 / 405 at 3072, 446 / 438 at 3584, 469 / 456 at 4096, 572 / 570 at 6144,
+// 735 / 745 at 8192; Zipf: 278 / 270 at 1024, 332 / 324 at 2048, 455 / 449 at 3584, 478 / 480 at 4096, 621 / 615 at 6144,
+// 749 / 772 at 8192.
 inline thread_local bool t_pdl_relaxed = true;
 struct PdlScope {
   bool saved;
@@ -362,7 +365,7 @@ struct PdlScope {
 inline int pdl_max_tokens() {
   static const int limit = [] {
     const char* v = std::getenv("AIMA_MOE_PDL_MAX_TOKENS");
-    return (v != nullptr && v[0] != '\0') ? std::atoi(v) : 2048;
+    return (v != nullptr && v[0] != '\0') ? std::atoi(v) : 4096;
   }();
   return limit;
 }
