@@ -14,6 +14,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <new>
 
@@ -44,6 +45,14 @@ constexpr uint64_t kDownBytesPerExpert = 2ull * kHidden * kInter;
 constexpr uint64_t kSharedGateBytes = 2ull * kHidden;
 constexpr uint64_t kSharedProjBytes = 2ull * kSharedInter * kHidden;
 constexpr uint64_t kNormBytes = 2ull * kHidden;
+
+// Every activation is read and written in 16-byte pieces; a pointer that does not allow that is refused before any launch.
+bool aligned16(std::initializer_list<const void*> pointers) {
+  for (const void* pointer : pointers) {
+    if (reinterpret_cast<uintptr_t>(pointer) % 16 != 0) return false;
+  }
+  return true;
+}
 
 size_t align_up(size_t value, size_t alignment) {
   return (value + alignment - 1) / alignment * alignment;
@@ -496,6 +505,8 @@ AIMA_EXPORT int aima_moe_prefill_launch(aima_moe_handle* handle, uint32_t layer,
   if (const int wrong_device = check_current_device(handle); wrong_device != AIMA_MOE_OK) return wrong_device;
   if (h2 == nullptr || residual == nullptr || out == nullptr)
     return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "prefill input/output is null");
+  if (!aligned16({h2, residual, out}))
+    return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "prefill input/output must be 16-byte aligned");
   if (tokens == 0) return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "tokens is zero");
   if (tokens > handle->config.max_prefill_tokens)
     return fail(AIMA_MOE_ERR_CAPACITY, "tokens %u exceed prepared capacity %u", tokens,
@@ -557,6 +568,8 @@ AIMA_EXPORT int aima_moe_prefill_stack_launch(aima_moe_handle* handle, uint32_t 
   if (const int wrong_device = check_current_device(handle); wrong_device != AIMA_MOE_OK) return wrong_device;
   if (x_in == nullptr || x_out == nullptr)
     return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "prefill stack input/output is null");
+  if (!aligned16({x_in, x_out}))
+    return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "prefill stack input/output must be 16-byte aligned");
   if (tokens == 0 || tokens > handle->config.max_prefill_tokens)
     return fail(AIMA_MOE_ERR_CAPACITY, "tokens %u outside prepared capacity %u", tokens,
                 handle->config.max_prefill_tokens);
@@ -655,11 +668,8 @@ AIMA_EXPORT int aima_moe_prefill_fused_launch(aima_moe_handle* handle, uint32_t 
   const size_t bytes = static_cast<size_t>(tokens) * kHidden * 2;
   if (next_norm_out != nullptr && ranges_overlap(next_norm_out, bytes, layer_out, bytes))
     return fail(AIMA_MOE_ERR_ALIAS, "next_norm_out aliases layer_out");
-  for (const void* pointer : {attn_out, residual_in, static_cast<const void*>(layer_out),
-                              static_cast<const void*>(next_norm_out), next_norm_weight}) {
-    if (reinterpret_cast<uintptr_t>(pointer) % 16 != 0)
-      return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "fused prefill pointers must be 16-byte aligned");
-  }
+  if (!aligned16({attn_out, residual_in, layer_out, next_norm_out, next_norm_weight}))
+    return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "fused prefill pointers must be 16-byte aligned");
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
   // entry: after_attn = bf16(attn_out + residual_in) and h2 = RMSNorm(after_attn) into the workspace
   cudaError_t error = launch_rmsnorm_rows(attn_out, residual_in, handle->host_layers[layer].norm_weight,
@@ -721,6 +731,7 @@ AIMA_EXPORT int aima_moe_gemm_bf16_launch(aima_moe_handle* handle, const void* a
   if (const int wrong_device = check_current_device(handle); wrong_device != AIMA_MOE_OK) return wrong_device;
   if (a == nullptr || b == nullptr || d == nullptr)
     return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "gemm pointer is null");
+  if (!aligned16({a, b, d})) return fail(AIMA_MOE_ERR_INVALID_ARGUMENT, "gemm pointers must be 16-byte aligned");
   if (m == 0 || n == 0 || k == 0 || k % 64 != 0 || n % 8 != 0)
     return fail(AIMA_MOE_ERR_UNSUPPORTED, "gemm needs k a multiple of 64 and n a multiple of 8");
   GroupedGemm g{};

@@ -250,3 +250,36 @@ def test_prefill_argument_checks(provider, package, synth):
     with pytest.raises(package.AimaMoeError) as capacity:
         provider.launch_selected_moe(post_attention=big, residual_hidden=big.clone(), model_layer=0)
     assert capacity.value.status == -8
+
+
+@pytest.mark.parametrize("tokens", [40, 300])
+@pytest.mark.parametrize("flag", [None, "FLAG_EXACT_ROUTER", "FLAG_SIMT_PRODUCTS"])
+def test_misaligned_pointers_are_refused_before_any_launch(package, gpu_layers, synth, tokens, flag):
+    """A view that starts two bytes into its allocation, as input or output: an error from the host, whatever kernel would
+    have met it first, and the handle goes on working."""
+    device = torch.device("cuda", 0)
+    good = synth.activations(SEED, tokens, "input", 0).to(device)
+    shifted = torch.empty(tokens * 2048 + 8, dtype=torch.bfloat16, device=device)[1:1 + tokens * 2048].view(tokens, 2048)
+    shifted.copy_(good)
+    provider = package.MoeProvider(layers=1, max_prefill_tokens=tokens, flags=getattr(package.provider, flag) if flag else 0)
+    try:
+        provider.bind_layer(0, gpu_layers(0)["cuda"])
+        want = provider.launch_selected_moe(post_attention=good, residual_hidden=good, model_layer=0)
+        provider.sync_metrics()
+        calls = [lambda: provider.launch_selected_moe(post_attention=shifted, residual_hidden=good, model_layer=0),
+                 lambda: provider.launch_selected_moe(post_attention=good, residual_hidden=shifted, model_layer=0),
+                 lambda: provider.launch_selected_moe(post_attention=good, residual_hidden=good, model_layer=0, out=shifted),
+                 lambda: provider.prefill_stack(shifted, torch.empty_like(good)),
+                 lambda: provider.prefill_stack(good, shifted),
+                 lambda: provider.gemm(shifted, good)]
+        for call in calls:
+            launched = provider.sync_metrics().kernel_launches
+            with pytest.raises(package.AimaMoeError) as error:
+                call()
+            assert error.value.status == -1                                # AIMA_MOE_ERR_INVALID_ARGUMENT
+            assert provider.sync_metrics().kernel_launches == launched
+        got = provider.launch_selected_moe(post_attention=good, residual_hidden=good, model_layer=0)
+        provider.sync_metrics()
+        assert torch.equal(got, want)
+    finally:
+        provider.release()
