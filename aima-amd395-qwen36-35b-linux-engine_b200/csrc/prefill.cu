@@ -700,30 +700,42 @@ cudaError_t launch_plan(PrefillWorkspace* ws, const int32_t* ids, int rows, int 
 }
 
 // ---------------------------------------------------------------------------
-// Copy of h2 rows into expert order, one warp per routed row: the rows of tiles with more than `copied_above` rows (0: all
-// of them); the product kernel gathers the others by token.  It ends where the plan does (expert_offsets[256]): beyond
-// that sorted_rows would hold what an earlier call left there.
+// Copy of h2 rows into expert order: the rows of tiles with more than `copied_above` rows (0: all of them); the product
+// kernel gathers the others by token.  One block per token, 16 bytes per thread: the row is read once and written to the up
+// to eight places the plan gave it.  Bound by the writes (268 MB at 8192 tokens: 53 -> 49 us beside one warp per routed row,
+// which read every row eight times from L2).  us per layer with eight hot experts at 1536 / 2048 / 8192 tokens: 126 / 152 /
+// 561, with 128 threads per token 129 / 154 / 561, with 64 138 / 160 / 556.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-gather_rows_kernel(const __nv_bfloat16* __restrict__ h2, const int32_t* __restrict__ ids, const int32_t* __restrict__ sorted_rows,
-                   const int32_t* __restrict__ expert_counts, const int32_t* __restrict__ expert_offsets, int tile_cap,
-                   int copied_above, __nv_bfloat16* __restrict__ gathered) {
+constexpr int kCopyThreads = kHidden / 8;
+
+__global__ void __launch_bounds__(kCopyThreads)
+gather_rows_kernel(const __nv_bfloat16* __restrict__ h2, const int32_t* __restrict__ ids,
+                   const int32_t* __restrict__ row_position, const int32_t* __restrict__ expert_counts,
+                   const int32_t* __restrict__ expert_offsets, int tile_cap, int copied_above,
+                   __nv_bfloat16* __restrict__ gathered) {
   pdl_enter();
   const int lane = threadIdx.x & 31;
-  const int pos = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (pos >= expert_offsets[kExperts]) return;
-  const int flat = sorted_rows[pos];
-  if (copied_above > 0) {
-    const int e = ids[flat];
-    const int count = expert_counts[e];
-    const int height = rows_per_tile(count, (count + tile_cap - 1) / tile_cap, tile_cap);
-    if (min(height, count - (pos - expert_offsets[e]) / height * height) <= copied_above) return;
+  const int token = blockIdx.x;
+  int position = 0;
+  bool copied = false;
+  if (lane < kTopK) {
+    const int e = ids[token * kTopK + lane];
+    position = row_position[token * kTopK + lane];
+    if (e >= 0 && e < kExperts) {          // rows of other ids are not in the plan
+      const int count = expert_counts[e];
+      const int height = rows_per_tile(count, (count + tile_cap - 1) / tile_cap, tile_cap);
+      copied = min(height, count - (position - expert_offsets[e]) / height * height) > copied_above;
+    }
   }
-  const int token = flat >> 3;
-  const uint4* src = reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(token) * kHidden);
-  uint4* dst = reinterpret_cast<uint4*>(gathered + static_cast<size_t>(pos) * kHidden);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) dst[i * 32 + lane] = __ldg(src + i * 32 + lane);
+  unsigned pending = __ballot_sync(0xffffffffu, copied);
+  if (pending == 0u) return;
+  const uint4 piece = __ldg(reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(token) * kHidden) + threadIdx.x);
+  while (pending != 0u) {
+    const int slot = __ffs(pending) - 1;
+    pending &= pending - 1u;
+    const int to = __shfl_sync(0xffffffffu, position, slot);
+    reinterpret_cast<uint4*>(gathered + static_cast<size_t>(to) * kHidden)[threadIdx.x] = piece;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1197,11 +1209,12 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   // us per layer, all gathered / by tile / all copied: eight hot experts 147 / 127 / 127 at 1536 tokens, 182 / 157 / 157 at
   // 2048, 303 / 267 / 273 at 3584; Zipf 322 / 293 / 303 at 1536, 343 / 334 / 340 at 2048, 510 / 475 / 451 at 3584; balanced
   // 331 / 336 / 355 at 1536, 350 / 348 / 374 at 2048, 442 / 436 / 431 at 3072, 468 / 460 / 459 at 3584.  A crossing of 64
-  // rows is slower at 2048 balanced tokens (363), 128 to 192 are as good as 96.
+  // rows is slower at 2048 balanced tokens (363), 128 to 192 are as good as 96.  (Plain stream order above 2048 tokens and a
+  // copy with one warp per routed row, the same for all three; gather_rows_kernel has what its present form gives.)
   const bool fused_dispatch = ws->fused_dispatch && !simt && T <= kGatherMaxTokens;
   const int copied_above = !fused_dispatch ? 0 : T > kCopyMinTokens ? kCopiedAbove : tile_cap;
   if (copied_above < tile_cap) {
-    code = launch_pdl(gather_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, h2, ws->topk_ids, ws->sorted_rows,
+    code = launch_pdl(gather_rows_kernel, dim3(T), dim3(kCopyThreads), 0, stream, h2, ws->topk_ids, ws->row_position,
                       ws->expert_counts, ws->expert_offsets, tile_cap, copied_above, ws->gathered);
     if (code != cudaSuccess) return set_error(error, error_bytes, code, "gather_rows_kernel");
     ++count;
