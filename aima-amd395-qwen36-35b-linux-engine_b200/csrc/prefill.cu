@@ -321,7 +321,7 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
     const float a = approx[static_cast<size_t>(token) * kExperts + e];
     const float delta = kCertKappa * x_norm * row_norms[e] + 9.5367431640625e-07f * fabsf(a + b[q]);
     upper[q] = finish_logit(a + delta, b[q], quant_eighths);
-    lower[q] = finish_logit(a - delta, b[q], quant_eighths);
+    lower[q] = selectable(finish_logit(a - delta, b[q], quant_eighths));      // a NaN bounds nothing from below
   }
   const float floor_value = warp_eighth_largest(lower, lane);
 

@@ -167,6 +167,32 @@ def test_nan_logits_of_a_short_call_stay_in_their_row(package, oracle, gpu_layer
     assert torch.equal(dbg["topk_weights"].cpu(), want["weights"])
 
 
+@pytest.mark.parametrize("flag", [None, "FLAG_EXACT_ROUTER", "FLAG_AUDIT_ROUTER"])
+def test_nan_logit_of_a_long_call_counts_as_minus_infinity(package, oracle, gpu_layers, synth, flag):
+    """The certified router beyond the short calls: one NaN logit in every token neither takes a slot nor costs one."""
+    device = torch.device("cuda", 0)
+    weights = gpu_layers(0)["cuda"]
+    broken = dict(weights, router=weights["router"].clone())
+    broken["router"][77, 5] = float("nan")
+    tokens = 200
+    h2 = synth.activations(SEED + 3, tokens, "input", 0)
+    provider = package.MoeProvider(layers=1, max_prefill_tokens=tokens, flags=getattr(package.provider, flag) if flag else 0)
+    try:
+        provider.bind_layer(0, broken)
+        views, dbg = provider.make_debug(tokens, prefill=True, with_logits=False)
+        provider.launch_selected_moe(post_attention=h2.to(device), residual_hidden=h2.to(device), model_layer=0, debug=views)
+        metrics = provider.sync_metrics()
+    finally:
+        provider.release()
+    bias = torch.zeros(256)
+    bias[77] = float("-inf")
+    want = oracle.router_prefill(h2, oracle.OracleLayer(gpu_layers(0)["cpu"], router_bias=bias))
+    assert torch.equal(dbg["topk_ids"].cpu(), want["ids"])
+    assert torch.equal(dbg["topk_scores"].cpu(), want["scores"])
+    assert torch.equal(dbg["topk_weights"].cpu(), want["weights"])
+    assert metrics.router_audit_mismatches == 0 and metrics.router_bound_violations == 0
+
+
 def test_calls_that_do_not_filter_leave_the_filter_statistics_alone(package, gpu_layers, synth):
     device = torch.device("cuda", 0)
     provider = package.MoeProvider(layers=1, max_prefill_tokens=129)
