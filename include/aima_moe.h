@@ -206,6 +206,7 @@ int aima_moe_set_forced_routing(aima_moe_handle* handle, const int32_t* ids,
 /* Prefill MoE half of `layer` for `tokens` rows.
  * h2 = post-attention RMSNorm output, residual = after_attn, both bf16
  * [tokens,2048]; out bf16 [tokens,2048] = bf16(residual + bf16(routed + shared)).
+ * As in every prefill entry the pointers are 16-byte aligned (checked).
  * Replaces probe_native_q8192_moe_prefill_layer0_oracle in its production form
  * (collect_oracle_comparisons = false), native_resident_engine.hip.cpp:1061-1094. */
 int aima_moe_prefill_launch(aima_moe_handle* handle, uint32_t layer,
@@ -264,7 +265,8 @@ int aima_moe_gemv_bf16_launch(const void* weight, const void* x, void* out,
 
 /* Dense D[m,n] = A[m,k] . B[n,k]^T, BF16 in/out, FP32 accumulate on the tensor
  * cores: the contract of Bf16GemmPlan::launch
- * (native/src/bf16_gemm.hip.cpp:220-234).  k % 64 == 0, n % 8 == 0. */
+ * (native/src/bf16_gemm.hip.cpp:220-234).  k % 64 == 0, n % 8 == 0, pointers
+ * 16-byte aligned. */
 int aima_moe_gemm_bf16_launch(aima_moe_handle* handle, const void* a, const void* b,
                               void* d, uint32_t m, uint32_t n, uint32_t k, void* stream);
 
