@@ -319,6 +319,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
   auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * kStages + 2 + b); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + kStages * kStageBytes + 8 * (2 * kStages + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + kStages * kStageBytes + 8 * (2 * kStages + 4) + 8);
+  const uint32_t drain_bar = bar_base + 8u * (2 * kStages + 6);
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // known to be the same in all lanes
   const int lane = threadIdx.x & 31;
@@ -333,6 +334,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
       mbar_init(tfull_bar(b), 1);
       mbar_init(tempty_bar(b), kEpilogueWarps);
     }
+    mbar_init(drain_bar, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -516,6 +518,13 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
   }
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0) {
+    // a wait ran out: the copies have been waited for above, and so are the MMAs under way, by a last commit
+    volatile int ignore = 0;
+    if (warp == 1 && elect_one()) umma_commit(drain_bar);
+    if (threadIdx.x == 0) mbar_wait_bounded(drain_bar, 0, &ignore);
+    __syncthreads();
+  }
   if (warp == 2) tmem_dealloc(tmem_base, kTmemColumns);
 }
 

@@ -1,5 +1,6 @@
-"""GPU test of what the two-SM product kernel does when a wait runs out: with a limit shorter than a unit takes, it stops in
-both blocks of every pair, lets its copies and MMAs land, returns with a status, and the next launch gives the right bits."""
+"""GPU test of what the product kernels do when a wait runs out: with a limit shorter than a unit takes, the two-SM one stops
+in both blocks of every pair, the one-SM one in its block; copies and MMAs land, it returns with a status, and the next launch
+gives the right bits."""
 from __future__ import annotations
 
 import ctypes
@@ -53,14 +54,15 @@ def test_dense_product_stops_and_recovers(product_probe, limit_ns):
            must_run_out=limit_ns <= 20_000)
 
 
+@pytest.mark.parametrize("pair", [0, 1])
 @pytest.mark.parametrize("limit_ns", [0, 4_000, 12_000, 5_000_000])
-def test_gathered_product_stops_and_recovers(product_probe, limit_ns):
+def test_gathered_product_stops_and_recovers(product_probe, limit_ns, pair):
     tokens, experts = 1024, 24
     generator = torch.Generator(device="cuda").manual_seed(4)
     x = torch.randn(tokens, 2048, generator=generator, device="cuda").to(torch.bfloat16)
     weights = (torch.randn(experts, 1024, 2048, generator=generator, device="cuda") * 0.05).to(torch.bfloat16)
     heights = [256, 160, 33, 96, 1, 224, 31, 128]
-    tiles = [(e, heights[(3 * e + t) % len(heights)]) for e in range(experts) for t in range(4)]
+    tiles = [(e, min(heights[(3 * e + t) % len(heights)], 256 if pair else 128)) for e in range(experts) for t in range(4)]
     rows = torch.tensor([r for _, r in tiles], dtype=torch.int32)
     total = int(rows.sum())
     row0 = (rows.cumsum(0) - rows).to(torch.int32).cuda()
@@ -73,5 +75,5 @@ def test_gathered_product_stops_and_recovers(product_probe, limit_ns):
     operands = product_probe.operands(x=x, gate_up=weights, tile_expert=tile_expert, tile_row0=row0, tile_rows=rows,
                                       tile_count=count, sorted_rows=sorted_rows, act=out, tokens=tokens, rows=total,
                                       experts=experts, max_tiles=len(tiles))
-    _check(lambda status, limit: product_probe.run_gate_up(ctypes.byref(operands), 1, 0, sms, _p(status), limit),
-           out, limit_ns, must_run_out=limit_ns == 0)
+    _check(lambda status, limit: product_probe.run_gate_up(ctypes.byref(operands), pair, 0, sms, _p(status), limit),
+           out, limit_ns, must_run_out=limit_ns == 0 and pair == 1)
