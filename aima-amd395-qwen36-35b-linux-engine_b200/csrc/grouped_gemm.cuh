@@ -91,6 +91,7 @@ struct TcExtra {
   // a_copied_rows of them), where the caller has put them; 256: none
   int copied_above = 256;
   uint64_t a_copied_rows = 0;
+  int k_splits = 1;     // two-SM form of kGemmPlainF32: K is cut into this many runs, each written to its own [rows, n] of c_f32
   bool pair = false;    // two-SM form; in the expert modes the plan's tiles then hold up to 256 rows
   unsigned long long wait_limit_ns = kWaitBudgetNs;    // limit of each wait of the kernel
 };

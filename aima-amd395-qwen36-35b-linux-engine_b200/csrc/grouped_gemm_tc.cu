@@ -68,6 +68,7 @@ struct TcProblem {
   unsigned long long wait_limit_ns;
   // two-SM form
   int dense_tile;         // dense modes: rows per tile
+  int k_splits;           // kGemmPlainF32: runs of K, each a unit of its own
   int copied_above;       // gather: tiles of more rows are read from the copied rows
   SharedProblem shared;   // expert modes: the shared expert's rows, in the same launch
   int shared_tiles;
@@ -670,7 +671,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // registers.
 template <int MODE>
 __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcProblem& pb, uint32_t taddr, int rank,
-                                                 int q, int h, int lane, uint8_t* stage, int chunk, bool shared, int row0,
+                                                 int q, int h, int lane, uint8_t* stage, int chunk, int split, bool shared, int row0,
                                                  int rows, const float* scale, uint32_t drained) {
   constexpr int kStep = 32 * (kPairEpilogueWarps / 4);
   const uint32_t stage_s = smem_u32(stage);
@@ -727,7 +728,7 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
   } else if (MODE == kGemmPlainF32) {
     // FP32 as it is: a row's 32 columns are one 128-byte store
     const int col0 = chunk * kPairN + rank * 128 + 32 * q;
-    float* dst = g.c_f32 + static_cast<size_t>(row0) * g.ldc + col0 + lane;
+    float* dst = g.c_f32 + (static_cast<size_t>(split) * g.dense_rows + row0) * g.ldc + col0 + lane;
 #pragma unroll 1
     for (int c0 = 32 * h; c0 < rows; c0 += kStep) {
       uint32_t r[32];
@@ -849,10 +850,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   __syncthreads();
   cluster_sync_all();
   const bool poisoned = *poison_slot != 0;
-  const int total_units = poisoned ? 0 : n_tiles * pb.n_chunks;
+  constexpr bool kSplit = MODE == kGemmPlainF32;
+  const int unit_chunks = kSplit ? pb.n_chunks * pb.k_splits : pb.n_chunks;
+  const int total_units = poisoned ? 0 : n_tiles * unit_chunks;
   const int n_pairs = gridDim.x >> 1;
   const int pair = blockIdx.x >> 1;
-  const int k_blocks = g.k / kBK;
+  const int k_blocks = g.k / kBK / (kSplit ? pb.k_splits : 1);
 
   // unit -> chunk of 256 weight rows, expert (-1: the shared expert, whose tiles come first), first row and number of
   // rows (1 .. 256) of the tile.  Every role asks for
@@ -860,19 +863,23 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   // them, are never waited for between two units: in the down product, whose units are eight stages long, they cost
   // half of a unit's time.
   struct Unit {
-    int chunk, expert, row0, rows;
+    int chunk, expert, row0, rows, split;
   };
   auto describe = [&](int unit) {
-    Unit u{0, 0, 0, 0};
+    Unit u{0, 0, 0, 0, 0};
     if (unit >= total_units) return u;
     if (kDense) {
       // eight row tiles x all chunks at a time: the pairs that run together then share both operands in L2
-      const int band = unit / (kPlainBand * pb.n_chunks);
+      const int band = unit / (kPlainBand * unit_chunks);
       const int height = min(kPlainBand, n_tiles - band * kPlainBand);
-      const int within = unit - band * kPlainBand * pb.n_chunks;
+      const int within = unit - band * kPlainBand * unit_chunks;
       u.chunk = within / height;
       u.row0 = (band * kPlainBand + within - u.chunk * height) * pb.dense_tile;
       u.rows = min(pb.dense_tile, g.dense_rows - u.row0);
+      if (kSplit) {
+        u.split = u.chunk / pb.n_chunks;
+        u.chunk -= u.split * pb.n_chunks;
+      }
     } else {
       int tile = unit / pb.n_chunks;
       u.chunk = unit - tile * pb.n_chunks;
@@ -919,6 +926,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       // what both blocks fetch for a stage: weights, and the tile's rows (gathered: in fours per block)
       uint32_t stage_bytes = 2 * (kStage2ABytes + half * kBK * 2);
       if (kGather && !tiled(u)) stage_bytes = 2 * kStage2ABytes + (gather_fours(min(half, u.rows)) + gather_fours(u.rows - half)) * (4 * kBK * 2);
+      const int k_first = kSplit ? u.split * k_blocks * kBK : 0;
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         if (elect_one()) {
@@ -936,7 +944,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
           else if (MODE == kGemmExpertDown && shared)
             tma_load_2d_pair(w_dst, &maps.shared_w[0], kb * kBK, u.chunk * kPairN + static_cast<int>(rank) * 128, leader_full);
           else
-            tma_load_2d_pair(w_dst, &maps.w, kb * kBK, w_row, leader_full);
+            tma_load_2d_pair(w_dst, &maps.w, k_first + kb * kBK, w_row, leader_full);
           if (!kGather) {
             int done = 0;
 #pragma unroll
@@ -944,7 +952,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
               const int size = 16 << b;
               if (half & size) {
                 tma_load_2d_pair(w_dst + kStage2ABytes + done * (kBK * 2), shared ? &maps.shared_rows[b] : &maps.rows[b],
-                                 kb * kBK, my_row0 + done, leader_full);
+                                 k_first + kb * kBK, my_row0 + done, leader_full);
                 done += size;
               }
             }
@@ -1114,7 +1122,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       if (!mbar_wait_bounded_warp(tfull_bar(buf), use & 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * kPairRows);
-      drain_transposed<MODE>(g, pb, taddr, static_cast<int>(rank), q, h, lane, my_stage, u.chunk, u.expert < 0, u.row0,
+      drain_transposed<MODE>(g, pb, taddr, static_cast<int>(rank), q, h, lane, my_stage, u.chunk, u.split, u.expert < 0, u.row0,
                              u.rows, scale_now, map_to_rank(tempty_bar(buf), 0));
     }
   }
@@ -1290,7 +1298,9 @@ cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extr
     ok = make_map(&maps.rows[b], g.a, gather ? extra.a_copied_rows : extra.a_rows, g.k, g.lda, 16u << b);
   const SharedProblem& shared = extra.shared;
   if (mode == kGemmPlain || mode == kGemmPlainF32) {
-    pb.dense_tile = dense_tile_rows(g.dense_rows, pb.n_chunks, extra.sm_count / 2);
+    pb.k_splits = mode == kGemmPlainF32 ? extra.k_splits : 1;
+    if (pb.k_splits < 1 || g.k / kBK % pb.k_splits != 0) return cudaErrorInvalidValue;
+    pb.dense_tile = dense_tile_rows(g.dense_rows, pb.n_chunks * pb.k_splits, extra.sm_count / 2);
   } else if (shared.rows > 0) {
     // the shared expert's rows in equal tiles
     const int tiles = (shared.rows + kPairRows - 1) / kPairRows;

@@ -57,89 +57,71 @@ __device__ __forceinline__ float warp_eighth_largest(const float* v, int lane) {
   return key_value(best);
 }
 
+// Where a value goes among the eight selected: the values above the threshold in lane order of this call, behind the
+// `held` ones taken before.  Returns how many are held then.
+__device__ __forceinline__ int take_values(bool take, float value, int expert, int held, int lane, float* sel_v, int* sel_i) {
+  const unsigned m = __ballot_sync(0xffffffffu, take);
+  const int pos = held + __popc(m & ((1u << lane) - 1u));
+  if (take && pos < kTopK) {
+    sel_v[pos] = value;
+    sel_i[pos] = expert;
+  }
+  return held + __popc(m);
+}
+
+// Second half of the reference's prefill selection: lane r < 8 holds the r-th gathered value and its expert.  Fixed bitonic
+// network of width 8 (a pair is exchanged when (value[left] > value[right]) equals the "ascending" flag of the left index),
+// softmax summed in slot order; lane r writes slot r and returns its expert.
+__device__ __forceinline__ int finish_route(float v, int expert, int lane, size_t token, int32_t* __restrict__ ids,
+                                            float* __restrict__ scores, float* __restrict__ weights,
+                                            __nv_bfloat16* __restrict__ dbg_weights) {
+#pragma unroll
+  for (int width = 2; width <= kTopK; width *= 2) {
+#pragma unroll
+    for (int stride = width / 2; stride > 0; stride /= 2) {
+      const float other = __shfl_xor_sync(0xffffffffu, v, stride);
+      const int other_expert = __shfl_xor_sync(0xffffffffu, expert, stride);
+      const bool is_left = (lane & stride) == 0;
+      const bool ascending = (lane & width) != 0;      // the same in both lanes of a pair
+      if (((is_left ? v : other) > (is_left ? other : v)) == ascending) {
+        v = other;
+        expert = other_expert;
+      }
+    }
+  }
+  const float ex = det_expf(__fsub_rn(v, __shfl_sync(0xffffffffu, v, 0)));
+  float denom = 0.0f;
+#pragma unroll
+  for (int r = 0; r < kTopK; ++r) denom = __fadd_rn(denom, __shfl_sync(0xffffffffu, ex, r));
+  if (lane < kTopK) {
+    const size_t o = token * kTopK + lane;
+    const uint16_t wb = float_to_bf16_bits(__fdiv_rn(ex, denom));
+    ids[o] = expert;
+    scores[o] = v;
+    weights[o] = bf16_bits_to_float(wb);
+    if (dbg_weights != nullptr) reinterpret_cast<uint16_t*>(dbg_weights)[o] = wb;
+  }
+  return lane < kTopK ? expert : -1;
+}
+
 // The reference's prefill selection on the final (BF16-rounded) logits of one
 // token held as v[q] = logit of expert 32 q + lane: threshold, gather in expert
-// order, fixed bitonic network, softmax; lanes 0..7 write slot `lane`.  `threshold` is the 8th largest of the values, none
+// order, then finish_route.  `threshold` is the 8th largest of the values, none
 // of which may be a NaN (selectable): then at least eight of them reach it and every slot is written.
 __device__ __forceinline__ int route_token(const float* v, float threshold, int lane, float* sel_v, int* sel_i,
                                             size_t token, int32_t* __restrict__ ids,
                                             float* __restrict__ scores, float* __restrict__ weights,
                                             __nv_bfloat16* __restrict__ dbg_weights) {
-  const unsigned lt_mask = (1u << lane) - 1u;
   int held = 0;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const bool take = v[q] > threshold;
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    if (take) {
-      const int pos = held + __popc(m & lt_mask);
-      sel_v[pos] = v[q];
-      sel_i[pos] = 32 * q + lane;
-    }
-    held += __popc(m);
-  }
+  for (int q = 0; q < 8; ++q) held = take_values(v[q] > threshold, v[q], 32 * q + lane, held, lane, sel_v, sel_i);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const bool take = v[q] == threshold;
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    if (take) {
-      const int pos = held + __popc(m & lt_mask);
-      if (pos < kTopK) {
-        sel_v[pos] = v[q];
-        sel_i[pos] = 32 * q + lane;
-      }
-    }
-    held += __popc(m);
-  }
+  for (int q = 0; q < 8; ++q) held = take_values(v[q] == threshold, v[q], 32 * q + lane, held, lane, sel_v, sel_i);
   __syncwarp();
-  float sv[kTopK];
-  int si[kTopK];
-#pragma unroll
-  for (int r = 0; r < kTopK; ++r) { sv[r] = sel_v[r]; si[r] = sel_i[r]; }
+  const float chosen = sel_v[lane & (kTopK - 1)];
+  const int expert = sel_i[lane & (kTopK - 1)];
   __syncwarp();
-  // fixed 8-wide bitonic network; a pair is exchanged when
-  // (value[left] > value[right]) equals the "ascending" flag of the left index
-#pragma unroll
-  for (int width = 2; width <= kTopK; width *= 2) {
-#pragma unroll
-    for (int stride = width / 2; stride > 0; stride /= 2) {
-#pragma unroll
-      for (int left = 0; left < kTopK; ++left) {
-        const int right = left ^ stride;
-        if (right > left) {
-          const bool ascending = (left & width) != 0;
-          if ((sv[left] > sv[right]) == ascending) {
-            const float tv = sv[left]; sv[left] = sv[right]; sv[right] = tv;
-            const int ti = si[left]; si[left] = si[right]; si[right] = ti;
-          }
-        }
-      }
-    }
-  }
-  float ex[kTopK];
-  float denom = 0.0f;
-#pragma unroll
-  for (int r = 0; r < kTopK; ++r) {
-    ex[r] = det_expf(__fsub_rn(sv[r], sv[0]));
-    denom = __fadd_rn(denom, ex[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < kTopK; ++r) {
-    if (lane == r) {
-      const size_t o = token * kTopK + r;
-      const uint16_t wb = float_to_bf16_bits(__fdiv_rn(ex[r], denom));
-      ids[o] = si[r];
-      scores[o] = sv[r];
-      weights[o] = bf16_bits_to_float(wb);
-      if (dbg_weights != nullptr) reinterpret_cast<uint16_t*>(dbg_weights)[o] = wb;
-    }
-  }
-  int selected = -1;      // lane r < 8 returns the expert of slot r
-#pragma unroll
-  for (int r = 0; r < kTopK; ++r) {
-    if (lane == r) selected = si[r];
-  }
-  return selected;
+  return finish_route(chosen, expert, lane, token, ids, scores, weights, dbg_weights);
 }
 
 // logit transform shared by the router kernels: optional harness hooks, then
@@ -260,9 +242,12 @@ prefill_router_kernel(const __nv_bfloat16* __restrict__ h2,
 // allows, the whole token is recomputed with the canonical dot (all 256
 // experts) and counted.  With audit_stride > 0 every audit_stride-th token is
 // recomputed in full as well and its ids compared with the certified ones.
-// One warp per token.
+// kWays warps share a token's dots: a call whose tokens would leave the chip half empty with one warp each is bound by
+// the latency of one token, which two or four warps cut.  At 8192 tokens the kernel takes 42 us (57 with candidates filed by
+// expert, the selection run by every lane and the statistics added per token), at 333 8 us (14).
 // ---------------------------------------------------------------------------
 constexpr int kCertWarps = 8;
+constexpr int kCertBlocksPerSm = 2;
 constexpr float kCertKappa = 6.103515625e-05f;   // 2^-14, ~4x the summed worst-case rounding terms
 
 // canonical 8-element step of the warp dot with BOTH operands still packed (same FMA order as fma8)
@@ -278,168 +263,240 @@ __device__ __forceinline__ float fma8_packed(const uint4& x, const uint4& w, flo
   return acc;
 }
 
-// The token's row stays packed in registers, and the candidates are recomputed two at a time: the
-// kernel is bound by the latency of the candidates' router rows coming from L2, so two rows are
-// requested before either is used.
-__global__ void __launch_bounds__(kCertWarps * 32, 2)
+// Tensor-core logits of one call: `splits` partial sums over K, each [tokens, 256], added in this order.  (The additions are
+// part of the distance the bound covers: three more roundings beside the 128 of the accumulator.)
+struct ApproxLogits {
+  const float* partial;
+  size_t stride;
+  int splits;
+};
+
+// The token's row stays packed in registers, and the candidates are recomputed two at a time: a pair shares the unpacking
+// of the row, and two router rows are on their way from L2 at once.  A lane keeps one candidate from then on, so that the
+// check of the bound, the selection and the softmax are one pass of the warp each.
+template <int kWays>
+__global__ void __launch_bounds__(kCertWarps * 32, kCertBlocksPerSm)
 prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
                                 const __nv_bfloat16* __restrict__ router,
                                 const __nv_bfloat16* __restrict__ shared_gate,
-                                const float* __restrict__ approx,
+                                const ApproxLogits approx,
                                 const float* __restrict__ row_norms,
                                 const float* __restrict__ bias, int quant_eighths, int tokens,
                                 int32_t* __restrict__ ids, float* __restrict__ scores,
                                 float* __restrict__ weights, float* __restrict__ shared_sigmoid,
                                 __nv_bfloat16* __restrict__ dbg_weights, unsigned long long* __restrict__ stats,
-                                int audit_stride) {
-  __shared__ float sel_v_s[kCertWarps * 8];
-  __shared__ int sel_i_s[kCertWarps * 8];
+                                int audit_stride, uint8_t* __restrict__ chunk_counts) {
+  constexpr int kTokens = kCertWarps / kWays;
+  __shared__ float exact_s[kTokens][kExperts];           // canonical dot of candidate c
+  __shared__ float approx_s[kTokens][kExperts];          // tensor-core logit of expert e
+  __shared__ float bound_s[kTokens][kExperts];           // and how far from it the canonical one may lie
+  __shared__ uint8_t list_s[kCertWarps][kExperts];       // expert of candidate c
+  __shared__ float gate_s[kTokens];
+  __shared__ float sel_v_s[kTokens * kTopK];
+  __shared__ int sel_i_s[kTokens * kTopK];
+  __shared__ int histogram[kExperts];
+  __shared__ int tally[5];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int token = blockIdx.x * kCertWarps + warp;
+  const int slot = warp / kWays;
+  const int part = warp % kWays;
+  const int token = blockIdx.x * kTokens + slot;
+  const bool valid = token < tokens;
+  histogram[threadIdx.x] = 0;
+  if (threadIdx.x < 5) tally[threadIdx.x] = 0;
+  __syncthreads();
   pdl_enter();
-  if (token >= tokens) return;
 
   uint4 xp[8];
-  float sumsq = 0.0f;
+  int n = 0;                        // candidates
+  uint8_t* list = list_s[warp];
+  // Canonical dots of the rows row_of(from), row_of(from + 1), row_of(from + step), row_of(from + step + 1), ... up to
+  // row_of(last): two rows at a time share the unpacking of the token's row.  Bound by the rows coming from L2 (302 MB at
+  // 8192 tokens); fetching the next half of a pair ahead costs registers that the rest of the kernel needs (43 -> 42 us
+  // without it).
+  auto walk = [&](int from, int step, int last, auto row_of, auto sink) {
+    if (from > last) return;
+    uint4 w[2][4];
+    auto fetch = [&](int c, int half) {
+      const uint4* row0 = reinterpret_cast<const uint4*>(row_of(c)) + lane + 128 * half;
+      const uint4* row1 = reinterpret_cast<const uint4*>(row_of(c + 1)) + lane + 128 * half;
 #pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    xp[g] = *(reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(token) * kHidden) + g * 32 + lane);
-    float x8[8];
-    unpack8(xp[g], x8);
+      for (int i = 0; i < 4; ++i) w[0][i] = __ldg(row0 + 32 * i);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sumsq = fmaf(x8[j], x8[j], sumsq);
-  }
-  sumsq = butterfly_sum(sumsq);
-  const float x_norm = sqrtf(sumsq) * 1.0001f;
-
-  float upper[8], lower[8], b[8];
+      for (int i = 0; i < 4; ++i) w[1][i] = __ldg(row1 + 32 * i);
+    };
+#pragma unroll 1
+    for (int c = from; c <= last; c += step) {
+      fetch(c, 0);
+      float acc0 = 0.0f, acc1 = 0.0f;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int e = 32 * q + lane;
-    b[q] = bias != nullptr ? bias[e] : 0.0f;
-    const float a = approx[static_cast<size_t>(token) * kExperts + e];
-    const float delta = kCertKappa * x_norm * row_norms[e] + 9.5367431640625e-07f * fabsf(a + b[q]);
-    upper[q] = finish_logit(a + delta, b[q], quant_eighths);
-    lower[q] = selectable(finish_logit(a - delta, b[q], quant_eighths));      // a NaN bounds nothing from below
-  }
-  const float floor_value = warp_eighth_largest(lower, lane);
-
-  // lane q (q < 8) keeps the candidate mask of experts 32 q .. 32 q + 31; the warp walks all masks
-  // and takes two candidates per trip
-  unsigned my_mask = 0u;
+      for (int i = 0; i < 4; ++i) {
+        acc0 = fma8_packed(xp[i], w[0][i], acc0);
+        acc1 = fma8_packed(xp[i], w[1][i], acc1);
+      }
+      fetch(c, 1);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const unsigned m = __ballot_sync(0xffffffffu, upper[q] >= floor_value);
-    if (lane == q) my_mask = m;
-  }
-  float v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) v[q] = -CUDART_INF_F;
-  int recomputed = 0;
-  int group = 0;
-  unsigned pending = __shfl_sync(0xffffffffu, my_mask, 0);
-  auto pop = [&]() -> int {
-    while (pending == 0u) {
-      if (++group >= 8) return -1;
-      pending = __shfl_sync(0xffffffffu, my_mask, group);
+      for (int i = 0; i < 4; ++i) {
+        acc0 = fma8_packed(xp[4 + i], w[0][i], acc0);
+        acc1 = fma8_packed(xp[4 + i], w[1][i], acc1);
+      }
+      sink(c, butterfly_sum(acc0), butterfly_sum(acc1));
     }
-    const int owner = __ffs(pending) - 1;
-    pending &= pending - 1u;
-    return 32 * group + owner;
   };
-  // canonical logits of two experts at once (e1 < 0: only e0); the owner lanes file them in v
-  auto exact_pair = [&](int e0, int e1, float& acc0, float& acc1) {
-    const uint4* row0 = reinterpret_cast<const uint4*>(router + static_cast<size_t>(e0) * kHidden) + lane;
-    const uint4* row1 = reinterpret_cast<const uint4*>(router + static_cast<size_t>(e1 >= 0 ? e1 : e0) * kHidden) + lane;
-    uint4 w0[8], w1[8];
+  if (valid) {
+    float sumsq = 0.0f;
+    float a[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) w0[i] = __ldg(row0 + i * 32);
+    for (int g = 0; g < 8; ++g)
+      xp[g] = *(reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(token) * kHidden) + g * 32 + lane);
+    const float* logits = approx.partial + static_cast<size_t>(token) * kExperts + lane;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) w1[i] = __ldg(row1 + i * 32);
-    acc0 = 0.0f;
-    acc1 = 0.0f;
+    for (int q = 0; q < 8; ++q) a[q] = logits[32 * q];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      acc0 = fma8_packed(xp[i], w0[i], acc0);
-      acc1 = fma8_packed(xp[i], w1[i], acc1);
+    for (int g = 0; g < 8; ++g) {
+      float x8[8];
+      unpack8(xp[g], x8);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sumsq = fmaf(x8[j], x8[j], sumsq);
     }
-    acc0 = butterfly_sum(acc0);
-    acc1 = butterfly_sum(acc1);
-    const float f0 = selectable(finish_logit(acc0, bias != nullptr ? __ldg(bias + e0) : 0.0f, quant_eighths));
-    const float f1 = selectable(finish_logit(acc1, bias != nullptr && e1 >= 0 ? __ldg(bias + e1) : 0.0f, quant_eighths));
+    for (int split = 1; split < approx.splits; ++split) {      // eight loads at a time: one by one each waits for L2
+      logits += approx.stride;
+      float more[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) more[q] = logits[32 * q];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] = __fadd_rn(a[q], more[q]);
+    }
+    float upper[8], lower[8], norm[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) norm[q] = __ldg(row_norms + 32 * q + lane);
+    sumsq = butterfly_sum(sumsq);
+    const float x_norm = sqrtf(sumsq) * 1.0001f;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      if (e0 == 32 * q + lane) v[q] = f0;
-      if (e1 == 32 * q + lane) v[q] = f1;
+      const int e = 32 * q + lane;
+      const float b = bias != nullptr ? bias[e] : 0.0f;
+      const float delta = kCertKappa * x_norm * norm[q] + 9.5367431640625e-07f * fabsf(a[q] + b);
+      if (part == 0) {
+        approx_s[slot][e] = a[q];
+        bound_s[slot][e] = delta;
+      }
+      upper[q] = finish_logit(a[q] + delta, b, quant_eighths);
+      lower[q] = selectable(finish_logit(a[q] - delta, b, quant_eighths));      // a NaN bounds nothing from below
     }
-  };
-  // is the canonical value further from the tensor-core value than the bound the filter relied on?
-  auto outside_bound = [&](float exact, int e) -> bool {
-    const float a = approx[static_cast<size_t>(token) * kExperts + e];
-    const float be = bias != nullptr ? bias[e] : 0.0f;
-    const float delta = kCertKappa * x_norm * row_norms[e] + 9.5367431640625e-07f * fabsf(a + be);
-    return fabsf(exact - a) > delta;
-  };
-  bool violated = false;
-  while (true) {
-    const int e0 = pop();
-    if (e0 < 0) break;
-    const int e1 = pop();
-    float acc0, acc1;
-    exact_pair(e0, e1, acc0, acc1);
-    if ((e0 & 31) == lane) violated = violated || outside_bound(acc0, e0);
-    if (e1 >= 0 && (e1 & 31) == lane) violated = violated || outside_bound(acc1, e1);
-    recomputed += e1 >= 0 ? 2 : 1;
-  }
-  violated = __any_sync(0xffffffffu, violated);
-  if (violated) {
-    // the premise of the filter failed for this token: take nothing from it
-    for (int e = 0; e < kExperts; e += 2) {
-      float acc0, acc1;
-      exact_pair(e, e + 1, acc0, acc1);
-    }
-  }
-  // exactly eight candidates (nine tokens in ten): all are selected and the threshold is their smallest.  (A value at or
-  // below -inf in the order of the keys takes the general rule.)
-  uint32_t smallest = 0xffffffffu;
+    const float floor_value = warp_eighth_largest(lower, lane);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    if (upper[q] >= floor_value) smallest = min(smallest, order_key(v[q]));
-  }
-  smallest = __reduce_min_sync(0xffffffffu, smallest);
-  const float threshold = (recomputed == kTopK && !violated && smallest > order_key(-CUDART_INF_F))
-                              ? key_value(smallest) : warp_eighth_largest(v, lane);
-  const int certified_id = route_token(v, threshold, lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
-                                       ids, scores, weights, dbg_weights);
-  bool audited = false, audit_mismatch = false;
-  if (audit_stride > 0 && token % audit_stride == 0 && !violated) {
-    for (int e = 0; e < kExperts; e += 2) {
-      float acc0, acc1;
-      exact_pair(e, e + 1, acc0, acc1);
+    for (int q = 0; q < 8; ++q) {
+      const bool take = upper[q] >= floor_value;
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (take) list[n + __popc(m & ((1u << lane) - 1u))] = static_cast<uint8_t>(32 * q + lane);
+      n += __popc(m);
     }
-    const int exact_id = route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
-                                     ids, scores, weights, dbg_weights);
-    audited = true;
-    audit_mismatch = __any_sync(0xffffffffu, lane < kTopK && exact_id != certified_id);
+    __syncwarp();
+    // candidate n stands for the shared expert's gate row
+    walk(2 * part, 2 * kWays, n, [&](int c) { return c < n ? router + static_cast<size_t>(list[c]) * kHidden : shared_gate; },
+         [&](int c, float acc0, float acc1) {
+           if (lane == 0) {
+             if (c < n) exact_s[slot][c] = acc0;
+             else gate_s[slot] = acc0;
+             if (c + 1 < n) exact_s[slot][c + 1] = acc1;
+             else if (c + 1 == n) gate_s[slot] = acc1;
+           }
+         });
   }
-  {
-    const uint4* row = reinterpret_cast<const uint4*>(shared_gate) + lane;
-    float acc = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc = fma8_packed(xp[i], __ldg(row + i * 32), acc);
-    acc = butterfly_sum(acc);
-    if (lane == 0) {
-      shared_sigmoid[token] = round_bf16(det_sigmoid(round_bf16(acc)));
-      if (stats != nullptr) {
-        atomicAdd(stats, static_cast<unsigned long long>(recomputed));
-        atomicAdd(stats + 1, 1ull);
-        if (violated) atomicAdd(stats + 2, 1ull);
-        if (audited) atomicAdd(stats + 3, 1ull);
-        if (audit_mismatch) atomicAdd(stats + 4, 1ull);
+  if (kWays == 1) __syncwarp();
+  else __syncthreads();
+
+  if (valid && part == 0) {
+    const float* exact = exact_s[slot];
+    float* sel_v = sel_v_s + slot * kTopK;
+    int* sel_i = sel_i_s + slot * kTopK;
+    const size_t row = static_cast<size_t>(token);
+    auto bias_of = [&](int e) { return bias != nullptr ? __ldg(bias + e) : 0.0f; };
+    // is a canonical value further from the tensor-core value than the bound the filter relied on?
+    bool violated = false;
+    for (int c = lane; c < n; c += 32) violated = violated || fabsf(exact[c] - approx_s[slot][list[c]]) > bound_s[slot][list[c]];
+    violated = __any_sync(0xffffffffu, violated);
+
+    int chosen = -1;
+    bool routed = false;
+    if (n >= kTopK && n <= 32 && !violated) {
+      // (nearly always) candidate c on lane c, in expert order; of exactly eight all are selected and the threshold is
+      // their smallest.  A threshold at or below -inf in the order of the keys leaves room for other experts: general rule.
+      const bool mine = lane < n;
+      const int e = mine ? list[lane] : 0;
+      const float v = mine ? selectable(finish_logit(exact[lane], bias_of(e), quant_eighths)) : 0.0f;
+      const uint32_t key = mine ? order_key(v) : 0u;
+      uint32_t eighth = 0u;
+      if (n == kTopK) {
+        eighth = __reduce_min_sync(0xffffffffu, mine ? key : 0xffffffffu);
+      } else {
+        uint32_t left = key;
+#pragma unroll 1
+        for (int r = 0; r < kTopK; ++r) {
+          eighth = __reduce_max_sync(0xffffffffu, left);
+          const unsigned owners = __ballot_sync(0xffffffffu, left == eighth);
+          if (lane == __ffs(owners) - 1) left = 0u;
+        }
+      }
+      if (eighth > order_key(-CUDART_INF_F)) {
+        const float threshold = key_value(eighth);
+        const int held = take_values(mine && v > threshold, v, e, 0, lane, sel_v, sel_i);
+        take_values(mine && v == threshold, v, e, held, lane, sel_v, sel_i);
+        __syncwarp();
+        chosen = finish_route(sel_v[lane & (kTopK - 1)], sel_i[lane & (kTopK - 1)], lane, row, ids, scores, weights, dbg_weights);
+        routed = true;
+        __syncwarp();
       }
     }
+    float v[8];
+    auto file = [&](int e, float acc) {       // the owner lane keeps the final logit of expert e
+      const float f = selectable(finish_logit(acc, bias_of(e), quant_eighths));
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (e == 32 * q + lane) v[q] = f;
+      }
+    };
+    auto general = [&]() {
+      return route_token(v, warp_eighth_largest(v, lane), lane, sel_v, sel_i, row, ids, scores, weights, dbg_weights);
+    };
+    if (!routed && !violated) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = -CUDART_INF_F;
+#pragma unroll 1
+      for (int c = 0; c < n; ++c) file(list[c], exact[c]);
+      chosen = general();
+    }
+    // a token whose filter's premise failed takes nothing from it; an audited one is routed both ways
+    const bool audited = audit_stride > 0 && token % audit_stride == 0 && !violated;
+    bool mismatch = false;
+    if (violated || audited) {
+walk(0, 2, kExperts - 1, [&](int e) { return router + static_cast<size_t>(e) * kHidden; },
+           [&](int e, float acc0, float acc1) {
+             file(e, acc0);
+             file(e + 1, acc1);
+           });
+      const int exact_id = general();
+      mismatch = audited && __any_sync(0xffffffffu, lane < kTopK && exact_id != chosen);
+      chosen = exact_id;
+    }
+    if (lane < kTopK) atomicAdd(&histogram[chosen], 1);
+    if (lane == 0) {
+      shared_sigmoid[token] = round_bf16(det_sigmoid(round_bf16(gate_s[slot])));
+      atomicAdd(&tally[0], n);
+      atomicAdd(&tally[1], 1);
+      if (violated) atomicAdd(&tally[2], 1);
+      if (audited) atomicAdd(&tally[3], 1);
+      if (mismatch) atomicAdd(&tally[4], 1);
+    }
   }
+  __syncthreads();
+  // rows of this block per expert, for the plan; the statistics once per block (8192 tokens adding to the same words in L2
+  // one by one)
+  if (chunk_counts != nullptr)
+    chunk_counts[static_cast<size_t>(blockIdx.x) * kExperts + threadIdx.x] = static_cast<uint8_t>(histogram[threadIdx.x]);
+  if (stats != nullptr && threadIdx.x < 5 && tally[threadIdx.x] != 0)
+    atomicAdd(stats + threadIdx.x, static_cast<unsigned long long>(tally[threadIdx.x]));
 }
 
 // ---------------------------------------------------------------------------
@@ -501,21 +558,28 @@ prefill_logits_small_kernel(const __nv_bfloat16* __restrict__ h2, const __nv_bfl
 __global__ void __launch_bounds__(kCertWarps * 32)
 prefill_select_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int quant_eighths, int tokens,
                       int32_t* __restrict__ ids, float* __restrict__ scores, float* __restrict__ weights,
-                      __nv_bfloat16* __restrict__ dbg_weights) {
+                      __nv_bfloat16* __restrict__ dbg_weights, uint8_t* __restrict__ chunk_counts) {
   __shared__ float sel_v_s[kCertWarps * 8];
   __shared__ int sel_i_s[kCertWarps * 8];
+  __shared__ int histogram[kExperts];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * kCertWarps + warp;
+  histogram[threadIdx.x] = 0;
+  __syncthreads();
   pdl_enter();
-  if (token >= tokens) return;
-  float v[8];
+  if (token < tokens) {
+    float v[8];
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
-    v[q] = selectable(finish_logit(logits[static_cast<size_t>(token) * kExperts + 32 * q + lane],
-                                   bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths));
-  route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8, static_cast<size_t>(token),
-              ids, scores, weights, dbg_weights);
+    for (int q = 0; q < 8; ++q)
+      v[q] = selectable(finish_logit(logits[static_cast<size_t>(token) * kExperts + 32 * q + lane],
+                                     bias != nullptr ? bias[32 * q + lane] : 0.0f, quant_eighths));
+    const int chosen = route_token(v, warp_eighth_largest(v, lane), lane, sel_v_s + warp * 8, sel_i_s + warp * 8,
+                                   static_cast<size_t>(token), ids, scores, weights, dbg_weights);
+    if (lane < kTopK) atomicAdd(&histogram[chosen], 1);
+  }
+  __syncthreads();
+  chunk_counts[static_cast<size_t>(blockIdx.x) * kExperts + threadIdx.x] = static_cast<uint8_t>(histogram[threadIdx.x]);
 }
 
 // Euclidean norms of the 256 router rows, rounded up a little; one warp per row.
@@ -550,77 +614,111 @@ __device__ __forceinline__ int rows_per_tile(int count, int n_tiles, int tile_ca
   return ((count + n_tiles - 1) / n_tiles + 31) & ~31;
 }
 
-// One cluster of eight blocks, 256 warps; a warp owns a contiguous run of flat rows.  Count per warp and expert in shared
-// memory, prefix over a block's warps, over the blocks through distributed shared memory, over the experts; then each
-// warp scatters its run.  Block 0 also publishes the counts, the offsets, the tile list and the reference's block-32
-// padded row count.  Bound by latency (the ids are 256 KB at T = 8192): as three kernels -- count, scan, scatter -- it
-// took 28 us there, most of it between the kernels.
-constexpr int kPlanBlocks = 8;
-constexpr int kPlanWarps = 32;
-constexpr int kPlanRounds = 8;      // rounds of 32 rows whose ids are requested together
+// Chunks: runs of `chunk_rows` flat rows, and how many rows of each expert a chunk has (one byte each).  The routers leave
+// the counts of their own blocks' tokens; count_rows_kernel makes them from the ids where those come from elsewhere (forced
+// routing, the all-256 router, other GPUs).  Ids outside [expert_lo, expert_hi) are not in the plan.
+constexpr int kCountRows = 64;
 
-__global__ void __cluster_dims__(kPlanBlocks, 1, 1) __launch_bounds__(kPlanWarps * 32, 1)
+__global__ void __launch_bounds__(kExperts)
+count_rows_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int expert_hi,
+                  uint8_t* __restrict__ chunk_counts) {
+  __shared__ int histogram[kExperts];
+  histogram[threadIdx.x] = 0;
+  __syncthreads();
+  pdl_enter();
+  const int row = blockIdx.x * kCountRows + threadIdx.x;
+  if (threadIdx.x < kCountRows && row < routed_rows) {
+    const int e = ids[row];
+    if (e >= expert_lo && e < expert_hi) atomicAdd(&histogram[e], 1);
+  }
+  __syncthreads();
+  chunk_counts[static_cast<size_t>(blockIdx.x) * kExperts + threadIdx.x] = static_cast<uint8_t>(histogram[threadIdx.x]);
+}
+
+// A block owns a run of chunks.  It adds up the counts of the chunks before its own and of all chunks (every block reads the
+// whole table, 256 KB at T = 8192, from L2), takes the prefix over the experts, and places its rows: a row's position is its
+// expert's offset, the rows of that expert in the chunks before, and its rank in the block, from a bit per row and expert in
+// shared memory.  No block waits for another.  Block 0 also publishes the counts, the offsets, the tile list and the
+// reference's block-32 padded row count.  Bound by latency: 8 us at T = 8192 and 5 us at 333 to 2048; one cluster of eight
+// blocks that counted the ids itself took 24 and 8 to 9 us.
+constexpr int kPlanThreads = 512;
+constexpr int kPlanMaxBlocks = 128;
+
+__global__ void __launch_bounds__(kPlanThreads, 1)
 plan_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int expert_hi, int tile_cap,
+            const uint8_t* __restrict__ chunk_counts, int chunks, int chunk_rows,
             int32_t* __restrict__ expert_counts, int32_t* __restrict__ expert_offsets,
             int32_t* __restrict__ tile_expert, int32_t* __restrict__ tile_row0, int32_t* __restrict__ tile_rows,
             int32_t* __restrict__ tile_count, int32_t* __restrict__ padded_rows,
             int32_t* __restrict__ sorted_rows, int32_t* __restrict__ row_position) {
-  __shared__ int cnt[kPlanWarps][kExperts];      // a warp's counts, then its exclusive prefix, then its next positions
-  __shared__ int block_counts[kExperts];
+  constexpr int kWarps = kPlanThreads / 32;
+  constexpr int kBits = kWarps + 1;              // words per expert, padded against bank conflicts
+  __shared__ __align__(16) int sums[2][kWarps][kExperts];      // of the chunks before this block's, of the others
+  unsigned* const bits = reinterpret_cast<unsigned*>(sums);     // once the sums have been read
+  static_assert(sizeof(unsigned) * kExperts * kBits <= sizeof(sums), "the bits take the place of the sums");
   __shared__ int base[kExperts];
   __shared__ int warp_sums[3][kExperts / 32];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int block = blockIdx.x;                  // the grid is one cluster
-  for (int e = lane; e < kExperts; e += 32) cnt[warp][e] = 0;
-  __syncwarp();
+  const int block = blockIdx.x;
   pdl_enter();
-  const int run = ((routed_rows + kPlanBlocks * kPlanWarps - 1) / (kPlanBlocks * kPlanWarps) + 31) & ~31;
-  const int row_lo = min(routed_rows, (block * kPlanWarps + warp) * run);
-  const int row_hi = min(routed_rows, row_lo + run);
-  // rows routed to experts held by another GPU are not part of this GPU's plan
-  auto fetch = [&](int row0, int* e) {
+  const int per_block = (chunks + gridDim.x - 1) / gridDim.x;
+  const int first = min(chunks, block * per_block);
+  const int row_lo = first * chunk_rows;
+  const int row_hi = min(routed_rows, min(chunks, first + per_block) * chunk_rows);
+
+  // sixteen experts per thread and load, 32 chunks at a time; the bytes of a batch add up in halves of a word
+  const int column = threadIdx.x & 15;
+  auto add_chunks = [&](int from, int to, int* out) {
+    int total[16];
 #pragma unroll
-    for (int i = 0; i < kPlanRounds; ++i) {
-      const int row = row0 + 32 * i + lane;
-      e[i] = row < row_hi ? ids[row] : -1;
-      if (e[i] < expert_lo || e[i] >= expert_hi) e[i] = -1;
+    for (int k = 0; k < 16; ++k) total[k] = 0;
+    constexpr int kStep = kPlanThreads / 16, kBatch = 8;       // loads of a batch are under way together
+    for (int c = from + (threadIdx.x >> 4); c < to; c += kStep * kBatch) {
+      uint4 w[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        w[i] = make_uint4(0, 0, 0, 0);
+        if (c + kStep * i < to)
+          w[i] = __ldg(reinterpret_cast<const uint4*>(chunk_counts + static_cast<size_t>(c + kStep * i) * kExperts) + column);
+      }
+      unsigned even[4] = {0, 0, 0, 0}, odd[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        const unsigned word[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          even[k] += word[k] & 0x00ff00ffu;
+          odd[k] += (word[k] >> 8) & 0x00ff00ffu;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        total[4 * k] += even[k] & 0xffffu;
+        total[4 * k + 1] += odd[k] & 0xffffu;
+        total[4 * k + 2] += even[k] >> 16;
+        total[4 * k + 3] += odd[k] >> 16;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) total[k] += __shfl_xor_sync(0xffffffffu, total[k], 16);
+    if (lane < 16) {
+#pragma unroll
+      for (int k = 0; k < 16; k += 4)
+        *reinterpret_cast<int4*>(out + 16 * column + k) = make_int4(total[k], total[k + 1], total[k + 2], total[k + 3]);
     }
   };
-  for (int row0 = row_lo; row0 < row_hi; row0 += 32 * kPlanRounds) {
-    int e[kPlanRounds];
-    fetch(row0, e);
-#pragma unroll
-    for (int i = 0; i < kPlanRounds; ++i) {
-      const unsigned same = __match_any_sync(0xffffffffu, e[i]);
-      if (e[i] >= 0 && (same & ((1u << lane) - 1u)) == 0u) cnt[warp][e[i]] += __popc(same);
-      __syncwarp();
-    }
-  }
+  add_chunks(0, first, sums[0][warp]);
+  add_chunks(first, chunks, sums[1][warp]);
   __syncthreads();
-  if (threadIdx.x < kExperts) {
-    int running = 0;
-#pragma unroll
-    for (int w = 0; w < kPlanWarps; ++w) {
-      const int c = cnt[w][threadIdx.x];
-      cnt[w][threadIdx.x] = running;
-      running += c;
-    }
-    block_counts[threadIdx.x] = running;
-  }
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   int count = 0, before = 0, v0 = 0, v1 = 0, v2 = 0;
   if (threadIdx.x < kExperts) {
 #pragma unroll
-    for (int b = 0; b < kPlanBlocks; ++b) {
-      uint32_t remote;
-      int c;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&block_counts[threadIdx.x])), "r"(b));
-      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(c) : "r"(remote) : "memory");
-      if (b < block) before += c;
-      count += c;
+    for (int w = 0; w < kWarps; ++w) {
+      before += sums[0][w][threadIdx.x];
+      count += sums[1][w][threadIdx.x];
     }
+    count += before;
     v0 = count;
     v1 = (count + tile_cap - 1) / tile_cap;
     v2 = (count + 31) / 32 * 32;
@@ -633,9 +731,8 @@ plan_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int
     }
     if (lane == 31) { warp_sums[0][warp] = v0; warp_sums[1][warp] = v1; warp_sums[2][warp] = v2; }
   }
-  // this block has read the others' counts; they may leave once it has arrived (waited for at the end)
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   __syncthreads();
+  for (int i = threadIdx.x; i < kExperts * kBits; i += kPlanThreads) bits[i] = 0u;
   if (threadIdx.x < kExperts) {
     const int e = threadIdx.x;
     const int n_tiles = (count + tile_cap - 1) / tile_cap;
@@ -665,38 +762,52 @@ plan_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_lo, int
     }
   }
   __syncthreads();
-  for (int e = lane; e < kExperts; e += 32) cnt[warp][e] += base[e];
-  __syncwarp();
-  for (int row0 = row_lo; row0 < row_hi; row0 += 32 * kPlanRounds) {
-    int e[kPlanRounds];
-    fetch(row0, e);
+  for (int row0 = row_lo; row0 < row_hi; row0 += kPlanThreads) {
+    const int row = row0 + static_cast<int>(threadIdx.x);
+    int e = row < row_hi ? ids[row] : -1;
+    if (e < expert_lo || e >= expert_hi) e = -1;
+    if (e >= 0) atomicOr(&bits[e * kBits + warp], 1u << lane);
+    __syncthreads();
+    if (e >= 0) {
+      int pos = base[e] + __popc(bits[e * kBits + warp] & ((1u << lane) - 1u));
+      for (int w = 0; w < warp; ++w) pos += __popc(bits[e * kBits + w]);
+      sorted_rows[pos] = row;
+      row_position[row] = pos;
+    }
+    if (row0 + kPlanThreads < row_hi) {          // the next rows of this block come behind these
+      __syncthreads();
+      if (threadIdx.x < kExperts) {
+        int held = 0;
 #pragma unroll
-    for (int i = 0; i < kPlanRounds; ++i) {
-      const unsigned same = __match_any_sync(0xffffffffu, e[i]);
-      const int rank = __popc(same & ((1u << lane) - 1u));
-      int pos = 0;
-      if (e[i] >= 0) pos = cnt[warp][e[i]] + rank;
-      __syncwarp();
-      if (e[i] >= 0) {
-        const int row = row0 + 32 * i + lane;
-        sorted_rows[pos] = row;
-        row_position[row] = pos;
-        if (rank == 0) cnt[warp][e[i]] += __popc(same);
+        for (int w = 0; w < kWarps; ++w) {
+          held += __popc(bits[threadIdx.x * kBits + w]);
+          bits[threadIdx.x * kBits + w] = 0u;
+        }
+        base[threadIdx.x] += held;
       }
-      __syncwarp();
+      __syncthreads();
     }
   }
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Enqueues the dispatch plan for `rows` routed rows whose expert ids are `ids`.
+// chunk_rows: flat rows per chunk of the counts that the router has left in ws->chunk_counts; 0: they are counted here
 // tile_cap: rows per tile of the plan -- 128 for the one-SM product kernels, 256 for the two-SM form
-cudaError_t launch_plan(PrefillWorkspace* ws, const int32_t* ids, int rows, int expert_lo, int expert_hi,
+cudaError_t launch_plan(PrefillWorkspace* ws, const int32_t* ids, int rows, int expert_lo, int expert_hi, int chunk_rows,
                         cudaStream_t stream, int* launches, int tile_cap = kTileRows) {
+  if (chunk_rows == 0) {
+    chunk_rows = kCountRows;
+    const cudaError_t code = launch_pdl(count_rows_kernel, dim3((rows + kCountRows - 1) / kCountRows), dim3(kExperts), 0, stream,
+                                        ids, rows, expert_lo, expert_hi, ws->chunk_counts);
+    if (code != cudaSuccess) return code;
+    *launches += 1;
+  }
+  const int chunks = (rows + chunk_rows - 1) / chunk_rows;
   *launches += 1;
-  return launch_pdl(plan_kernel, dim3(kPlanBlocks), dim3(kPlanWarps * 32), 0, stream, ids, rows, expert_lo, expert_hi,
-                    tile_cap, ws->expert_counts, ws->expert_offsets, ws->tile_expert, ws->tile_row0, ws->tile_rows,
-                    ws->tile_count, ws->padded_rows, ws->sorted_rows, ws->row_position);
+  return launch_pdl(plan_kernel, dim3(min(chunks, kPlanMaxBlocks)), dim3(kPlanThreads), 0, stream, ids, rows, expert_lo,
+                    expert_hi, tile_cap, static_cast<const uint8_t*>(ws->chunk_counts), chunks, chunk_rows, ws->expert_counts,
+                    ws->expert_offsets, ws->tile_expert, ws->tile_row0, ws->tile_rows, ws->tile_count, ws->padded_rows,
+                    ws->sorted_rows, ws->row_position);
 }
 
 // ---------------------------------------------------------------------------
@@ -989,10 +1100,28 @@ int set_error(char* error, size_t error_bytes, cudaError_t code, const char* wha
   return static_cast<int>(code);
 }
 
+// Warps per token of the certified router: as many as keep every block of the launch resident at once.  us per layer with
+// 1 / 2 / 4 warps per token, balanced routing: 272 / 269 / 268 at 129 tokens, 282 / 278 / 277 at 333, 288 / 285 / 283 at
+// 592, 303 / 299 / 305 at 1024, 331 / 335 / 344 at 2047.
+int certified_ways(int tokens, int sm_count) {
+  const int warps = kCertBlocksPerSm * kCertWarps * sm_count;
+  return 4 * tokens <= warps ? 4 : 2 * tokens <= warps ? 2 : 1;
+}
+
+// Runs of K of the router logits: few rows are few units, each bound by how fast one pair of SMs can fetch 256 router rows.
+// us per layer with 1 / 2 / 4 / 8 runs, balanced routing: 271 / 270 / 268 / 269 at 129 tokens, 281 / 278 / 277 / 278 at 333,
+// 301 / 299 / 299 / 300 at 1024, 332 / 330 / 331 / 335 at 2047, 436 / 433 / 441 / 446 at 4096.
+constexpr int kSplitMaxTokens = 1024;      // four splits up to here, two beyond
+int router_splits(int tokens) { return tokens <= kSplitMaxTokens ? 4 : 2; }
+size_t approx_logit_count(size_t tokens) {
+  const size_t small = tokens < kSplitMaxTokens ? tokens : kSplitMaxTokens;
+  return (2 * tokens > 4 * small ? 2 * tokens : 4 * small) * kExperts;
+}
+
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 struct Layout {
-  size_t ids, scores, weights, sigmoid, approx, stats, counts, offsets, sorted, position,
+  size_t ids, scores, weights, sigmoid, approx, stats, chunk_counts, counts, offsets, sorted, position,
       tile_expert, tile_row0, tile_rows, tile_count, padded, gathered, act, down, shared_act,
       shared_scaled, x0, x1, h2, total;
 };
@@ -1007,8 +1136,9 @@ Layout layout_for(size_t T) {
   l.scores = take(rows * 4);
   l.weights = take(rows * 4);
   l.sigmoid = take(T * 4);
-  l.approx = take(T * kExperts * 4);
+  l.approx = take(approx_logit_count(T) * 4);
   l.stats = take(5 * sizeof(unsigned long long));
+  l.chunk_counts = take((T + 1) / 2 * kExperts);      // two tokens per chunk at least
   l.counts = take(kExperts * 4);
   l.offsets = take((kExperts + 1) * 4);
   l.sorted = take(rows * 4);
@@ -1072,6 +1202,7 @@ int prefill_workspace_allocate(PrefillWorkspace* ws, uint32_t capacity_tokens, i
   ws->shared_sigmoid = reinterpret_cast<float*>(b + l.sigmoid);
   ws->approx_logits = reinterpret_cast<float*>(b + l.approx);
   ws->router_stats = reinterpret_cast<unsigned long long*>(b + l.stats);
+  ws->chunk_counts = b + l.chunk_counts;
   ws->expert_counts = reinterpret_cast<int32_t*>(b + l.counts);
   ws->expert_offsets = reinterpret_cast<int32_t*>(b + l.offsets);
   ws->sorted_rows = reinterpret_cast<int32_t*>(b + l.sorted);
@@ -1144,6 +1275,7 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   const bool simt = ws->use_simt_gemm;
   const __nv_bfloat16* h2 = static_cast<const __nv_bfloat16*>(call.h2);
 
+  int chunk_rows = 0;      // of the counts the router leaves for the plan; 0: none
   const bool exact_router = ws->exact_router || (dbg != nullptr && dbg->router_logits != nullptr) ||
                             call.router_row_norms == nullptr;
   if (exact_router) {
@@ -1163,8 +1295,9 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
       code = launch_pdl(prefill_select_kernel, dim3((T + kCertWarps - 1) / kCertWarps), dim3(kCertWarps * 32), 0, stream,
                         static_cast<const float*>(ws->approx_logits), call.router_bias, call.quant_eighths, T,
                         ws->topk_ids, ws->topk_scores, ws->topk_weights,
-                        dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr);
+                        dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr, ws->chunk_counts);
     if (code != cudaSuccess) return set_error(error, error_bytes, code, "router of a short call");
+    chunk_rows = kCertWarps * kTopK;
     count += 2;
   } else {
     // tensor-core logits for the candidate filter, then exact recomputation of the candidates
@@ -1175,13 +1308,20 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
     TcExtra rx{};
     rx.status = ws->status; rx.sm_count = ws->sm_count; rx.a_rows = static_cast<uint64_t>(T); rx.experts_in_b = 1;
     rx.pair = true;
+    rx.k_splits = router_splits(T);
     if ((code = launch_grouped_gemm_tc(kGemmPlainF32, r, rx, stream)) != cudaSuccess)
       return set_error(error, error_bytes, code, "router logits product");
-    code = launch_pdl(prefill_router_certified_kernel, dim3((T + kCertWarps - 1) / kCertWarps), dim3(kCertWarps * 32),
-                      0, stream, static_cast<const __nv_bfloat16*>(call.h2), call.layer.router,
-                      call.layer.shared_gate, ws->approx_logits, call.router_row_norms, call.router_bias,
+    const int ways = certified_ways(T, ws->sm_count);
+    const auto kernel = ways == 4 ? prefill_router_certified_kernel<4>
+                                  : ways == 2 ? prefill_router_certified_kernel<2> : prefill_router_certified_kernel<1>;
+    const int block_tokens = kCertWarps / ways;
+    chunk_rows = block_tokens * kTopK;
+    const ApproxLogits approx{ws->approx_logits, static_cast<size_t>(T) * kExperts, rx.k_splits};
+    code = launch_pdl(kernel, dim3((T + block_tokens - 1) / block_tokens), dim3(kCertWarps * 32), 0, stream, h2,
+                      call.layer.router, call.layer.shared_gate, approx, call.router_row_norms, call.router_bias,
                       call.quant_eighths, T, ws->topk_ids, ws->topk_scores, ws->topk_weights, ws->shared_sigmoid,
-                      dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr, ws->router_stats, ws->router_audit_stride);
+                      dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr, ws->router_stats,
+                      ws->router_audit_stride, ws->chunk_counts);
     if (code != cudaSuccess)
       return set_error(error, error_bytes, code, "prefill_router_certified_kernel");
     count += 2;
@@ -1193,10 +1333,11 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
         ws->topk_weights, ws->topk_scores);
     if ((code = cudaGetLastError()) != cudaSuccess) return set_error(error, error_bytes, code, "forced_routing_kernel");
     ++count;
+    chunk_rows = 0;
   }
 
   const int tile_cap = simt ? kTileRows : 2 * kTileRows;
-  if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, stream, &count, tile_cap)) != cudaSuccess)
+  if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, chunk_rows, stream, &count, tile_cap)) != cudaSuccess)
     return set_error(error, error_bytes, code, "dispatch plan");
 
   // Dispatch.  Rows come to the gate_up product by token index, gathered by the kernel itself (TMA gather4), or from a copy
@@ -1385,11 +1526,11 @@ int prefill_layer_launch_ep(PrefillWorkspace* ws, const PrefillCall& call, EpPre
   rx.status = ws->status; rx.sm_count = ws->sm_count; rx.a_rows = static_cast<uint64_t>(T_loc); rx.experts_in_b = 1;
   if ((code = launch_grouped_gemm_tc(kGemmPlainF32, r, rx, stream)) != cudaSuccess)
     return set_error(error, error_bytes, code, "router logits product");
-  prefill_router_certified_kernel<<<(T_loc + kCertWarps - 1) / kCertWarps, kCertWarps * 32, 0, stream>>>(
+  prefill_router_certified_kernel<1><<<(T_loc + kCertWarps - 1) / kCertWarps, kCertWarps * 32, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(call.h2), call.layer.router, call.layer.shared_gate,
-      ws->approx_logits, call.router_row_norms, call.router_bias, call.quant_eighths, T_loc, ws->topk_ids,
+      ApproxLogits{ws->approx_logits, 0, 1}, call.router_row_norms, call.router_bias, call.quant_eighths, T_loc, ws->topk_ids,
       ws->topk_scores, ws->topk_weights, ws->shared_sigmoid,
-      dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr, ws->router_stats, ws->router_audit_stride);
+      dbg ? static_cast<__nv_bfloat16*>(dbg->topk_weights) : nullptr, ws->router_stats, ws->router_audit_stride, nullptr);
   if ((code = cudaGetLastError()) != cudaSuccess) return set_error(error, error_bytes, code, "prefill_router_certified_kernel");
   count += 2;
   if ((code = cudaEventRecord(ws->router_event, stream)) != cudaSuccess ||
@@ -1422,7 +1563,7 @@ int prefill_layer_launch_ep(PrefillWorkspace* ws, const PrefillCall& call, EpPre
   // 3. plan over the global rows that land on this GPU's experts
   const int expert_lo = ep->rank * call.experts_local;
   const int expert_hi = expert_lo + call.experts_local;
-  if ((code = launch_plan(ws, ids_all, rows, expert_lo, expert_hi, stream, &count)) != cudaSuccess)
+  if ((code = launch_plan(ws, ids_all, rows, expert_lo, expert_hi, 0, stream, &count)) != cudaSuccess)
     return set_error(error, error_bytes, code, "dispatch plan");
 
   mark();

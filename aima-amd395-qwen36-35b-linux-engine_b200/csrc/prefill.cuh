@@ -43,12 +43,13 @@ struct PrefillWorkspace {
   float* topk_scores = nullptr;       // [T, 8]
   float* topk_weights = nullptr;      // [T, 8] BF16-rounded, stored as FP32
   float* shared_sigmoid = nullptr;    // [T]    bf16(sigmoid(bf16 gate logit)) as FP32
-  float* approx_logits = nullptr;     // [T, 256] tensor-core router logits (candidate filter only)
+  float* approx_logits = nullptr;     // [K splits, T, 256] tensor-core router logits (candidate filter only)
   // [5] of the certified router: candidates recomputed exactly, tokens routed, tokens whose candidates broke the filter's
   //     bound (recomputed in full), tokens audited, audit mismatches
   unsigned long long* router_stats = nullptr;
   int router_audit_stride = 0;        // qualification: every n-th token is also routed from all 256 canonical logits
   // dispatch plan
+  uint8_t* chunk_counts = nullptr;    // [chunks, 256] rows per expert of each chunk of flat rows
   int32_t* expert_counts = nullptr;   // [256]
   int32_t* expert_offsets = nullptr;  // [257]
   int32_t* sorted_rows = nullptr;     // [8T]  flat (token*8+slot) rows grouped by expert
