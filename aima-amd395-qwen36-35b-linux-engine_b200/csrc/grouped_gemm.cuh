@@ -87,10 +87,7 @@ struct TcExtra {
   uint64_t a_rows;      // rows of the A allocation (TMA bounds; reads beyond are zero-filled)
   int experts_in_b;     // experts held in b0 (expert modes), else 1
   SharedProblem shared = {};    // two-SM form, expert modes
-  // gate_up with gather_src, two-SM form: tiles of more rows than this are read from `a` (rows in expert order,
-  // a_copied_rows of them), where the caller has put them; 256: none
-  int copied_above = 256;
-  uint64_t a_copied_rows = 0;
+  bool fetch = false;   // gate_up with gather_src, two-SM form: rows by cp.async instead of TMA gathers
   int k_splits = 1;     // two-SM form of kGemmPlainF32: K is cut into this many runs, each written to its own [rows, n] of c_f32
   bool pair = false;    // two-SM form; in the expert modes the plan's tiles then hold up to 256 rows
   unsigned long long wait_limit_ns = kWaitBudgetNs;    // limit of each wait of the kernel

@@ -69,7 +69,6 @@ struct TcProblem {
   // two-SM form
   int dense_tile;         // dense modes: rows per tile
   int k_splits;           // kGemmPlainF32: runs of K, each a unit of its own
-  int copied_above;       // gather: tiles of more rows are read from the copied rows
   SharedProblem shared;   // expert modes: the shared expert's rows, in the same launch
   int shared_tiles;
 };
@@ -542,7 +541,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcProblem pb) 
 // what its rows cost, rounded up to 32, and each weight byte enters shared memory once per up to 256 rows.
 //
 //   full[s]    leader only.  Completed by the TMA loads of BOTH blocks (cta_group::2 loads signal the
-//              leader's barrier).
+//              leader's barrier), and with fetched rows by an arrival for the second block's rows[s].
+//   rows[s]    fetched rows: this block's rows of stage s have landed (cp.async arrives by itself).
 //   empty[s]   both blocks: the MMAs reading stage s have retired (tcgen05.commit, multicast to the pair).
 //   tfull[b]   both blocks: accumulator b is complete (commit, multicast).
 //   tempty[b]  leader only: the eight epilogue warps of each block have drained accumulator b.
@@ -788,10 +788,16 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
   }
 }
 
-template <int MODE, bool kGather>
+// Where the rows of A come from: they lie in the order of the plan already; by token index through TMA gathers; or by token
+// index through cp.async.
+enum RowFeed { kRowsInOrder = 0, kRowsGathered = 1, kRowsFetched = 2 };
+
+template <int MODE, int kFeed>
 __global__ void __launch_bounds__(kPairThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProblem pb) {
   static_assert(MODE != kGemmSharedGateUp && MODE != kGemmSharedDown, "the shared expert runs inside the expert modes");
+  constexpr bool kGather = kFeed == kRowsGathered;
+  constexpr bool kFetch = kFeed == kRowsFetched;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -805,6 +811,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
   volatile int* issued_stages = reinterpret_cast<volatile int*>(tail + 16);      // by the producer and the two gather warps
   const uint32_t drain_bar = smem_u32(tail + 32);
+  const uint32_t rows_bar0 = smem_u32(tail + 40);
+  auto rows_bar = [&](int s) { return rows_bar0 + 8u * s; };
   uint8_t* store_stage = smem_gen + kStages2 * kStage2Bytes + kTc2BarrierBytes;
   uint8_t* gather_tables = store_stage + kPairEpilogueWarps * kStoreStage2Bytes;
 
@@ -816,8 +824,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages2; ++s) {
-      mbar_init(full_bar(s), 1);
+      mbar_init(full_bar(s), kFetch ? 2 : 1);
       mbar_init(empty_bar(s), 1);
+      if (kFetch) mbar_init(rows_bar(s), kGatherThreads);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
@@ -897,9 +906,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     return u;
   };
   // a wait ran out in this warp (or it saw the flag of one that did): both blocks of the pair stop
-  // gather: whether the tile's rows lie one after the other all the same -- the shared expert's in the input, a tall
-  // tile's where they were copied -- and come by tile loads.  (Both gather warps then have a box of 16 rows at least.)
-  auto tiled = [&](const Unit& u) { return u.rows > 32 && (u.expert < 0 || u.rows > pb.copied_above); };
+  // Rows that lie one after the other all the same -- the shared expert's, in the input -- come by tile loads: from the
+  // gather warps (which then have a box of 16 rows each at least), or from the warp that loads the weights.
+  auto tiled = [&](const Unit& u) { return u.rows > 32 && u.expert < 0; };
+  auto fetched = [&](const Unit& u) { return kFetch && u.expert >= 0; };
   auto timeout = [&]() {
     if (lane == 0) {
       atomicCAS(pb.status, 0, kStatusTimeoutMbarrier);
@@ -926,6 +936,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       // what both blocks fetch for a stage: weights, and the tile's rows (gathered: in fours per block)
       uint32_t stage_bytes = 2 * (kStage2ABytes + half * kBK * 2);
       if (kGather && !tiled(u)) stage_bytes = 2 * kStage2ABytes + (gather_fours(min(half, u.rows)) + gather_fours(u.rows - half)) * (4 * kBK * 2);
+      if (fetched(u)) stage_bytes = 2 * kStage2ABytes;
       const int k_first = kSplit ? u.split * k_blocks * kBK : 0;
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
@@ -945,7 +956,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
             tma_load_2d_pair(w_dst, &maps.shared_w[0], kb * kBK, u.chunk * kPairN + static_cast<int>(rank) * 128, leader_full);
           else
             tma_load_2d_pair(w_dst, &maps.w, k_first + kb * kBK, w_row, leader_full);
-          if (!kGather) {
+          if (!kGather && !fetched(u)) {
             int done = 0;
 #pragma unroll
             for (int b = 3; b >= 0; --b) {
@@ -973,7 +984,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     // then always waits for both, so that neither can fall behind the ring or run ahead of it by a whole round, which a
     // barrier's parity would not tell.  (One warp for all groups, or the warp that loads the weights, is slower: 456 against
     // 380 us per layer at 2048 tokens.)  Why tall tiles are not gathered: 256 rows are 1440 cycles of gather4 a stage against
-    // 512 of tensor time; with the shared expert's tiles read by tile loads a layer of 1024 tokens went from 324 to 314 us.
+    // 512 of tensor time.
     // The tile's token indices wait in shared memory, one private copy per warp.
     int4* table = reinterpret_cast<int4*>(gather_tables + (warp - 2) * kGatherTableBytes);
     const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
@@ -1023,7 +1034,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
 #pragma unroll
             for (int b = 2; b >= 0; --b) {
               if (my_boxes & (1 << b)) {
-                tma_load_2d_pair(dst + done * (kBK * 2), u.expert < 0 ? &maps.shared_rows[b] : &maps.rows[b], kb * kBK,
+                tma_load_2d_pair(dst + done * (kBK * 2), &maps.shared_rows[b], kb * kBK,
                                  u.row0 + static_cast<int>(rank) * half + done, leader_full);
                 done += 16 << b;
               }
@@ -1042,6 +1053,72 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
       }
     }
     if (lane == 0) issued_stages[warp - 1] = issued;
+  } else if (kFetch && (warp == 2 || warp == 3)) {
+    // ------------------------------ row fetch (both blocks) --------------------
+    // Rows by token index with cp.async, 16 bytes per thread: eight threads take the 64 columns of a row, the two warps groups
+    // of four rows in turn.  The copies arrive on the block's own barrier by themselves; nobody waits for them here.  Moving
+    // a stage's 128 rows takes the two warps no longer than the tensor cores need for them (512 cycles; 1440 by TMA gathers).
+    // Only rows that exist are fetched; what a stage holds beyond them ends in accumulator columns that nobody reads.  Every
+    // thread arrives once per stage, whatever it has fetched: a warp left out of a stage could fall behind by a whole round
+    // of the ring, which a barrier's parity would not tell.
+    const int sub = lane >> 3, piece = lane & 7;
+    const int in_eight = 4 * (warp - 2) + sub;                   // row within every eight of this block's half
+    const uint32_t dst0 = smem_base + kStage2ABytes + in_eight * 128 + ((piece ^ in_eight) << 4);
+    const uint8_t* src0 = reinterpret_cast<const uint8_t*>(g.gather_src) + piece * 16;
+    const uint32_t row_bytes = static_cast<uint32_t>(g.lda) * 2;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool alive = true;
+    auto mine_of = [&](const Unit& u) { return max(0, min(pair_width(u.rows) / 2, u.rows - static_cast<int>(rank) * (pair_width(u.rows) / 2))); };
+    // one unit ahead: token indices (-1: not a row of this tile)
+    auto tokens = [&](const Unit& u, int* t) {
+      const int mine = fetched(u) ? mine_of(u) : 0;
+      const int first = u.row0 + static_cast<int>(rank) * (pair_width(u.rows) / 2);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) t[j] = 8 * j + in_eight < mine ? g.sorted_rows[first + 8 * j + in_eight] >> 3 : -1;
+    };
+    Unit next = describe(pair), later = describe(pair + n_pairs);
+    int token[16];
+    tokens(next, token);
+    for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
+      const Unit u = next;
+      const uint8_t* src[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) src[j] = token[j] >= 0 ? src0 + static_cast<size_t>(token[j]) * row_bytes : nullptr;
+      next = later;
+      tokens(next, token);
+      later = describe(unit + 2 * n_pairs);
+      const int eights = fetched(u) ? (mine_of(u) + 7) / 8 : 0;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_bounded_warp(empty_bar(stage), phase ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
+        const uint32_t dst = dst0 + stage * kStage2Bytes;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (j < eights && src[j] != nullptr) cp_async_16(dst + j * 1024, src[j] + kb * (kBK * 2));
+        }
+        cp_async_arrive_noinc(rows_bar(stage));
+        if (++stage == kStages2) { stage = 0; phase ^= 1u; }
+      }
+    }
+    cp_async_wait_all();
+  } else if (kFetch && warp == 1 && !leader) {
+    // ------------------------------ relay (second block) -----------------------
+    // Tells the leader, whose MMAs read this block's rows too, that a stage's rows have landed.  They stay in this SM: its
+    // own tensor core reads them, ordered by the proxy fence; the arrival is only the signal.  (With release semantics of
+    // cluster scope an arrival took 1.6 us, more than everything else in a stage.)
+    const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool alive = true;
+    for (int unit = pair; unit < total_units && alive; unit += n_pairs) {
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_bounded_warp(rows_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
+        fence_async_proxy();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(leader_full0 + 8u * stage);
+        if (++stage == kStages2) { stage = 0; phase ^= 1u; }
+      }
+    }
   } else if (warp == 1) {
     if (leader) {
       // ------------------------------ MMA issuer (leader) ------------------------
@@ -1060,6 +1137,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kPairRows);
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
+          if (kFetch) {
+            if (!mbar_wait_bounded_warp(rows_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
+            fence_async_proxy();                // written by cp.async, read by the tensor cores
+          }
           tc_fence_after();
           if (elect_one()) {
             const uint32_t w_addr = smem_base + stage * kStage2Bytes;
@@ -1239,9 +1320,9 @@ cudaError_t launch_mode(const TcMaps& maps, const TcProblem& pb, int grid, cudaS
 }
 
 // two-SM form: clusters of two blocks, launched like launch_pdl
-template <int MODE, bool kGather>
+template <int MODE, int kFeed>
 cudaError_t launch_pair_mode(const TcPairMaps& maps, const TcProblem& pb, int grid, cudaStream_t stream) {
-  const cudaError_t e = opt_in_dynamic_smem<grouped_gemm_pair_kernel<MODE, kGather>>(kTc2SmemBytes);
+  const cudaError_t e = opt_in_dynamic_smem<grouped_gemm_pair_kernel<MODE, kFeed>>(kTc2SmemBytes);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(grid & ~1);
@@ -1257,7 +1338,7 @@ cudaError_t launch_pair_mode(const TcPairMaps& maps, const TcProblem& pb, int gr
   attributes[1].val.programmaticStreamSerializationAllowed = t_pdl_relaxed ? 1 : 0;
   config.attrs = attributes;
   config.numAttrs = 2;
-  return cudaLaunchKernelEx(&config, grouped_gemm_pair_kernel<MODE, kGather>, maps, pb);
+  return cudaLaunchKernelEx(&config, grouped_gemm_pair_kernel<MODE, kFeed>, maps, pb);
 }
 
 // Rows per tile of a dense product over `chunks` chunks of 256 columns: the height whose last wave of units wastes
@@ -1281,7 +1362,8 @@ int dense_tile_rows(int rows, int chunks, int pairs) {
 cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extra, TcProblem pb, cudaStream_t stream) {
   TcPairMaps maps;
   const uint64_t experts = static_cast<uint64_t>(extra.experts_in_b);
-  const bool gather = mode == kGemmExpertGateUp && g.gather_src != nullptr;
+  const bool fetch = mode == kGemmExpertGateUp && g.gather_src != nullptr && extra.fetch;
+  const bool gather = mode == kGemmExpertGateUp && g.gather_src != nullptr && !fetch;
   bool ok = true;
   if (mode == kGemmExpertGateUp) {
     pb.n_chunks = g.n / (kPairN / 2);
@@ -1292,10 +1374,7 @@ cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extr
     ok = make_map(&maps.w, g.b0, (mode == kGemmExpertDown ? experts : 1) * static_cast<uint64_t>(g.n), g.k, g.k);
   }
   if (ok && gather) ok = make_map(&maps.one_row, g.gather_src, extra.a_rows, g.k, g.lda, 1u);
-  pb.copied_above = extra.copied_above;
-  const bool tiles = !gather || extra.copied_above < kPairRows;
-  for (int b = 0; ok && tiles && b < (gather ? 3 : 4); ++b)
-    ok = make_map(&maps.rows[b], g.a, gather ? extra.a_copied_rows : extra.a_rows, g.k, g.lda, 16u << b);
+  for (int b = 0; ok && !gather && !fetch && b < 4; ++b) ok = make_map(&maps.rows[b], g.a, extra.a_rows, g.k, g.lda, 16u << b);
   const SharedProblem& shared = extra.shared;
   if (mode == kGemmPlain || mode == kGemmPlainF32) {
     pb.k_splits = mode == kGemmPlainF32 ? extra.k_splits : 1;
@@ -1317,11 +1396,12 @@ cudaError_t launch_pair(GemmMode mode, const GroupedGemm& g, const TcExtra& extr
   }
   if (!ok) return cudaErrorNotSupported;
   if (mode == kGemmExpertGateUp)
-    return gather ? launch_pair_mode<kGemmExpertGateUp, true>(maps, pb, extra.sm_count, stream)
-                  : launch_pair_mode<kGemmExpertGateUp, false>(maps, pb, extra.sm_count, stream);
-  if (mode == kGemmExpertDown) return launch_pair_mode<kGemmExpertDown, false>(maps, pb, extra.sm_count, stream);
-  if (mode == kGemmPlain) return launch_pair_mode<kGemmPlain, false>(maps, pb, extra.sm_count, stream);
-  if (mode == kGemmPlainF32) return launch_pair_mode<kGemmPlainF32, false>(maps, pb, extra.sm_count, stream);
+    return fetch    ? launch_pair_mode<kGemmExpertGateUp, kRowsFetched>(maps, pb, extra.sm_count, stream)
+           : gather ? launch_pair_mode<kGemmExpertGateUp, kRowsGathered>(maps, pb, extra.sm_count, stream)
+                    : launch_pair_mode<kGemmExpertGateUp, kRowsInOrder>(maps, pb, extra.sm_count, stream);
+  if (mode == kGemmExpertDown) return launch_pair_mode<kGemmExpertDown, kRowsInOrder>(maps, pb, extra.sm_count, stream);
+  if (mode == kGemmPlain) return launch_pair_mode<kGemmPlain, kRowsInOrder>(maps, pb, extra.sm_count, stream);
+  if (mode == kGemmPlainF32) return launch_pair_mode<kGemmPlainF32, kRowsInOrder>(maps, pb, extra.sm_count, stream);
   return cudaErrorInvalidValue;
 }
 

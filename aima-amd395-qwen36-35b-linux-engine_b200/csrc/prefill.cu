@@ -811,41 +811,23 @@ cudaError_t launch_plan(PrefillWorkspace* ws, const int32_t* ids, int rows, int 
 }
 
 // ---------------------------------------------------------------------------
-// Copy of h2 rows into expert order: the rows of tiles with more than `copied_above` rows (0: all of them); the product
-// kernel gathers the others by token.  One block per token, 16 bytes per thread: the row is read once and written to the up
-// to eight places the plan gave it.  Bound by the writes (268 MB at 8192 tokens: 53 -> 49 us beside one warp per routed row,
-// which read every row eight times from L2).  us per layer with eight hot experts at 1536 / 2048 / 8192 tokens: 126 / 152 /
-// 561, with 128 threads per token 129 / 154 / 561, with 64 138 / 160 / 556.
+// Copy of h2 rows into expert order, for the products that do not fetch their rows by token index (qualification: the
+// CUDA-core cross-check, and the flag that asks for the copy).  One block per token, 16 bytes per thread: the row is read
+// once and written to the up to eight places the plan gave it.
 // ---------------------------------------------------------------------------
 constexpr int kCopyThreads = kHidden / 8;
 
 __global__ void __launch_bounds__(kCopyThreads)
 gather_rows_kernel(const __nv_bfloat16* __restrict__ h2, const int32_t* __restrict__ ids,
-                   const int32_t* __restrict__ row_position, const int32_t* __restrict__ expert_counts,
-                   const int32_t* __restrict__ expert_offsets, int tile_cap, int copied_above,
-                   __nv_bfloat16* __restrict__ gathered) {
+                   const int32_t* __restrict__ row_position, __nv_bfloat16* __restrict__ gathered) {
   pdl_enter();
-  const int lane = threadIdx.x & 31;
   const int token = blockIdx.x;
-  int position = 0;
-  bool copied = false;
-  if (lane < kTopK) {
-    const int e = ids[token * kTopK + lane];
-    position = row_position[token * kTopK + lane];
-    if (e >= 0 && e < kExperts) {          // rows of other ids are not in the plan
-      const int count = expert_counts[e];
-      const int height = rows_per_tile(count, (count + tile_cap - 1) / tile_cap, tile_cap);
-      copied = min(height, count - (position - expert_offsets[e]) / height * height) > copied_above;
-    }
-  }
-  unsigned pending = __ballot_sync(0xffffffffu, copied);
-  if (pending == 0u) return;
   const uint4 piece = __ldg(reinterpret_cast<const uint4*>(h2 + static_cast<size_t>(token) * kHidden) + threadIdx.x);
-  while (pending != 0u) {
-    const int slot = __ffs(pending) - 1;
-    pending &= pending - 1u;
-    const int to = __shfl_sync(0xffffffffu, position, slot);
-    reinterpret_cast<uint4*>(gathered + static_cast<size_t>(to) * kHidden)[threadIdx.x] = piece;
+#pragma unroll
+  for (int slot = 0; slot < kTopK; ++slot) {
+    const int e = ids[token * kTopK + slot];
+    if (e >= 0 && e < kExperts)            // rows of other ids are not in the plan
+      reinterpret_cast<uint4*>(gathered + static_cast<size_t>(row_position[token * kTopK + slot]) * kHidden)[threadIdx.x] = piece;
   }
 }
 
@@ -1256,10 +1238,7 @@ __global__ void forced_routing_kernel(const int32_t* __restrict__ ids, const __n
   topk_scores[i] = 0.0f;
 }
 
-// dispatch of the routed rows (prefill_layer_launch)
-constexpr int kCopyMinTokens = 1024;
-constexpr int kGatherMaxTokens = 3584;
-constexpr int kCopiedAbove = 96;
+constexpr int kGatherMaxTokens = 128;
 
 int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStream_t stream,
                          int* launches, char* error, size_t error_bytes) {
@@ -1340,23 +1319,17 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   if ((code = launch_plan(ws, ws->topk_ids, rows, 0, kExperts, chunk_rows, stream, &count, tile_cap)) != cudaSuccess)
     return set_error(error, error_bytes, code, "dispatch plan");
 
-  // Dispatch.  Rows come to the gate_up product by token index, gathered by the kernel itself (TMA gather4), or from a copy
-  // in expert order, read by tile loads.  gather4 moves four rows per ~45 cycles, which the weight stream hides while a tile
-  // has few rows and not when it has many, so what decides is the rows of a TILE: those with more than kCopiedAbove are
-  // copied and read, the others gathered.  (The shared expert's rows lie in order anyway and are never gathered.)
-  //   up to kCopyMinTokens   nothing is copied: the copy kernel, which finds its tiles by itself, costs balanced routing more
-  //                          than a tall tile loses (balanced routing at 1024 tokens 314 us, 319 with the launch)
-  //   above kGatherMaxTokens everything is copied: nearly all tiles are tall
-  // us per layer, all gathered / by tile / all copied: eight hot experts 147 / 127 / 127 at 1536 tokens, 182 / 157 / 157 at
-  // 2048, 303 / 267 / 273 at 3584; Zipf 322 / 293 / 303 at 1536, 343 / 334 / 340 at 2048, 510 / 475 / 451 at 3584; balanced
-  // 331 / 336 / 355 at 1536, 350 / 348 / 374 at 2048, 442 / 436 / 431 at 3072, 468 / 460 / 459 at 3584.  A crossing of 64
-  // rows is slower at 2048 balanced tokens (363), 128 to 192 are as good as 96.  (Plain stream order above 2048 tokens and a
-  // copy with one warp per routed row, the same for all three; gather_rows_kernel has what its present form gives.)
-  const bool fused_dispatch = ws->fused_dispatch && !simt && T <= kGatherMaxTokens;
-  const int copied_above = !fused_dispatch ? 0 : T > kCopyMinTokens ? kCopiedAbove : tile_cap;
-  if (copied_above < tile_cap) {
-    code = launch_pdl(gather_rows_kernel, dim3(T), dim3(kCopyThreads), 0, stream, h2, ws->topk_ids, ws->row_position,
-                      ws->expert_counts, ws->expert_offsets, tile_cap, copied_above, ws->gathered);
+  // Dispatch: the gate_up product takes its rows by token index, through TMA gathers in a short call and through cp.async
+  // beyond kGatherMaxTokens.  A gather moves four rows per 45 cycles and is issued by one thread: the shortest way for a few
+  // rows, 1440 cycles a stage against 512 of tensor time for a tall tile.  us per layer, TMA gathers / cp.async: eight hot
+  // experts 33 / 37 at 16 tokens, 40 / 40 at 64, 50 / 44 at 128, 92 / 72 at 592; Zipf 73 / 75 at 16, 123 / 123 at 128,
+  // 190 / 183 at 333, 260 / 233 at 1024; balanced 121 / 122 at 16, 268 / 269 at 128, 280 / 281 at 333, 302 / 305 at 1024.
+  // Beyond that TMA gathers were helped by a copy of the rows in expert order, read by tile loads (268 MB written and read
+  // back at 8192 tokens); copy / cp.async: balanced 337 / 334 at 2047, 442 / 424 at 4096, 730 / 699 at 8192, Zipf 330 / 313,
+  // 489 / 450, 769 / 716, hot 146 / 134, 290 / 261, 585 / 517.
+  const bool fused_dispatch = ws->fused_dispatch && !simt;
+  if (!fused_dispatch) {
+    code = launch_pdl(gather_rows_kernel, dim3(T), dim3(kCopyThreads), 0, stream, h2, ws->topk_ids, ws->row_position, ws->gathered);
     if (code != cudaSuccess) return set_error(error, error_bytes, code, "gather_rows_kernel");
     ++count;
   }
@@ -1377,8 +1350,7 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
   if (fused_dispatch) {
     g.gather_src = h2;
     extra.a_rows = static_cast<uint64_t>(T);
-    extra.copied_above = copied_above;
-    extra.a_copied_rows = static_cast<uint64_t>(ws->capacity) * kTopK;
+    extra.fetch = T > kGatherMaxTokens;
   } else {
     extra.a_rows = static_cast<uint64_t>(ws->capacity) * kTopK;
   }
