@@ -6,7 +6,7 @@
 namespace aima {
 
 // 16 warps, 4 per SM sub-partition: warp 0 control (exchanges, top-8, layer plan), warp 4 issues the
-// bulk copies, warp 8 predicts the next layer's experts, warp 12 is spare, the other twelve stream
+// bulk copies, warp 8 predicts the next layer's experts, warp 12 holds the tensor memory, the other twelve stream
 // the weight ring.  Warp 0 and the twelve streaming warps form the "consumer" group of 13 warps that
 // meets at named barrier 1.
 constexpr int kDecodeConsumerWarps = 13;
@@ -32,9 +32,9 @@ constexpr size_t kEpExchangeBytes = 2ull * kTopK * kHidden * 8;   // per-GPU exp
 constexpr int kDecodeReplicas = 2;
 constexpr unsigned kDecodeEpochPeriod = 65535u * 65536u;   // the device-resident epoch counter counts modulo this
 // Ring items outstanding per block (0: no limit): before it asks for a slot the producer waits until the item
-// issued this many items ago has landed.  0.6105 ms per token without, 0.704 / 0.601 / 0.601 / 0.600 / 0.602 with a
-// limit of 1 / 2 / 3 / 4 / 6 (A/B inside one call).
-constexpr int kDecodeDefaultInFlight = 4;
+// issued this many items ago has landed.  us for 20 launches of one layer / for a launch of 40 with a limit of 3 / 4 / 5 / 6 /
+// none: 386 / 378 / 373 / 372 / 400, and 543 / 543 / 543 / 543 / 552 (A/B inside one call).
+constexpr int kDecodeDefaultInFlight = 6;
 constexpr int kDecodeLogitWords = 2 * kDecodeReplicas * kExperts;   // real + predicted, 64-bit words
 constexpr int kDecodeActStride = 9 * kInter + 64;   // 32-bit words per activation copy; word 9*512 = the shared gate logit
 
