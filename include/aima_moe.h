@@ -86,8 +86,7 @@ typedef struct aima_moe_config {
 #define AIMA_MOE_FLAG_EXACT_ROUTER 2u
 /* Prefill, for A/B timing and qualification: copy the routed activation rows into expert order first
  * (one materialised copy read by tiled TMA loads) for every call.  By default the gate_up tensor-core kernel
- * gathers them by token index itself in calls of up to 1024 tokens; up to 3584 tokens the rows of tiles with more
- * than 96 rows are copied and the others gathered; longer calls copy.  Same bits. */
+ * fetches them by token index itself.  Same bits. */
 #define AIMA_MOE_FLAG_MATERIALIZED_DISPATCH 8u
 /* Expert-parallel prefill: split the plan's tiles into 2 (or 4) parts and, with copy kernels on two more
  * streams, put the rows of one part into expert order / store the results of another back to their owners
