@@ -83,7 +83,7 @@ namespace {
 // the waiter is at most one phase behind, so consecutive uses of a slot must be
 // consumed in order by the same warps.  Every warp of the group waits for and
 // releases every item of its slots, whether it has a row of it or not.
-constexpr int kRingSlots = 6;
+constexpr int kRingSlots = kDecodeRingSlots;
 constexpr int kGroups = 3;
 constexpr int kGroupWarps = 4;
 constexpr int kStreamWarps = kGroups * kGroupWarps;
@@ -412,9 +412,7 @@ moe_decode_persistent_kernel(const DecodeParams p) {
         const unsigned use = seq / kRingSlots;
         unsigned diag[4] = {0, 0, 0, 0};
         bool ok = true;
-        // Requests queue in the SM's path to L2, and every small load or store of the block -- the polls
-        // and stores of the grid-wide hand-overs -- waits behind them: no more than max_in_flight items
-        // are outstanding at a time (enough to cover bandwidth x latency, not more).
+        // The item issued max_in_flight ago has to have landed (what that gives: kDecodeDefaultInFlight).
         if (p.max_in_flight > 0) {
           while (ok && seq - landed >= static_cast<unsigned>(p.max_in_flight)) {
             ok = mbar_wait_bounded(full_bar(landed % kRingSlots), (landed / kRingSlots) & 1u, abort_flag, diag);
@@ -1454,6 +1452,7 @@ cudaError_t launch_variant(const DecodeParams& params, int grid_blocks, cudaStre
   const cudaError_t e = opt_in_dynamic_smem<moe_decode_persistent_kernel<kEp, kExtras, kMulti>>(kDecodeSmemBytes);
   if (e != cudaSuccess) return e;
   DecodeParams local = params;
+  local.max_in_flight = decode_in_flight_limit(params.max_in_flight);
   void* args[] = {&local};
   return cudaLaunchCooperativeKernel(
       reinterpret_cast<const void*>(moe_decode_persistent_kernel<kEp, kExtras, kMulti>), dim3(grid_blocks),

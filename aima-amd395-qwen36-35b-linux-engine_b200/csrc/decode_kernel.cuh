@@ -31,10 +31,15 @@ constexpr size_t kEpExchangeBytes = 2ull * kTopK * kHidden * 8;   // per-GPU exp
 // late whatever the count, 8 had been the flat optimum).
 constexpr int kDecodeReplicas = 2;
 constexpr unsigned kDecodeEpochPeriod = 65535u * 65536u;   // the device-resident epoch counter counts modulo this
-// Ring items outstanding per block (0: no limit): before it asks for a slot the producer waits until the item
-// issued this many items ago has landed.  us for 20 launches of one layer / for a launch of 40 with a limit of 3 / 4 / 5 / 6 /
-// none: 386 / 378 / 373 / 372 / 400, and 543 / 543 / 543 / 543 / 552 (A/B inside one call).
+constexpr int kDecodeRingSlots = 6;      // weight ring of a block: slots of 32 KB
+// Before it asks for a slot the producer waits until the item it issued this many items ago has landed (0: it asks at once).
+// A wait for an item more than a ring back would look at a barrier that has moved on two phases since, which its parity does
+// not tell from one that has not moved: decode_in_flight_limit() holds every value to the ring.
 constexpr int kDecodeDefaultInFlight = 6;
+constexpr int decode_in_flight_limit(int asked) {
+  return asked <= 0 ? 0 : asked < kDecodeRingSlots ? asked : kDecodeRingSlots;
+}
+static_assert(decode_in_flight_limit(kDecodeDefaultInFlight) == kDecodeDefaultInFlight, "the default is within the ring");
 constexpr int kDecodeLogitWords = 2 * kDecodeReplicas * kExperts;   // real + predicted, 64-bit words
 constexpr int kDecodeActStride = 9 * kInter + 64;   // 32-bit words per activation copy; word 9*512 = the shared gate logit
 
@@ -54,7 +59,7 @@ struct DecodeParams {
   const float* router_bias;      // [256] or nullptr
   int quant_eighths;
   int speculate;                 // 1: request the predicted experts' rows before the routing is known
-  int max_in_flight;             // ring items a block may have requested but not yet received (0: no limit)
+  int max_in_flight;             // kDecodeDefaultInFlight or what the host asks for; held to the ring at the launch
   float eps;
   int first_layer;
   int n_layers;

@@ -149,8 +149,7 @@ size_t decode_scratch_size() {
   return kExchangeBytes + align_up(static_cast<size_t>(kDecodeReplicas) * kDecodeActStride * 4, 256);
 }
 
-// AIMA_MOE_DECODE_IN_FLIGHT in the environment overrides how many ring items a block of the decode
-// kernel may have outstanding (0: no limit).
+// AIMA_MOE_DECODE_IN_FLIGHT in the environment takes the place of kDecodeDefaultInFlight.
 int decode_max_in_flight() {
   static const int value = [] {
     const char* v = std::getenv("AIMA_MOE_DECODE_IN_FLIGHT");
