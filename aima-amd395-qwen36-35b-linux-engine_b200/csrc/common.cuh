@@ -246,13 +246,24 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                :: "r"(bar), "r"(bytes) : "memory");
 }
+// kCluster: the phase may be completed by another block of the cluster that publishes its shared memory; the wait then orders
+// nothing by itself (mbar_wait_bounded_warp has the fence).
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  if (kCluster) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  }
   return ok != 0;
 }
 // One lane of a converged warp, for issuing TMA and tcgen05 instructions: their operands live in the warp's uniform
@@ -319,10 +330,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // every look at the barrier, the flag and the clock is a vote, so all lanes leave with one verdict.  A wait that each lane
 // decided for itself could end true in some and false in others when the phase completes while the limit runs out, and the
 // two groups would then wait for each other without one.  One probe inline: it suspends the warp for up to 4 us by itself.
+// With kCluster the fence after it makes visible what another block of the cluster has written to its shared memory and
+// published with its arrival (a fence for shared memory alone, as on the other side).
+template <bool kCluster>
 static __device__ __noinline__ bool mbar_wait_bounded_warp_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                                 unsigned long long limit_ns) {
   const unsigned long long start = global_timer_ns();
-  while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
+  while (!__all_sync(0xffffffffu, mbar_test<kCluster>(bar, parity))) {
     if (__any_sync(0xffffffffu, *abort_flag != 0 || global_timer_ns() - start > limit_ns)) {
       *abort_flag = kStatusTimeoutMbarrier;
       return false;
@@ -330,10 +344,14 @@ static __device__ __noinline__ bool mbar_wait_bounded_warp_slow(uint32_t bar, ui
   }
   return true;
 }
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait_bounded_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                        unsigned long long limit_ns = kWaitBudgetNs) {
-  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
-  return mbar_wait_bounded_warp_slow(bar, parity, abort_flag, limit_ns);
+  if (!__all_sync(0xffffffffu, mbar_test<kCluster>(bar, parity)) &&
+      !mbar_wait_bounded_warp_slow<kCluster>(bar, parity, abort_flag, limit_ns))
+    return false;
+  if (kCluster) asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+  return true;
 }
 
 // Programmatic dependent launch.  A kernel launched with launch_pdl may have its blocks placed

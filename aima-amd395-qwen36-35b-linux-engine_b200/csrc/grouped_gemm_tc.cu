@@ -587,11 +587,19 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrival on a barrier of either block, without cluster-scope release: what it orders are tensor-memory reads (complete
-// before it, tcgen05.wait::ld), and a release at that scope would first wait for every global store of the thread -- in
-// the epilogue, 3000 cycles per unit.
+// Arrival on the barrier for a drained accumulator, of either block, without cluster-scope release: what it orders are
+// tensor-memory reads (complete before it, tcgen05.wait::ld) and no writes to shared memory, and a release at that scope would
+// first wait for every global store of the thread -- in the epilogue, 3000 cycles per unit.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
+}
+// Arrival on the other block's barrier that publishes the shared-memory writes this thread has made or waited for; the other
+// side takes them over with mbar_wait_bounded_warp<true>.  Both fences are restricted to shared memory.  us per layer with
+// them / with arrive.release.cluster and try_wait.acquire.cluster, which order global memory as well: 286 / 588 at 333
+// tokens, 364 / 690 at 2047 with the norms, 714 / 1198 at 8192; without any order at cluster scope 286, 364 and 716.
+__device__ __forceinline__ void mbar_publish_cluster(uint32_t cluster_addr) {
+  asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
 }
 // TMA tile loads of one block of the pair; the bytes are accounted on the LEADER's barrier
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
@@ -1124,9 +1132,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     cp_async_wait_all();
   } else if (kFetch && warp == 1 && !leader) {
     // ------------------------------ relay (second block) -----------------------
-    // Tells the leader, whose MMAs read this block's rows too, that a stage's rows have landed.  They stay in this SM: its
-    // own tensor core reads them, ordered by the proxy fence; the arrival is only the signal.  (With release semantics of
-    // cluster scope an arrival took 1.6 us, more than everything else in a stage.)
+    // Tells the leader, whose MMAs read this block's rows too, that a stage's rows have landed: acquired from this block's
+    // threads by the wait, handed to the async proxy by the fence, and published to the leader by the arrival.
     const uint32_t leader_full0 = map_to_rank(full_bar(0), 0);
     int stage = 0;
     uint32_t phase = 0;
@@ -1136,7 +1143,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
         if (!mbar_wait_bounded_warp(rows_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         fence_async_proxy();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(leader_full0 + 8u * stage);
+        if (lane == 0) mbar_publish_cluster(leader_full0 + 8u * stage);
         if (++stage == kStages2) { stage = 0; phase ^= 1u; }
       }
     }
@@ -1157,10 +1164,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kPairRows);
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded_warp(full_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
+          if (!mbar_wait_bounded_warp<kFetch>(full_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
           if (kFetch) {
             if (!mbar_wait_bounded_warp(rows_bar(stage), phase, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
-            fence_async_proxy();                // written by cp.async, read by the tensor cores
+            fence_async_proxy();                // rows of both blocks: written by cp.async, read by the tensor cores
           }
           tc_fence_after();
           if (elect_one()) {
