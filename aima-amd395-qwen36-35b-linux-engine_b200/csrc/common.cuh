@@ -365,12 +365,14 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 // Whether launch_pdl relaxes the serialisation is the calling thread's choice for the span of one
-// host call (PdlScope).  Overlapping the boundaries of a prefill layer's six or seven kernels gains most where they are short
+// host call (PdlScope).  Overlapping the boundaries of a prefill layer's six kernels gains most where they are short
 // and loses at the top, where kernels of 100 us and more compete with blocks that wait; the prefill entry points relax the
-// order up to pdl_max_tokens().  us per layer, plain order / relaxed, balanced routing: 133 / 121 at 16 tokens, 298 / 289
-// at 333, 318 / 310 at 1024, 350 / 339 at 2048, 416 / 405 at 3072, 446 / 438 at 3584, 469 / 456 at 4096, 572 / 570 at 6144,
-// 735 / 745 at 8192; Zipf: 278 / 270 at 1024, 332 / 324 at 2048, 455 / 449 at 3584, 478 / 480 at 4096, 621 / 615 at 6144,
-// 749 / 772 at 8192.
+// order up to pdl_max_tokens().  us per layer, plain order / relaxed, balanced routing: 127 / 118 at 16 tokens, 280 / 271
+// at 333, 312 / 302 at 1024, 343 / 338 at 2048, 392 / 390 at 3072, 439 / 435 at 4096, 475 / 472 at 5000, 539 / 530 at 6144,
+// 718 / 725 at 8192; Zipf 92 / 80, 163 / 152, 252 / 239, 337 / 330, 402 / 403, 480 / 480, 543 / 548, 614 / 614, 724 / 742; eight
+// hot experts 43 / 35, 65 / 56, 96 / 82, 151 / 143, 225 / 216, 267 / 272, 338 / 342, 417 / 418, 542 / 547.  From 2048 tokens on
+// one side spreads by 3 to 10 % (power cap): the three routings together gain clearly up to 3072 tokens, nothing from 4096 to
+// 6144, and lose at 8192.
 inline thread_local bool t_pdl_relaxed = true;
 struct PdlScope {
   bool saved;

@@ -54,7 +54,7 @@
 // R2, the first blind chunk) into tensor memory as soon as it lands and hand its slot back, so that three more items stream
 // while the block waits for its input; the dots read them from there (556 -> 543 us per token through 40 layers).  A launch
 // of one layer has its input at once; it is a variant of its own without the code for what lies between two layers
-// (384 -> 371 us for 20 launches, with the in-flight limit in decode_kernel.cuh).
+// (384 -> 371 us for 20 launches, 2 of them by the wait of kDecodeDefaultInFlight, four before).
 //
 // Prediction.  A grid-wide hand-over through L2 costs about 1.5 us of pure latency
 // (store, then a poll round trip), a layer has three of them, and nothing that

@@ -33,6 +33,11 @@ constexpr int kDecodeReplicas = 2;
 constexpr unsigned kDecodeEpochPeriod = 65535u * 65536u;   // the device-resident epoch counter counts modulo this
 constexpr int kDecodeRingSlots = 6;      // weight ring of a block: slots of 32 KB
 // Before it asks for a slot the producer waits until the item it issued this many items ago has landed (0: it asks at once).
+// us for 20 launches of one layer / for a launch of 40 with 3 / 4 / 5 / 6 / 0: 375.0 / 372.0 / 370.9 / 370.5 / 383.1, and 536.9 /
+// 536.8 / 536.8 / 536.5 / 544.4 (medians of nine in turn, spread 0.1 %; on one GPU, not timed under expert parallelism).  Six
+// is the whole ring and holds nothing back: the slot asked for is free only after the item before it in that slot has landed.
+// What it changes is that the producer first waits at the slot's `full` barrier and then at `empty`; why that is faster than
+// waiting at `empty` alone is not known.
 // A wait for an item more than a ring back would look at a barrier that has moved on two phases since, which its parity does
 // not tell from one that has not moved: decode_in_flight_limit() holds every value to the ring.
 constexpr int kDecodeDefaultInFlight = 6;

@@ -609,11 +609,11 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(leader_bar) : "memory");
 }
 // The same for weights that are read once, or by neighbouring units at the same time: marked to leave L2 first, so that the
-// stream of weights does not push out the rows, the activations and the outputs that are read again.  us per call with the
-// mark (without: the figure that keeps the ratio to one earlier build, each timed in turn with it), balanced routing, weights
-// of three layers in rotation: 119 (124) at 16 tokens, 286 (286) at 333, 309 (313) at 1024, 367 (378) at 2047 with the norms,
-// 1802 (1826) for four layers of 4096.  With eight hot experts, whose weights many tiles share, no difference: 130 (132) at
-// 2047, 488 to 515 (489 to 509) at 8192.
+// stream of weights does not push out the rows, the activations and the outputs that are read again.  us per layer with the
+// mark / with the normal priority, timed in turn, balanced routing, weights of three layers in rotation: 118 / 124 at 16
+// tokens, 270 / 282 at 333, 300 / 307 at 1024, 332 / 341 at 2047, 414 / 428 at 4096.  No difference beyond the spread of 5 %
+// and more at 8192 tokens (728 / 729) and with eight hot experts, whose weights many tiles share (182 / 189 at 2047, 514 / 511
+// at 8192).
 __device__ __forceinline__ uint64_t policy_stream() {
   uint64_t policy;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
@@ -931,11 +931,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
     }
     return u;
   };
-  // a wait ran out in this warp (or it saw the flag of one that did): both blocks of the pair stop
   // Rows that lie one after the other all the same -- the shared expert's, in the input -- come by tile loads: from the
   // gather warps (which then have a box of 16 rows each at least), or from the warp that loads the weights.
   auto tiled = [&](const Unit& u) { return u.rows > 32 && u.expert < 0; };
   auto fetched = [&](const Unit& u) { return kFetch && u.expert >= 0; };
+  // a wait ran out in this warp (or it saw the flag of one that did): both blocks of the pair stop
   auto timeout = [&]() {
     if (lane == 0) {
       atomicCAS(pb.status, 0, kStatusTimeoutMbarrier);
@@ -1241,8 +1241,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
   if (*abort_flag != 0) {
     // Raised in both blocks, before the barrier above.  Nothing is issued any more; what is under way has to land before
     // shared memory and tensor memory are given up: the MMAs (a last commit, to both blocks) and the loads of the last
-    // round of the ring (the leader's full barriers).  A stage that not every loader got to never completes; its wait gives
-    // the copies that were issued the whole budget.
+    // round of the ring (the leader's full barriers).  A stage that not every loader got to (or, with fetched rows, the
+    // relay) never completes; its wait gives the copies that were issued the whole budget.  Fetched rows have been waited
+    // for by the warps that fetch.
     volatile int ignore = 0;
     if (warp == 1 && leader && elect_one()) umma_commit_pair(drain_bar);
     if (threadIdx.x == 0) {
@@ -1371,8 +1372,8 @@ cudaError_t launch_pair_mode(const TcPairMaps& maps, const TcProblem& pb, int gr
 
 // Rows per tile of a dense product over `chunks` chunks of 256 columns: the height whose last wave of units wastes
 // least.  A unit's time goes with its rows, in steps of 32, but not below what issuing a stage costs (about 128 rows);
-// smaller tiles then only help to spread a product over the chip.  Router logits (one chunk) at 1024 / 8192 rows: 32- /
-// 128-row tiles.
+// smaller tiles then only help to spread a product over the chip.  Router logits (a run of K is a chunk here: four and two)
+// at 1024 / 8192 rows: 64- / 224-row tiles.
 int dense_tile_rows(int rows, int chunks, int pairs) {
   int best = kPairRows;
   long long best_cost = -1;

@@ -471,7 +471,7 @@ prefill_router_certified_kernel(const __nv_bfloat16* __restrict__ h2,
     const bool audited = audit_stride > 0 && token % audit_stride == 0 && !violated;
     bool mismatch = false;
     if (violated || audited) {
-walk(0, 2, kExperts - 1, [&](int e) { return router + static_cast<size_t>(e) * kHidden; },
+      walk(0, 2, kExperts - 1, [&](int e) { return router + static_cast<size_t>(e) * kHidden; },
            [&](int e, float acc0, float acc1) {
              file(e, acc0);
              file(e + 1, acc1);
@@ -503,10 +503,9 @@ walk(0, 2, kExperts - 1, [&](int e) { return router + static_cast<size_t>(e) * k
 // Router of a short call: all 256 canonical logits straight away, spread over the chip by EXPERT -- a block holds two
 // router rows in registers and walks the tokens -- then one warp per token selects.  The tensor-core filter needs the
 // whole router matrix in each 32-token tile and then a chain of dependent loads per token: 20 + 13 us at 16 tokens,
-// whatever their number, against 17 us for both here, growing with the tokens.  us per layer, filter / all logits, balanced
-// routing: 140 / 121 at 16 tokens, 254 / 240 at 64, 281 / 270 at 128, 285 / 280 at 192, 288 / 287 at 256, 289 / 294 at 320,
-// 292 / 311 at 512; with Zipf or eight hot experts they cross at 256 as well.  The limit is where the gain is still above
-// the spread between boxes (4 %, 7 % and 15 % at 128 tokens for the three routings).
+// whatever their number, against 17 us for both here, growing with the tokens.  us per layer, filter / all logits: balanced
+// routing 126 / 118 at 16 tokens, 236 / 229 at 64, 264 / 261 at 128, 269 / 270 at 160, 272 / 278 at 256; Zipf 79 / 69, 98 / 92,
+// 118 / 115, 128 / 127, 145 / 152; eight hot experts 43 / 35, 47 / 41, 53 / 50, 51 / 51, 57 / 63.  They cross at 160 tokens.
 // ---------------------------------------------------------------------------
 constexpr int kSmallRouterTokens = 128;
 
@@ -1083,17 +1082,19 @@ int set_error(char* error, size_t error_bytes, cudaError_t code, const char* wha
 }
 
 // Warps per token of the certified router: as many as keep every block of the launch resident at once.  us per layer with
-// 1 / 2 / 4 warps per token, balanced routing: 272 / 269 / 268 at 129 tokens, 282 / 278 / 277 at 333, 288 / 285 / 283 at
-// 592, 303 / 299 / 305 at 1024, 331 / 335 / 344 at 2047.
+// 1 / 2 / 4 warps per token, balanced routing: 268 / 265 / 264 at 129 tokens, 280 / 276 / 276 at 333, 289 / 287 / 284 at
+// 592, 311 / 305 / 313 at 1024, 317 / 312 / 320 at 1184 (the last with two), 343 / 349 / 362 at 2047.
 int certified_ways(int tokens, int sm_count) {
   const int warps = kCertBlocksPerSm * kCertWarps * sm_count;
   return 4 * tokens <= warps ? 4 : 2 * tokens <= warps ? 2 : 1;
 }
 
 // Runs of K of the router logits: few rows are few units, each bound by how fast one pair of SMs can fetch 256 router rows.
-// us per layer with 1 / 2 / 4 / 8 runs, balanced routing: 271 / 270 / 268 / 269 at 129 tokens, 281 / 278 / 277 / 278 at 333,
-// 301 / 299 / 299 / 300 at 1024, 332 / 330 / 331 / 335 at 2047, 436 / 433 / 441 / 446 at 4096.
-constexpr int kSplitMaxTokens = 1024;      // four splits up to here, two beyond
+// us per layer with 1 / 2 / 4 / 8 runs, balanced routing, weights of three layers in rotation: 265 / 262 / 262 / 262 at 129
+// tokens, 278 / 276 / 276 / 277 at 333, 309 / 306 / 306 / 307 at 1024, 348 / 346 / 346 / 349 at 2047, 437 / 438 / 439 / 447 at
+// 4096 (the median moves by 1 to 2 % from loop to loop).  Two builds in turn, two runs / four: 287.0 / 286.2 at 333 tokens,
+// 309.3 / 308.4 at 1024, two runs of one build within 0.2 %.
+constexpr int kSplitMaxTokens = 1024;      // four runs up to here, two beyond
 int router_splits(int tokens) { return tokens <= kSplitMaxTokens ? 4 : 2; }
 size_t approx_logit_count(size_t tokens) {
   const size_t small = tokens < kSplitMaxTokens ? tokens : kSplitMaxTokens;
@@ -1321,12 +1322,15 @@ int prefill_layer_launch(PrefillWorkspace* ws, const PrefillCall& call, cudaStre
 
   // Dispatch: the gate_up product takes its rows by token index, through TMA gathers in a short call and through cp.async
   // beyond kGatherMaxTokens.  A gather moves four rows per 45 cycles and is issued by one thread: the shortest way for a few
-  // rows, 1440 cycles a stage against 512 of tensor time for a tall tile.  us per layer, TMA gathers / cp.async: eight hot
-  // experts 33 / 37 at 16 tokens, 40 / 40 at 64, 50 / 44 at 128, 92 / 72 at 592; Zipf 73 / 75 at 16, 123 / 123 at 128,
-  // 190 / 183 at 333, 260 / 233 at 1024; balanced 121 / 122 at 16, 268 / 269 at 128, 280 / 281 at 333, 302 / 305 at 1024.
-  // Beyond that TMA gathers were helped by a copy of the rows in expert order, read by tile loads (268 MB written and read
-  // back at 8192 tokens); copy / cp.async: balanced 337 / 334 at 2047, 442 / 424 at 4096, 730 / 699 at 8192, Zipf 330 / 313,
-  // 489 / 450, 769 / 716, hot 146 / 134, 290 / 261, 585 / 517.
+  // rows, 1440 cycles a stage against 512 of tensor time for a tall tile.  us per layer, TMA gathers / cp.async: balanced
+  // routing 118 / 119 at 16 tokens, 232 / 234 at 64, 252 / 256 at 96, 262 / 263 at 128, 275 / 276 at 333, 304 / 305 at 1024;
+  // Zipf 69 / 70 at 16, 93 / 93 at 64, 109 / 106 at 96, 117 / 114 at 128, 168 / 156 at 333, 254 / 235 at 1024; eight hot
+  // experts 39 / 40 at 16, 41 / 40 at 64, 46 / 43 at 96, 50 / 46 at 128, 63 / 57 at 333, 102 / 82 at 1024.  Balanced rows, which
+  // keep the tiles short, never gain from cp.async below 2047 tokens; skewed ones do from 64 on.  The line favours the balanced
+  // ones (1 %) up to 128 tokens, at 2 % with Zipf and 9 % with eight hot experts there, and the skewed ones beyond.
+  // Above 1024 tokens TMA gathers were once helped by a copy of the rows in expert order, read by tile loads (268 MB written
+  // and read back at 8192 tokens); copy / cp.async: balanced 337 / 334 at 2047, 442 / 424 at 4096, 730 / 699 at 8192, Zipf
+  // 330 / 313, 489 / 450, 769 / 716, hot 146 / 134, 290 / 261, 585 / 517.
   const bool fused_dispatch = ws->fused_dispatch && !simt;
   if (!fused_dispatch) {
     code = launch_pdl(gather_rows_kernel, dim3(T), dim3(kCopyThreads), 0, stream, h2, ws->topk_ids, ws->row_position, ws->gathered);

@@ -60,7 +60,9 @@ struct PrefillWorkspace {
   int32_t* tile_count = nullptr;      // [1]
   int32_t* padded_rows = nullptr;     // [1] block-32 padded row count of the reference plan
   // activations
-  __nv_bfloat16* gathered = nullptr;      // [8T, 2048] h2 rows in sorted order
+  // [8T, 2048] h2 rows in sorted order: for the copy flag, the CUDA-core products and the expert-parallel pipeline; a call
+  // that fetches its rows by token index leaves it alone
+  __nv_bfloat16* gathered = nullptr;
   __nv_bfloat16* expert_act = nullptr;    // [8T, 512]
   __nv_bfloat16* expert_down = nullptr;   // [8T, 2048] weighted, sorted order
   __nv_bfloat16* shared_act = nullptr;    // [T, 512]
