@@ -638,8 +638,8 @@ count_rows_kernel(const int32_t* __restrict__ ids, int routed_rows, int expert_l
 // whole table, 256 KB at T = 8192, from L2), takes the prefix over the experts, and places its rows: a row's position is its
 // expert's offset, the rows of that expert in the chunks before, and its rank in the block, from a bit per row and expert in
 // shared memory.  No block waits for another.  Block 0 also publishes the counts, the offsets, the tile list and the
-// reference's block-32 padded row count.  Bound by latency: 8 us at T = 8192 and 5 us at 333 to 2048; one cluster of eight
-// blocks that counted the ids itself took 24 and 8 to 9 us.
+// reference's block-32 padded row count.  Bound by latency: alone 11 us at T = 8192 and 8 at 2048, 8 at 8192 in the running
+// layer; one cluster of eight blocks that counted the ids itself took 24 alone at 8192.
 constexpr int kPlanThreads = 512;
 constexpr int kPlanMaxBlocks = 128;
 
