@@ -587,16 +587,13 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrival on the barrier for a drained accumulator, of either block, without cluster-scope release: what it orders are
-// tensor-memory reads (complete before it, tcgen05.wait::ld) and no writes to shared memory, and a release at that scope would
-// first wait for every global store of the thread -- in the epilogue, 3000 cycles per unit.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
-}
-// Arrival on the other block's barrier that publishes the shared-memory writes this thread has made or waited for; the other
-// side takes them over with mbar_wait_bounded_warp<true>.  Both fences are restricted to shared memory.  us per layer with
-// them / with arrive.release.cluster and try_wait.acquire.cluster, which order global memory as well: 286 / 588 at 333
-// tokens, 364 / 690 at 2047 with the norms, 714 / 1198 at 8192; without any order at cluster scope 286, 364 and 716.
+// Arrival on a barrier of either block that publishes what this thread has done or waited for -- shared-memory writes of a
+// block's own threads, tensor-memory reads -- to the other block, which takes it over with mbar_wait_bounded_warp<true>.  Both
+// fences are restricted to shared memory: a release of everything first waits for the thread's global stores (3000 cycles per
+// unit in the epilogue).  us per layer for the row relay with them / with arrive.release.cluster and try_wait.acquire.cluster:
+// 286 / 588 at 333 tokens, 364 / 690 at 2047 with the norms, 714 / 1198 at 8192; without any order at cluster scope 286, 364 and
+// 716.  For the drained accumulators, with / without: 310 / 310 at 1024 tokens, 367 / 367 at 2047, 1802 / 1800 for four layers of
+// 4096, 322 / 323 for the dense product of 8192 x 12352 x 2048.
 __device__ __forceinline__ void mbar_publish_cluster(uint32_t cluster_addr) {
   asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
@@ -704,7 +701,7 @@ __device__ __forceinline__ void drain_transposed(const GroupedGemm& g, const TcP
   auto release = [&]() {
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive_cluster(drained);
+    if (lane == 0) mbar_publish_cluster(drained);
   };
   if (32 * h >= rows) {
     release();
@@ -1160,7 +1157,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ TcPairMaps maps, const TcProble
         next = describe(unit + n_pairs);
         const int buf = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
-        if (!mbar_wait_bounded_warp(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
+        if (!mbar_wait_bounded_warp<true>(tempty_bar(buf), (use & 1u) ^ 1u, abort_flag, pb.wait_limit_ns)) { alive = false; timeout(); break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(buf * kPairRows);
         for (int kb = 0; kb < k_blocks; ++kb) {
